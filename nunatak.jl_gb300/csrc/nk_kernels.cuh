@@ -195,6 +195,7 @@ struct GeometryView {
     const double* H; const double* bed;
     double* s; double* N; double* mu; double* phi; double2* phi_uv; double2* tau;
     double rho_i, rho_w, gacc;
+    double rw_ri, float_ratio;        // ρw / ρi of the flotation H + (ρw / ρi) b, and 1 - ρi / ρw of a floating surface
     int grounding, gl_stress, use_mask;
     double mask_min, mask_trans;
     const double2* ud = nullptr;      // prescribed (u, v) per face, NaN where free: the right-hand side there

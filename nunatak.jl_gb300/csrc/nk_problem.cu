@@ -1549,6 +1549,7 @@ static GeometryView problem_geometry_view(nk_problem* P) {
     v.g = P->fine.g;
     v.H = P->H; v.bed = P->bed; v.s = P->s; v.N = P->N; v.mu = P->mu; v.phi = P->phi; v.phi_uv = P->phi_uv; v.tau = P->tau;
     v.rho_i = P->pd.ice_density; v.rho_w = P->pd.ocean_density; v.gacc = P->pd.gravitational_acceleration;
+    v.rw_ri = v.rho_w / v.rho_i; v.float_ratio = 1 - v.rho_i / v.rho_w;
     v.grounding = P->pd.grounding; v.gl_stress = P->pd.grounding_line_driving_stress; v.use_mask = P->pd.use_ice_mask;
     v.mask_min = P->pd.mask_minimum_thickness; v.mask_trans = P->pd.mask_transition_thickness;
     v.ud = P->ud;
@@ -3320,14 +3321,7 @@ static void stage_request(const ServerRequest& R, nk_problem* P, double* pin) {
     NK_CUDA(cudaMemsetAsync(P->x, 0, P->plane * sizeof(double2), s));
     if (!R.u0.empty()) stage(NK_FIELD_U, R.u0, uin);
     if (!R.v0.empty()) stage(NK_FIELD_V, R.v0, uin + nu);
-    GeometryView gv;
-    gv.g = P->fine.g;
-    gv.H = P->H; gv.bed = P->bed; gv.s = P->s; gv.N = P->N; gv.mu = P->mu; gv.phi = P->phi; gv.phi_uv = P->phi_uv; gv.tau = P->tau;
-    gv.rho_i = P->pd.ice_density; gv.rho_w = P->pd.ocean_density; gv.gacc = P->pd.gravitational_acceleration;
-    gv.grounding = P->pd.grounding; gv.gl_stress = P->pd.grounding_line_driving_stress; gv.use_mask = P->pd.use_ice_mask;
-    gv.mask_min = P->pd.mask_minimum_thickness; gv.mask_trans = P->pd.mask_transition_thickness;
-    gv.ud = P->ud;
-    launch_geometry(gv, s);
+    launch_problem_geometry(P);   // on P's stream, which is s
 }
 
 // Enqueue on P's stream: u and v of P's solution into the output part of the pinned block `pin`.
