@@ -1,0 +1,469 @@
+// nk_cluster.cu — the coarse levels of the multigrid V-cycle in one thread-block cluster.
+//
+// A level of a few thousand cells is a microsecond of arithmetic on a few SMs, but a grid-wide launch per sweep costs
+// 3.5-9 us of launch, index and load latency whatever its size.  From the first level that fits down to the coarsest,
+// the whole rest of v_cycle! (multigrid_preconditioner.jl:144-163) runs here: pre-sweeps from zero, residual,
+// restriction, the coarsest sweeps, prolongation, post-sweeps.
+//
+// Layout.  The CTAs of the cluster split the rows of every level.  A thread keeps its cells' iterate and the scaled
+// stencil rows in registers, and the masked iterate lives in shared memory with a one-point halo (two buffers per
+// level, all levels resident).  A sweep reads seven neighbours from its own CTA's buffer, writes the other buffer, and
+// pushes its first and last row into the neighbour CTAs' halo rows through distributed shared memory.  Restriction and
+// prolongation read the other level's rows wherever they live.
+//
+// Arithmetic.  A sweep is x' = x + w (b - A x) with w = 1 / rowsum.  A row of A couples five points of its own component
+// and four of the other, and its nine coefficients change only with the coefficients, so -w A is formed once per solve
+// (k_inverse_row_sum, nk_solver.cu) and a sweep costs eighteen multiply-adds a cell.  (The grid-wide kernels difference the
+// neighbours before they multiply; against the sum of products that only moves the rounding, by the size of the rounding
+// of x' itself.)  The residual is the same expression over w.
+//
+// What binds it: latency, a sweep being seven shared loads, the multiply-adds and one cluster barrier.  Split: sixteen
+// CTAs of 512 threads with one cell a thread where the level allows beat eight CTAs (128 x 64 solve 66.8 against 70.5 us a CG iteration, 320 x 160 DIVA 109.9
+// against 125.9), 256 threads (71.7) and levels of 1024 cells kept inside the first CTA, without cluster barriers but with
+// its one shared-memory pipe (72.4).
+// Measured, a whole CG iteration, grid-wide launches with the former one-block coarsest kernel against this one:
+// 128 x 64 mixed 105 -> 67 us, 320 x 160 DIVA 182 -> 110, 1024 x 512 297 -> 254, 300 x 180 FP64 203 -> 167.
+#include <cooperative_groups.h>
+
+#include <mutex>
+
+#include "nk_kernels.cuh"
+#include "nk_transfer.cuh"
+
+namespace nk {
+
+namespace cg = cooperative_groups;
+
+constexpr int CLUSTER_THREADS = 512;
+constexpr int CLUSTER_MAX_CTAS = 16;             // the largest cluster (above 8 by an opt-in attribute)
+constexpr int CLUSTER_CTA_CELLS = 256;           // cells of the top level per CTA, until the cluster is full
+constexpr size_t CLUSTER_SMEM_LIMIT = 200 * 1024;
+
+constexpr int CLUSTER_MAX_ROWS = 1000;           // (j magic) >> 20 divides exactly while j * rows < 2^20
+
+// Cells a thread may own.  A cell's stencil, right-hand side and iterate take 26 registers in FP32 and 52 in FP64, of
+// the 128 a thread has; four cells in FP32 spilled (1360 bytes) and were slower than leaving the level to the grid.
+template <typename T>
+constexpr int cluster_max_cells() { return sizeof(T) == 4 ? 2 : 1; }
+
+// One level as a CTA of the cluster sees it.
+template <typename T>
+struct ClusterLevel {
+    using V2 = typename Vec2<T>::type;
+    using V4 = typename Vec4<T>::type;
+    int Nx, Ny, pitch, px, py, cx, cy;
+    V2* x; V2* b; const V4* st; const uint8_t* mask;
+    int rows, W, off, size;    // rows per CTA, padded row length, offset of the two buffers, entries of one
+    unsigned magic;
+    int j0, cnt;               // this CTA's first row and number of rows
+    int south, north;          // ranks that hold the rows below and above (-1: none, the halo stays zero)
+    int south_row;             // row index, in the buffers of `south`, of its north halo
+    __device__ __forceinline__ int owner(int j) const { return (int)(((unsigned)j * magic) >> 20); }
+    __device__ __forceinline__ int count(int rank) const { int c = Ny - rank * rows; return c < 0 ? 0 : (c > rows ? rows : c); }
+};
+
+template <typename T>
+__device__ __forceinline__ ClusterLevel<T> cluster_level(const ClusterLevels<T>& C, int l, int rank, long long d) {
+    ClusterLevel<T> K;
+    const LevelView<T>& L = C.lv[l];
+    K.Nx = L.o.g.Nx; K.Ny = L.o.g.Ny; K.pitch = L.o.g.pitch; K.px = L.o.g.px; K.py = L.o.g.py;
+    K.cx = L.cx; K.cy = L.cy;
+    K.x = L.x; K.b = L.b; K.st = L.st; K.mask = L.o.mask;
+    rebase_all(d, K.x, K.b, K.st, K.mask);
+    K.rows = C.rows[l];
+    K.magic = C.magic[l];
+    K.off = C.off[l];
+    K.W = K.Nx + 2;
+    K.size = (K.rows + 2) * K.W;
+    K.j0 = rank * K.rows;
+    K.cnt = K.count(rank);
+    K.south = K.north = -1;
+    K.south_row = 0;
+    if (K.cnt > 0) {
+        int js = K.j0 - 1, jn = K.j0 + K.cnt;
+        if (js < 0 && K.py) js = K.Ny - 1;
+        if (jn >= K.Ny) jn = K.py ? 0 : -1;
+        if (js >= 0) { K.south = K.owner(js); K.south_row = K.count(K.south) + 1; }
+        if (jn >= 0) K.north = K.owner(jn);
+    }
+    return K;
+}
+
+// A thread's cells of one level: the iterate, w b and the rows of -w A (E, W, N, S, centre of the own component; centre
+// and three neighbours of the other), so that a sweep is a chain of multiply-adds.
+template <typename T, int CPT>
+struct ClusterCells {
+    using V2 = typename Vec2<T>::type;
+    V2 x[CPT], bw[CPT];
+    T u[CPT][9], v[CPT][9];
+    int p[CPT];                // index in a buffer, -1 for no cell
+    unsigned flags[CPT];
+};
+constexpr unsigned CELL_U = 1, CELL_V = 2;            // the component takes part in the strain rates
+constexpr unsigned CELL_WEST = 4, CELL_EAST = 8;      // first / last column of a periodic axis: repeated in the pad
+constexpr unsigned CELL_SOUTH = 16, CELL_NORTH = 32;  // first / last row of the CTA: pushed into the neighbour's halo
+constexpr unsigned CELL_IU = 64, CELL_IV = 128;       // identity rows
+constexpr int CELL_COL = 8;                           // the column index starts at this bit
+
+template <typename T, int CPT>
+__device__ __forceinline__ int cell_i(const ClusterCells<T, CPT>& c, int k) { return (int)(c.flags[k] >> CELL_COL); }
+
+// The cells' places and stencil rows; w[k] = 1 / rowsum.
+template <typename T, int CPT>
+__device__ __forceinline__ void cluster_setup(const ClusterLevel<T>& K, ClusterCells<T, CPT>& c, typename Vec2<T>::type* w) {
+    using V4 = typename Vec4<T>::type;
+    const int n = K.cnt * K.Nx, plane = K.Nx * K.Ny;
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+        const int e = (int)threadIdx.x + k * CLUSTER_THREADS;
+        c.p[k] = -1;
+        c.flags[k] = 0;
+        if (e >= n) continue;
+        const int jl = e / K.Nx, i = e - jl * K.Nx;
+        c.p[k] = (jl + 1) * K.W + i + 1;
+        const uint8_t m = __ldg(K.mask + (K.j0 + jl) * K.pitch + i);
+        const V4* st = K.st + K.j0 * K.Nx + e;
+        V4 a = st[0], b = st[plane], f = st[2 * plane], h = st[3 * plane], o = st[4 * plane];
+        T* u = c.u[k];
+        T* v = c.v[k];
+        u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w; u[4] = b.x; u[5] = b.y; u[6] = b.z; u[7] = b.w; u[8] = o.x;
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; v[4] = h.x; v[5] = h.y; v[6] = h.z; v[7] = h.w; v[8] = o.y;
+        w[k].x = o.z;
+        w[k].y = o.w;
+        c.flags[k] = ((m & U_INACTIVE) ? 0u : CELL_U) | ((m & V_INACTIVE) ? 0u : CELL_V) | ((K.px && i == 0) ? CELL_WEST : 0u) |
+                     ((K.px && i == K.Nx - 1) ? CELL_EAST : 0u) | ((jl == 0 && K.south >= 0) ? CELL_SOUTH : 0u) |
+                     ((jl == K.cnt - 1 && K.north >= 0) ? CELL_NORTH : 0u) | ((m & U_IDENTITY) ? CELL_IU : 0u) |
+                     ((m & V_IDENTITY) ? CELL_IV : 0u) | ((unsigned)i << CELL_COL);
+    }
+}
+// 1 / rowsum of cell k (the residual's divisor)
+template <typename T, int CPT>
+__device__ __forceinline__ typename Vec2<T>::type cluster_weight(const ClusterLevel<T>& K, int k) {
+    auto o = K.st[4 * K.Nx * K.Ny + K.j0 * K.Nx + (int)threadIdx.x + k * CLUSTER_THREADS];
+    typename Vec2<T>::type w;
+    w.x = o.z;
+    w.y = o.w;
+    return w;
+}
+
+// w (b - A x) of cell k from the masked iterate in `in`
+template <typename T, int CPT>
+__device__ __forceinline__ typename Vec2<T>::type cluster_delta(const ClusterLevel<T>& K, const ClusterCells<T, CPT>& c, int k,
+                                                                const typename Vec2<T>::type* in) {
+    using V2 = typename Vec2<T>::type;
+    const V2* q = in + c.p[k];
+    V2 E = q[1], Wt = q[-1], N = q[K.W], S = q[-K.W], NW = q[K.W - 1], SE = q[1 - K.W];
+    T mu = (c.flags[k] & CELL_U) ? c.x[k].x : T(0), mv = (c.flags[k] & CELL_V) ? c.x[k].y : T(0);
+    const T* u = c.u[k];
+    const T* v = c.v[k];
+    T ya = c.bw[k].x + u[4] * c.x[k].x + u[0] * E.x + u[1] * Wt.x, yb = u[5] * mv + u[6] * N.y + u[7] * NW.y + u[8] * Wt.y;
+    T za = c.bw[k].y + v[4] * c.x[k].y + v[0] * N.y + v[1] * S.y, zb = v[5] * mu + v[6] * E.x + v[7] * SE.x + v[8] * S.x;
+    V2 d;
+    d.x = ya + (yb + (u[2] * N.x + u[3] * S.x));
+    d.y = za + (zb + (v[2] * E.y + v[3] * Wt.y));
+    return d;
+}
+
+// Cell k's masked pair m into buffer `buf` (offset from the start of shared memory), its periodic copies, and the halo
+// rows of the neighbour CTAs.
+template <typename T, int CPT>
+__device__ __forceinline__ void cluster_put(cg::cluster_group& cl, typename Vec2<T>::type* sm, const ClusterLevel<T>& K, int buf,
+                                            const ClusterCells<T, CPT>& c, int k, typename Vec2<T>::type m) {
+    using V2 = typename Vec2<T>::type;
+    const unsigned f = c.flags[k];
+    const int p = c.p[k], Nx = K.Nx;
+    V2* b = sm + buf;
+    b[p] = m;
+    if (f & CELL_WEST) b[p + Nx] = m;
+    if (f & CELL_EAST) b[p - Nx] = m;
+    if (f & (CELL_SOUTH | CELL_NORTH)) {
+        const int col = cell_i<T, CPT>(c, k) + 1;
+        if (f & CELL_SOUTH) {   // this row is the north halo of the CTA below
+            V2* r = cl.map_shared_rank(b, K.south) + K.south_row * K.W + col;
+            *r = m;
+            if (f & CELL_WEST) r[Nx] = m;
+            if (f & CELL_EAST) r[-Nx] = m;
+        }
+        if (f & CELL_NORTH) {   // and the south halo of the CTA above
+            V2* r = cl.map_shared_rank(b, K.north) + col;
+            *r = m;
+            if (f & CELL_WEST) r[Nx] = m;
+            if (f & CELL_EAST) r[-Nx] = m;
+        }
+    }
+}
+template <typename T, int CPT>
+__device__ __forceinline__ typename Vec2<T>::type cluster_masked(const ClusterCells<T, CPT>& c, int k, typename Vec2<T>::type x) {
+    if (!(c.flags[k] & CELL_U)) x.x = T(0);
+    if (!(c.flags[k] & CELL_V)) x.y = T(0);
+    return x;
+}
+
+// Row j of level K's buffer, in whichever CTA holds it: column i is entry i + 1
+template <typename T>
+__device__ __forceinline__ const typename Vec2<T>::type* cluster_row(cg::cluster_group& cl, typename Vec2<T>::type* sm,
+                                                                    const ClusterLevel<T>& K, int buf, int j) {
+    const int rank = K.owner(j);
+    return cl.map_shared_rank(sm + buf, rank) + (j - rank * K.rows + 1) * K.W + 1;
+}
+
+// The fine points 2 I - 1 .. 2 I + 2 (I alone on an axis that is not halved) of one axis of the restriction: their
+// indices and the weights of a face-located and of a centre-located component (ridx and rweight; a point beyond a Bounded
+// edge has weight zero and reads the edge).
+template <typename T>
+__device__ __forceinline__ void restriction_axis(int I, int Nc, int Nf, bool periodic, int c, int* at, T* face, T* centre) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        if (c == 1) {
+            at[a] = I;
+            face[a] = centre[a] = a == 1 ? T(1) : T(0);
+        } else {
+            int i = 2 * I + a - 1;
+            at[a] = periodic ? (i < 0 ? i + Nf : (i >= Nf ? i - Nf : i)) : (i < 0 ? 0 : (i > Nf - 1 ? Nf - 1 : i));
+            face[a] = a == 1 ? T(1) : (a == 3 || (a == 0 && !periodic && I == 0) ? T(0) : T(1) / T(2));
+            T w = a == 1 || a == 2 ? T(3) / T(4) : T(1) / T(4);
+            if (!periodic) {
+                if ((I == 0 && a == 0) || (I == Nc - 1 && a == 3)) w = T(0);
+                if ((I == 0 && a == 1) || (I == Nc - 1 && a == 2)) w += T(1) / T(4);
+            }
+            centre[a] = w;
+        }
+    }
+}
+
+template <typename T, int CPT>
+__global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __grid_constant__ ClusterLevels<T> C, const int* done) {
+    long long d;
+    if (!batch_slot(C.lv[0].o.g, d)) return;   // the same answer in every CTA of a cluster (one slot)
+    if (d) rebase(done, d);
+    if (done && *(volatile const int*)done) return;
+    using V2 = typename Vec2<T>::type;
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = blockIdx.x, last = C.n - 1;
+    extern __shared__ __align__(32) unsigned char smem_raw[];
+    V2* sm = reinterpret_cast<V2*>(smem_raw);
+
+    ClusterCells<T, CPT> c;
+    V2 w[CPT];
+    ClusterLevel<T> K = cluster_level(C, 0, rank, d);
+    cluster_setup<T, CPT>(K, c, w);
+#pragma unroll
+    for (int k = 0; k < CPT; ++k)
+        if (c.p[k] >= 0) {
+            const int e = (int)threadIdx.x + k * CLUSTER_THREADS, i = cell_i<T, CPT>(c, k);
+            V2 b = K.b[(K.j0 + (e - i) / K.Nx) * K.pitch + i];
+            c.bw[k].x = b.x * w[k].x;
+            c.bw[k].y = b.y * w[k].y;
+        }
+    for (int e = threadIdx.x; e < C.total; e += CLUSTER_THREADS) { V2 z; z.x = z.y = T(0); sm[e] = z; }
+    cl.sync();   // the zeroed halos are in place before a neighbour writes into them
+    // down
+    for (int l = 0;; ++l) {
+        const int buf0 = K.off, buf1 = K.off + K.size;
+        const int ns = l == last ? C.coarsest : C.sweeps;
+#pragma unroll
+        for (int k = 0; k < CPT; ++k)   // the first sweep from zero: x = w b
+            if (c.p[k] >= 0) {
+                c.x[k] = c.bw[k];
+                cluster_put<T, CPT>(cl, sm, K, buf0, c, k, cluster_masked<T, CPT>(c, k, c.x[k]));
+            }
+        cl.sync();
+        int cur = buf0;
+        for (int s = 1; s < ns; ++s) {
+            const int nxt = cur == buf0 ? buf1 : buf0;
+#pragma unroll
+            for (int k = 0; k < CPT; ++k)
+                if (c.p[k] >= 0) {
+                    V2 dl = cluster_delta<T, CPT>(K, c, k, sm + cur);
+                    c.x[k].x += dl.x;
+                    c.x[k].y += dl.y;
+                    cluster_put<T, CPT>(cl, sm, K, nxt, c, k, cluster_masked<T, CPT>(c, k, c.x[k]));
+                }
+            cl.sync();
+            cur = nxt;
+        }
+        if (l == last) break;
+        const int res = cur == buf0 ? buf1 : buf0;   // the residual takes the free buffer
+#pragma unroll
+        for (int k = 0; k < CPT; ++k)
+            if (c.p[k] >= 0) {
+                V2 r = cluster_delta<T, CPT>(K, c, k, sm + cur), wk = cluster_weight<T, CPT>(K, k);
+                r.x = wk.x == T(0) ? T(0) : r.x / wk.x;
+                r.y = wk.y == T(0) ? T(0) : r.y / wk.y;
+                sm[res + c.p[k]] = cluster_masked<T, CPT>(c, k, r);
+            }
+        ClusterLevel<T> N = cluster_level(C, l + 1, rank, d);
+        cluster_setup<T, CPT>(N, c, w);
+        cl.sync();
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) {
+            if (c.p[k] < 0) continue;
+            const int e = (int)threadIdx.x + k * CLUSTER_THREADS, I = cell_i<T, CPT>(c, k), J = N.j0 + (e - I) / N.Nx;
+            int at[4], row[4];
+            T fx[4], cx[4], fy[4], cy[4];
+            restriction_axis<T>(I, N.Nx, K.Nx, K.px, N.cx, at, fx, cx);
+            restriction_axis<T>(J, N.Ny, K.Ny, K.py, N.cy, row, fy, cy);
+            T su = T(0), sv = T(0);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const V2* r = cluster_row<T>(cl, sm, K, res, row[b]);
+                T hu = T(0), hv = T(0);
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    V2 q = r[at[a]];
+                    if (a < 3) hu += fx[a] * q.x;
+                    hv += cx[a] * q.y;
+                }
+                su += cy[b] * hu;
+                if (b < 3) sv += fy[b] * hv;
+            }
+            V2 b;
+            b.x = (c.flags[k] & CELL_IU) ? T(0) : su;
+            b.y = (c.flags[k] & CELL_IV) ? T(0) : sv;
+            N.b[J * N.pitch + I] = b;   // read back by this thread on the way up
+            c.bw[k].x = b.x * w[k].x;
+            c.bw[k].y = b.y * w[k].y;
+        }
+        K = N;
+    }
+    // up: the coarser level's iterate is in the buffer its last sweep wrote
+    int coarse_buf = K.off + (((C.coarsest - 1) & 1) ? K.size : 0);
+    for (int l = last - 1; l >= 0; --l) {
+        ClusterLevel<T> N = cluster_level(C, l, rank, d);
+        cluster_setup<T, CPT>(N, c, w);
+        const int down = (C.sweeps - 1) & 1;   // the buffer that holds the iterate of the way down
+        int cur = N.off + (down ? 0 : N.size);
+        const int old = N.off + (down ? N.size : 0);
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) {
+            if (c.p[k] < 0) continue;
+            const int e = (int)threadIdx.x + k * CLUSTER_THREADS, i = cell_i<T, CPT>(c, k), j = N.j0 + (e - i) / N.Nx;
+            V2 b = N.b[j * N.pitch + i], x = sm[old + c.p[k]];
+            c.bw[k].x = b.x * w[k].x;
+            c.bw[k].y = b.y * w[k].y;
+            // an inactive row is an identity row: its iterate is w b after every sweep, and shared memory holds zero
+            if (!(c.flags[k] & CELL_U)) x.x = c.bw[k].x;
+            if (!(c.flags[k] & CELL_V)) x.y = c.bw[k].y;
+            int fi1, fi2, ci1, ci2, fj1, fj2, cj1, cj2;   // face and centre parents of each axis
+            T fa1, fa2, ca1, ca2, fb1, fb2, cb1, cb2;
+            parents<T>(i, K.Nx, K.px, true, K.cx, fi1, fi2, fa1, fa2);
+            parents<T>(i, K.Nx, K.px, false, K.cx, ci1, ci2, ca1, ca2);
+            parents<T>(j, K.Ny, K.py, true, K.cy, fj1, fj2, fb1, fb2);
+            parents<T>(j, K.Ny, K.py, false, K.cy, cj1, cj2, cb1, cb2);
+            if (fj2 >= K.Ny) { fj2 = fj1; fb2 = T(0); }   // the north wall face of a Bounded axis carries zero
+            const V2 *ru1 = cluster_row<T>(cl, sm, K, coarse_buf, cj1), *ru2 = cluster_row<T>(cl, sm, K, coarse_buf, cj2);
+            const V2 *rv1 = cluster_row<T>(cl, sm, K, coarse_buf, fj1), *rv2 = cluster_row<T>(cl, sm, K, coarse_buf, fj2);
+            T pu = fa1 * (cb1 * ru1[fi1].x + cb2 * ru2[fi1].x) + fa2 * (cb1 * ru1[fi2].x + cb2 * ru2[fi2].x);
+            T pv = ca1 * (fb1 * rv1[ci1].y + fb2 * rv2[ci1].y) + ca2 * (fb1 * rv1[ci2].y + fb2 * rv2[ci2].y);
+            if (!(c.flags[k] & CELL_IU)) x.x += pu;
+            if (!(c.flags[k] & CELL_IV)) x.y += pv;
+            c.x[k] = x;
+            cluster_put<T, CPT>(cl, sm, N, cur, c, k, cluster_masked<T, CPT>(c, k, x));
+        }
+        cl.sync();
+        for (int s = 0; s < C.sweeps; ++s) {
+            const int nxt = cur == N.off ? N.off + N.size : N.off;
+            const bool out = l == 0 && s == C.sweeps - 1;
+#pragma unroll
+            for (int k = 0; k < CPT; ++k)
+                if (c.p[k] >= 0) {
+                    V2 dl = cluster_delta<T, CPT>(N, c, k, sm + cur);
+                    c.x[k].x += dl.x;
+                    c.x[k].y += dl.y;
+                    if (!out) cluster_put<T, CPT>(cl, sm, N, nxt, c, k, cluster_masked<T, CPT>(c, k, c.x[k]));
+                }
+            if (!out) cl.sync();
+            cur = nxt;
+        }
+        coarse_buf = cur;
+        K = N;
+    }
+#pragma unroll
+    for (int k = 0; k < CPT; ++k)
+        if (c.p[k] >= 0) {
+            const int e = (int)threadIdx.x + k * CLUSTER_THREADS, i = cell_i<T, CPT>(c, k);
+            K.x[(K.j0 + (e - i) / K.Nx) * K.pitch + i] = c.x[k];
+        }
+    cl.sync();   // no CTA leaves while another may still read its shared memory
+}
+
+// Rows per CTA and buffer offsets of levels lv[0 .. n-1] (lv[0] the finest of them); false if they do not fit.
+template <typename T>
+bool cluster_plan(ClusterLevels<T>& C) {
+    if (C.n < 1 || C.n > MAX_COARSE_LEVELS || C.sweeps < 1 || C.coarsest < 1) return false;
+    long long top = (long long)C.lv[0].o.g.Nx * C.lv[0].o.g.Ny;
+    const int ctas = (int)((top + CLUSTER_CTA_CELLS - 1) / CLUSTER_CTA_CELLS);
+    C.ctas = 1;
+    while (C.ctas < ctas && C.ctas < CLUSTER_MAX_CTAS) C.ctas *= 2;
+    long long off = 0;
+    C.cells = 1;
+    for (int l = 0; l < C.n; ++l) {
+        const DevGrid<T>& g = C.lv[l].o.g;
+        int rows = (g.Ny + C.ctas - 1) / C.ctas;
+        long long cells = (long long)rows * g.Nx;
+        if (!C.lv[l].st || g.Ny > CLUSTER_MAX_ROWS || cells > (long long)cluster_max_cells<T>() * CLUSTER_THREADS) return false;
+        int need = (int)((cells + CLUSTER_THREADS - 1) / CLUSTER_THREADS);
+        while (C.cells < need) C.cells *= 2;
+        C.rows[l] = rows;
+        C.magic[l] = ((1u << 20) + rows - 1) / rows;   // j / rows = (j magic) >> 20 for every row j < CLUSTER_MAX_ROWS
+        C.off[l] = (int)off;
+        off += 2ll * (rows + 2) * (g.Nx + 2);
+        if (off * (long long)sizeof(typename Vec2<T>::type) > (long long)CLUSTER_SMEM_LIMIT) return false;
+    }
+    C.total = (int)off;
+    return true;
+}
+
+template <typename T, int CPT>
+static void launch_cluster(const ClusterLevels<T>& C, const int* done, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C.ctas, 1, batch_slots());
+    cfg.blockDim = dim3(CLUSTER_THREADS);
+    cfg.dynamicSmemBytes = (size_t)C.total * sizeof(typename Vec2<T>::type);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C.ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_coarse_cluster<T, CPT>, C, done);
+}
+template <typename T>
+void launch_coarse_cluster(const ClusterLevels<T>& C, const int* done, cudaStream_t s) {
+    if constexpr (cluster_max_cells<T>() >= 2) {
+        if (C.cells == 2) launch_cluster<T, 2>(C, done, s);
+        else launch_cluster<T, 1>(C, done, s);
+    } else {
+        launch_cluster<T, 1>(C, done, s);
+    }
+    count_launch();
+}
+template <typename T, int CPT>
+static void allow_cluster() {
+    cudaFuncSetAttribute(k_coarse_cluster<T, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLUSTER_SMEM_LIMIT);
+    cudaFuncSetAttribute(k_coarse_cluster<T, CPT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+// The kernels' shared-memory limit and cluster size on the current device: set once a device, when its first multigrid
+// problem is created (the attributes are the device's, and setting them is not captured).
+void configure_coarse_cluster() {
+    constexpr int MAX_DEVICES = 64;
+    static std::once_flag once[MAX_DEVICES];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    auto allow = [] {
+        allow_cluster<float, 1>();
+        allow_cluster<float, 2>();
+        allow_cluster<double, 1>();
+    };
+    if (dev < 0 || dev >= MAX_DEVICES) allow();
+    else std::call_once(once[dev], allow);
+}
+
+template bool cluster_plan<float>(ClusterLevels<float>&);
+template bool cluster_plan<double>(ClusterLevels<double>&);
+template void launch_coarse_cluster<float>(const ClusterLevels<float>&, const int*, cudaStream_t);
+template void launch_coarse_cluster<double>(const ClusterLevels<double>&, const int*, cudaStream_t);
+
+}  // namespace nk

@@ -62,7 +62,7 @@ void launch_impose_prescribed(const DevGrid<double>& g, double2* x, const double
 // inverse diagonal (Jacobi) of the fine grid
 void launch_inverse_diagonal(const OpView<double>& o, double2* invd, cudaStream_t s);
 template <typename T>
-void launch_inverse_row_sum(const OpView<T>& o, typename Vec2<T>::type* irs, cudaStream_t s);
+void launch_inverse_row_sum(const OpView<T>& o, typename Vec2<T>::type* irs, cudaStream_t s, typename Vec4<T>::type* st = nullptr);
 
 struct CGView {
     OpView<double> o;
@@ -349,12 +349,14 @@ struct LevelView {
     typename Vec2<T>::type* q;
     T* t;                            // line-smoother scratch (one T per cell)
     const typename Vec2<T>::type* irs;  // inverse ℓ1 row sums
+    const typename Vec4<T>::type* st = nullptr;   // -w A by rows, w = irs (a level that nk_cluster.cu may hold, or null)
     int cx, cy;                      // coarsening factor from the finer level (1 or 2)
 };
 template <typename T>
 __device__ __forceinline__ void rebase(LevelView<T>& L, long long d) {
     rebase(L.o, d);
     shift_ptr(L.x, d); shift_ptr(L.x2, d); shift_ptr(L.b, d); shift_ptr(L.q, d); shift_ptr(L.t, d); shift_ptr(L.irs, d);
+    shift_ptr(L.st, d);
 }
 // Mean device time in ms of `repeats` launches of one level's sweep (kind STRIP_SMOOTH, x -> x2) or residual
 // (STRIP_RESIDUAL, into q) with walks of `rows` rows; negative if a CUDA call failed (the strip autotuner)
@@ -371,15 +373,6 @@ void launch_smooth_point(const LevelView<T>& L, const typename Vec2<T>::type* x_
 // the first two sweeps from a zero guess in one pass (x1 = b / rowsum formed on load)
 template <typename T>
 void launch_smooth_first2(const LevelView<T>& L, typename Vec2<T>::type* x_out, const int* done, cudaStream_t s);
-// the coarsest level's sweeps in one thread block with the level in shared memory (x_in = nullptr: from zero;
-// from_zero: the first sweep is x = b / rowsum); result in x_out
-template <typename T>
-bool coarsest_smem_fits(const LevelView<T>& L, int plane);
-template <typename T>
-void configure_coarsest_smem();
-template <typename T>
-void launch_coarsest_smem(const LevelView<T>& L, int plane, const typename Vec2<T>::type* x_in, int sweeps, int from_zero,
-                          typename Vec2<T>::type* x_out, const int* done, cudaStream_t s);
 // q = A x (line smoother first half) or q = b - A x (residual)
 template <typename T>
 void launch_level_apply(const LevelView<T>& L, const typename Vec2<T>::type* x, typename Vec2<T>::type* q, int residual,
@@ -411,6 +404,22 @@ struct CoarseLevels {
 };
 template <typename T>
 void launch_coarse_vcycle(const CoarseLevels<T>& C, const int* done, cudaStream_t s);
+// The levels from lv[0] down to the coarsest, lv[n - 1], run by one thread-block cluster (nk_cluster.cu).
+template <typename T>
+struct ClusterLevels {
+    LevelView<T> lv[MAX_COARSE_LEVELS];
+    int rows[MAX_COARSE_LEVELS], off[MAX_COARSE_LEVELS];   // rows per CTA, offset of the level's two buffers (pairs)
+    unsigned magic[MAX_COARSE_LEVELS];                     // j / rows by multiplication
+    int n, sweeps, coarsest;                               // levels, smoothing_sweeps, coarsest_sweeps
+    int ctas, cells, total;                                // cluster size, cells per thread (1, 2), pairs of shared memory
+};
+// Cells of the largest level that a cluster holds: 16 CTAs x 512 threads x 2 cells in FP32 (1 cell in FP64)
+constexpr long long cluster_limit_cells(bool fp64) { return fp64 ? 8192 : 16384; }
+template <typename T>
+bool cluster_plan(ClusterLevels<T>& C);   // fills rows, off, ctas, cells and total; false if the levels do not fit
+template <typename T>
+void launch_coarse_cluster(const ClusterLevels<T>& C, const int* done, cudaStream_t s);
+void configure_coarse_cluster();
 // FP64 <-> FP32 conversions of vectors and of the coefficient record
 void launch_to_float(const DevGrid<double>& g, const double2* src, float2* dst, const int* done, cudaStream_t s);
 void launch_to_double(const DevGrid<double>& g, const float2* src, double2* dst, const int* done, cudaStream_t s);

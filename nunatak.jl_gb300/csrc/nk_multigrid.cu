@@ -9,57 +9,11 @@
 // does a whole Jacobi sweep (the reference computes q = A x in one launch, then x += (b - q) / rowsum).
 // Every kernel takes the conjugate-gradient `done` flag and returns once the solve has stopped.
 #include "nk_kernels.cuh"
+#include "nk_transfer.cuh"
 
 namespace nk {
 
 __device__ __forceinline__ bool stopped(const int* done) { return done && *(volatile const int*)done; }
-
-// ---- restriction / prolongation index rules (0-based) ------------------------------------------------------
-__device__ __forceinline__ void offsets(bool face, int c, int& a0, int& a1) {
-    if (c == 1) { a0 = 0; a1 = 0; } else if (face) { a0 = -1; a1 = 1; } else { a0 = -1; a1 = 2; }
-}
-__device__ __forceinline__ int wrapn(int i, int n) { int r = i % n; return r < 0 ? r + n : r; }
-// restriction_index (multigrid_preconditioner.jl:268-271)
-__device__ __forceinline__ int ridx(int I, int a, int Nf, bool periodic, bool face, int c) {
-    if (c == 1) return I;
-    int i = 2 * I + a;
-    if (periodic) return wrapn(i, Nf);
-    if (face) return i < 0 ? 0 : i;
-    return i < 0 ? 0 : (i > Nf - 1 ? Nf - 1 : i);
-}
-// restriction_weight (:273-283)
-template <typename T>
-__device__ __forceinline__ T rweight(int I, int a, int Nc, bool periodic, bool face, int c) {
-    if (c == 1) return T(1);
-    if (face) {
-        if (!periodic && 2 * I + a < 0) return T(0);
-        return a == 0 ? T(1) : T(1) / T(2);
-    }
-    T w = (a == 0 || a == 1) ? T(3) / T(4) : T(1) / T(4);
-    if (periodic) return w;
-    bool outside = (I == 0 && a == -1) || (I == Nc - 1 && a == 2);
-    bool folded = (I == 0 && a == 0) || (I == Nc - 1 && a == 1);
-    w = w + (folded ? T(1) / T(4) : T(0));
-    return outside ? T(0) : w;
-}
-// parents (:286-305)
-template <typename T>
-__device__ __forceinline__ void parents(int i, int Nc, bool periodic, bool face, int c, int& I1, int& I2, T& w1, T& w2) {
-    if (c == 1) { I1 = i; I2 = i; w1 = T(1); w2 = T(0); return; }
-    int I = i / 2;
-    bool odd1 = (i % 2) == 0;   // the 1-based index i + 1 is odd
-    if (face) {
-        int up = periodic ? wrapn(I + 1, Nc) : I + 1;
-        I1 = I; I2 = odd1 ? I : up;
-        w1 = odd1 ? T(1) : T(1) / T(2);
-        w2 = odd1 ? T(0) : T(1) / T(2);
-    } else {
-        int Ip = odd1 ? I - 1 : I + 1;
-        I1 = I;
-        I2 = periodic ? wrapn(Ip, Nc) : (Ip < 0 ? 0 : (Ip > Nc - 1 ? Nc - 1 : Ip));
-        w1 = T(3) / T(4); w2 = T(1) / T(4);
-    }
-}
 
 // ---- coarse coefficients (_coarsen_coefficients!, :331-344), accumulated in FP64 ---------------------------------
 template <typename T, typename TF>
@@ -554,193 +508,6 @@ void launch_copy_plane(const DevGrid<T>& g, typename Vec2<T>::type* dst, const t
     k_copy_plane<T><<<grid, 256, 0, s>>>(g, dst, src, n, done); count_launch();
 }
 
-// ---- the coarsest level in shared memory ----------------------------------------------------------------------
-// The coarsest level takes many sweeps (20 by default) of a grid of about a thousand cells: as separate launches
-// each sweep is a few microseconds of latency on the solve's critical path.  For FP32 levels of at most 1024 cells
-// one block of 1024 threads runs every sweep on-chip, each thread owning one cell.  Everything that does not
-// change between sweeps (shared-memory indices, mask tests, metrics, 2η, η̄Hᶠᶠ times the wall factor, Az β, b,
-// 1/rowsum) is computed once into registers; a sweep (1) builds the masked velocities (interior_u / interior_v)
-// of the current x on the grid padded by one point (wrapped when periodic, zero outside a Bounded range),
-// (2) computes every centre's Δy Txx, Δx Tyy and every corner's shear once (the expressions of the column-marching
-// apply), (3) combines them into x' = x + (b - A x) / rowsum and (4) stores x', with block barriers between the
-// phases.  (A variant holding several cells per thread, with the constants re-read each sweep, was slower than
-// separate launches, in FP64 as well; those levels keep the launches.)
-template <typename T>
-__global__ void __launch_bounds__(1024, 1)
-    k_coarsest_smem_1(LevelView<T> L, int plane, const typename Vec2<T>::type* __restrict__ xin, int sweeps, int from_zero,
-                      typename Vec2<T>::type* xout, const int* done) {
-    NK_BATCH_ENTER(L.o.g, L, xin, xout, done)
-    if (stopped(done)) return;
-    using V2 = typename Vec2<T>::type;
-    const DevGrid<T>& g = L.o.g;
-    const int Nx = g.Nx, Ny = g.Ny, tid = threadIdx.x, nt = blockDim.x;
-    const int n = Nx * Ny, ncorner = (Nx + 1) * (Ny + 1), PW = Nx + 2, npad = (Nx + 2) * (Ny + 2);
-    extern __shared__ __align__(32) unsigned char smem[];
-    V2* x = reinterpret_cast<V2*>(smem);       // plane
-    V2* st = x + plane;                        // n
-    V2* M = st + n;                            // npad
-    T* sh = reinterpret_cast<T*>(M + npad);    // ncorner
-    for (int k = tid; k < plane; k += nt) {
-        V2 z;
-        z.x = T(0);
-        z.y = T(0);
-        x[k] = xin ? xin[k] : z;
-    }
-    // padded masked points of this thread: e0 = tid, e1 = tid + nt
-    int pk[2];
-    uint8_t pf[2];                             // bit 0: u taken, bit 1: v taken
-#pragma unroll
-    for (int a = 0; a < 2; ++a) {
-        int e = tid + a * nt;
-        pk[a] = 0;
-        pf[a] = 0;
-        if (e < npad) {
-            int i = e % PW - 1, j = e / PW - 1;
-            bool uok = (g.px || (i >= 0 && i <= Nx)) && !g.out_y(j);
-            bool vok = !g.out_x(i) && (g.py || (j >= 0 && j <= Ny));
-            if (uok || vok) {
-                int k = g.idx(g.px ? g.wrap(i, Nx) : i, g.py ? g.wrap(j, Ny) : j);
-                uint8_t mk = L.o.mask[k];
-                pk[a] = k;
-                pf[a] = (uok && !(mk & U_INACTIVE) ? 1 : 0) | (vok && !(mk & V_INACTIVE) ? 2 : 0);
-            }
-        }
-    }
-    // the cell c = tid: centre stress constants and the combination constants
-    const bool has_cell = tid < n;
-    int ci = has_cell ? tid % Nx : 0, cj = has_cell ? tid / Nx : 0;
-    int kc = g.idx(ci, cj);
-    T c_rdxc = T(0), c_rdyc = T(0), c_dyc = T(0), c_dxc = T(0), c_2eta = T(0), c_dxf = T(0), c_dyf = T(0), azbu = T(0), azbv = T(0);
-    V2 bb, ww;
-    bb.x = bb.y = ww.x = ww.y = T(0);
-    uint8_t c_mask = 0;
-    int sw_idx = -1, ss_idx = -1, t01_idx = 0, t10_idx = 0;
-    if (has_cell) {
-        c_rdxc = g.rdxc[ci]; c_rdyc = g.rdyc[cj]; c_dyc = g.dyc[cj]; c_dxc = g.dxc[ci];
-        c_dxf = g.dxf[ci]; c_dyf = g.dyf[cj];
-        typename Vec4<T>::type cc = L.o.coef[kc];
-        c_2eta = T(2) * cc.x;
-        azbu = (c_dxf * c_dyc) * cc.z;
-        azbv = (c_dxc * c_dyf) * cc.w;
-        bb = L.b[kc];
-        ww = L.irs[kc];
-        c_mask = L.o.mask[kc];
-        if (ci > 0) sw_idx = tid - 1; else if (g.px) sw_idx = cj * Nx + Nx - 1;
-        if (cj > 0) ss_idx = tid - Nx; else if (g.py) ss_idx = (Ny - 1) * Nx + ci;
-        int jn = (g.py && cj + 1 == Ny) ? 0 : cj + 1, ie = (g.px && ci + 1 == Nx) ? 0 : ci + 1;
-        t01_idx = jn * (Nx + 1) + ci;
-        t10_idx = cj * (Nx + 1) + ie;
-    }
-    // corners of this thread: f0 = tid, f1 = tid + nt
-    int fm[2][3];                              // padded indices of (i, j), (i, j - 1), (i - 1, j)
-    T f_rdyf[2], f_rdxf[2], f_eta[2];
-#pragma unroll
-    for (int a = 0; a < 2; ++a) {
-        int f = tid + a * nt;
-        fm[a][0] = fm[a][1] = fm[a][2] = 0;
-        f_rdyf[a] = f_rdxf[a] = f_eta[a] = T(0);
-        if (f < ncorner) {
-            int i = f % (Nx + 1), j = f / (Nx + 1);
-            fm[a][0] = (j + 1) * PW + i + 1;
-            fm[a][1] = j * PW + i + 1;
-            fm[a][2] = (j + 1) * PW + i;
-            f_rdyf[a] = g.rdyf[j];
-            f_rdxf[a] = g.rdxf[i];
-            T eta = L.o.coef[g.ff_idx(i, j)].y;
-            f_eta[a] = g.peripheral_ff(i, j) ? eta * L.o.wall_factor : eta;
-        }
-    }
-    __syncthreads();
-    for (int sweep = 0; sweep < sweeps; ++sweep) {
-        V2 xx = x[kc], nv;
-        if (from_zero && sweep == 0) {
-            nv.x = bb.x * ww.x;
-            nv.y = bb.y * ww.y;
-        } else {
-#pragma unroll
-            for (int a = 0; a < 2; ++a) {
-                if (tid + a * nt < npad) {
-                    V2 v = x[pk[a]], m;
-                    m.x = (pf[a] & 1) ? v.x : T(0);
-                    m.y = (pf[a] & 2) ? v.y : T(0);
-                    M[tid + a * nt] = m;
-                }
-            }
-            __syncthreads();
-            if (has_cell) {
-                int p0 = (cj + 1) * PW + ci + 1;
-                V2 m0 = M[p0], me = M[p0 + 1], mn = M[p0 + PW];
-                T exx = (me.x - m0.x) * c_rdxc;
-                T eyy = (mn.y - m0.y) * c_rdyc;
-                V2 sv;
-                sv.x = c_dyc * (c_2eta * (T(2) * exx + eyy));
-                sv.y = c_dxc * (c_2eta * (T(2) * eyy + exx));
-                st[tid] = sv;
-            }
-#pragma unroll
-            for (int a = 0; a < 2; ++a) {
-                if (tid + a * nt < ncorner) {
-                    V2 m0 = M[fm[a][0]], ms = M[fm[a][1]], mw = M[fm[a][2]];
-                    T e = (m0.x - ms.x) * f_rdyf[a] + (m0.y - mw.y) * f_rdxf[a];
-                    sh[tid + a * nt] = f_eta[a] * e;
-                }
-            }
-            __syncthreads();
-            if (has_cell) {
-                V2 s0 = st[tid], sw, ss;
-                sw.x = sw.y = ss.x = ss.y = T(0);
-                if (sw_idx >= 0) sw = st[sw_idx];
-                if (ss_idx >= 0) ss = st[ss_idx];
-                T t00 = sh[cj * (Nx + 1) + ci], t01 = sh[t01_idx], t10 = sh[t10_idx];
-                T divu = (s0.x - sw.x) + (c_dxf * t01 - c_dxf * t00);
-                T divv = (s0.y - ss.y) + (c_dyf * t10 - c_dyf * t00);
-                V2 q;
-                q.x = (c_mask & U_IDENTITY) ? xx.x : azbu * xx.x - divu;
-                q.y = (c_mask & V_IDENTITY) ? xx.y : azbv * xx.y - divv;
-                nv.x = xx.x + (bb.x - q.x) * ww.x;
-                nv.y = xx.y + (bb.y - q.y) * ww.y;
-            }
-        }
-        __syncthreads();
-        if (has_cell) x[kc] = nv;
-        __syncthreads();
-    }
-    if (has_cell) xout[kc] = x[kc];
-}
-
-// True when the level can run in one block: FP32, at most one cell, one corner beyond the cells and two padded
-// points per thread.
-template <typename T>
-bool coarsest_smem_fits(const LevelView<T>& L, int plane) {
-    (void)plane;
-    int nx = L.o.g.Nx, ny = L.o.g.Ny;
-    return sizeof(T) == 4 && nx * ny <= 1024 && (nx + 2) * (ny + 2) <= 2048 && (nx + 1) * (ny + 1) <= 2048;
-}
-template <typename T>
-void configure_coarsest_smem() {
-    if constexpr (sizeof(T) == 4) {
-        static bool done = [] {
-            int dev = 0, v = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-            cudaFuncSetAttribute(k_coarsest_smem_1<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-            return true;
-        }();
-        (void)done;
-    }
-}
-template <typename T>
-void launch_coarsest_smem(const LevelView<T>& L, int plane, const typename Vec2<T>::type* x_in, int sweeps, int from_zero,
-                          typename Vec2<T>::type* x_out, const int* done, cudaStream_t s) {
-    if constexpr (sizeof(T) == 4) {
-        int nx = L.o.g.Nx, ny = L.o.g.Ny;
-        size_t bytes = (size_t)plane * sizeof(typename Vec2<T>::type) + (size_t)nx * ny * sizeof(typename Vec2<T>::type) +
-                       (size_t)(nx + 2) * (ny + 2) * sizeof(typename Vec2<T>::type) + (size_t)(nx + 1) * (ny + 1) * sizeof(T);
-        k_coarsest_smem_1<T><<<dim3(1, 1, batch_slots()), 1024, bytes, s>>>(L, plane, x_in, sweeps, from_zero, x_out, done);
-        count_launch();
-    }
-}
-
 // ---- fused coarse V-cycle: one thread block runs every remaining level ----------------------------------------
 // The coarse levels of a V-cycle are a few thousand cells or less, where a grid-wide launch per sweep costs more
 // than the sweep.  One 1024-thread block walks the rest of v_cycle! (:144-163) level by level — smooth, residual,
@@ -823,9 +590,6 @@ void launch_coarse_vcycle(const CoarseLevels<T>& C, const int* done, cudaStream_
 #define NK_INSTANTIATE(T)                                                                                                   \
     template void launch_smooth_point<T>(const LevelView<T>&, const Vec2<T>::type*, Vec2<T>::type*, int, const int*, cudaStream_t); \
     template void launch_smooth_first2<T>(const LevelView<T>&, Vec2<T>::type*, const int*, cudaStream_t); \
-    template bool coarsest_smem_fits<T>(const LevelView<T>&, int); \
-    template void configure_coarsest_smem<T>(); \
-    template void launch_coarsest_smem<T>(const LevelView<T>&, int, const Vec2<T>::type*, int, int, Vec2<T>::type*, const int*, cudaStream_t); \
     template void launch_level_apply<T>(const LevelView<T>&, const Vec2<T>::type*, Vec2<T>::type*, int, const int*, cudaStream_t);  \
     template void launch_line_relax<T>(const LevelView<T>&, Vec2<T>::type*, int, const int*, cudaStream_t);                        \
     template void launch_restrict<T>(const LevelView<T>&, const LevelView<T>&, const Vec2<T>::type*, Vec2<T>::type*, Vec2<T>::type*, \

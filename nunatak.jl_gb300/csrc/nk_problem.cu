@@ -146,6 +146,7 @@ struct Level {
     typename Vec4<T>::type* coef = nullptr;
     uint8_t* mask = nullptr;
     typename Vec2<T>::type* irs = nullptr;
+    typename Vec4<T>::type* st = nullptr;   // stencil rows of a level that the cluster kernel holds
     typename Vec2<T>::type *x = nullptr, *x2 = nullptr, *b = nullptr, *q = nullptr;
     T* t = nullptr;
     DevGrid<T> g{};
@@ -289,7 +290,7 @@ struct nk_problem {
         v.o.coef = L.coef;
         v.o.mask = L.mask;
         v.o.wall_factor = pd.side_walls == NK_NO_SLIP ? TT(2) : TT(0);
-        v.x = L.x; v.x2 = L.x2; v.b = L.b; v.q = L.q; v.t = L.t; v.irs = L.irs;
+        v.x = L.x; v.x2 = L.x2; v.b = L.b; v.q = L.q; v.t = L.t; v.irs = L.irs; v.st = L.st;
         v.cx = L.cx; v.cy = L.cy;
         return v;
     }
@@ -328,7 +329,8 @@ template <typename T>
 static size_t metric_len(const Level<T>& L, int axis) { return (size_t)((axis == 0 ? L.Nx : L.Ny) + 2 * METRIC_PAD + 2); }
 
 template <typename T>
-static void reserve_level(Arena& A, Level<T>& L, std::vector<std::pair<void**, size_t>>& slots, bool own_coef, bool own_xb) {
+static void reserve_level(Arena& A, Level<T>& L, std::vector<std::pair<void**, size_t>>& slots, bool own_coef, bool own_xb,
+                          bool stencils) {
     size_t pl = L.plane();
     size_t mlen = 4 * (metric_len(L, 0) + metric_len(L, 1));
     slots.push_back({(void**)&L.metrics, A.reserve(mlen * sizeof(T))});
@@ -337,6 +339,7 @@ static void reserve_level(Arena& A, Level<T>& L, std::vector<std::pair<void**, s
         slots.push_back({(void**)&L.mask, A.reserve(pl)});
     }
     slots.push_back({(void**)&L.irs, A.reserve(pl * sizeof(typename Vec2<T>::type))});
+    if (stencils) slots.push_back({(void**)&L.st, A.reserve(5 * (size_t)L.Nx * L.Ny * sizeof(typename Vec4<T>::type))});
     if (own_xb) {
         slots.push_back({(void**)&L.x, A.reserve(pl * sizeof(typename Vec2<T>::type))});
         slots.push_back({(void**)&L.b, A.reserve(pl * sizeof(typename Vec2<T>::type))});
@@ -344,6 +347,12 @@ static void reserve_level(Arena& A, Level<T>& L, std::vector<std::pair<void**, s
     slots.push_back({(void**)&L.x2, A.reserve(pl * sizeof(typename Vec2<T>::type))});
     slots.push_back({(void**)&L.q, A.reserve(pl * sizeof(typename Vec2<T>::type))});
     slots.push_back({(void**)&L.t, A.reserve(pl * sizeof(T))});
+}
+
+// Levels that the cluster kernel can hold keep their stencil rows (plan_cluster says which of them it does hold).
+template <typename T>
+static bool cluster_candidate(const nk_problem* P, const Level<T>& L) {
+    return P->sd.smoother == NK_SMOOTHER_POINT_JACOBI && (long long)L.Nx * L.Ny <= cluster_limit_cells(sizeof(T) == 8);
 }
 
 template <typename T>
@@ -479,11 +488,11 @@ static void build(nk_problem* P, bool dry = false) {
     slots.push_back({(void**)&P->rate_params, A.reserve(16 * sizeof(double))});
     if (P->precond == NK_PRECONDITIONER_MULTIGRID) {
         if (P->mixed) {
-            for (int l = 0; l <= P->nlevels; ++l) reserve_level(A, P->lv32[l], slots, true, true);
+            for (int l = 0; l <= P->nlevels; ++l) reserve_level(A, P->lv32[l], slots, true, true, cluster_candidate(P, P->lv32[l]));
         } else {
             // level 0 is the fine grid: coefficients, mask and vectors are the fine ones (x = z, b = r)
-            reserve_level(A, P->lv64[0], slots, false, false);
-            for (int l = 1; l <= P->nlevels; ++l) reserve_level(A, P->lv64[l], slots, true, true);
+            reserve_level(A, P->lv64[0], slots, false, false, cluster_candidate(P, P->lv64[0]));
+            for (int l = 1; l <= P->nlevels; ++l) reserve_level(A, P->lv64[l], slots, true, true, cluster_candidate(P, P->lv64[l]));
         }
     }
     if (dry) return;   // sizing only: A.size is the device footprint
@@ -530,24 +539,24 @@ static void update_preconditioner(nk_problem* P) {
     if (!P->mixed) {
         auto& lv = P->lv64;
         LevelView<double> v0 = P->level_view(lv[0]);
-        launch_inverse_row_sum<double>(v0.o, lv[0].irs, s);
+        launch_inverse_row_sum<double>(v0.o, lv[0].irs, s, lv[0].st);
         for (int l = 1; l <= P->nlevels; ++l) {
             LevelView<double> v = P->level_view(lv[l]);
             launch_coarsen<double, double>(v, lv[l - 1].g, lv[l - 1].coef, lv[l].coef, s);
             launch_mask<double>(v.o, lv[l].mask, s);
-            launch_inverse_row_sum<double>(v.o, lv[l].irs, s);
+            launch_inverse_row_sum<double>(v.o, lv[l].irs, s, lv[l].st);
         }
     } else {
         auto& lv = P->lv32;
         launch_coef_to_float(P->fine.g, P->fine.coef, lv[0].coef, s);
         LevelView<float> v0 = P->level_view(lv[0]);
-        launch_inverse_row_sum<float>(v0.o, lv[0].irs, s);
+        launch_inverse_row_sum<float>(v0.o, lv[0].irs, s, lv[0].st);
         for (int l = 1; l <= P->nlevels; ++l) {
             LevelView<float> v = P->level_view(lv[l]);
             if (l == 1) launch_coarsen<float, double>(v, P->fine.g, P->fine.coef, lv[1].coef, s);
             else launch_coarsen<float, float>(v, lv[l - 1].g, lv[l - 1].coef, lv[l].coef, s);
             launch_mask<float>(v.o, lv[l].mask, s);
-            launch_inverse_row_sum<float>(v.o, lv[l].irs, s);
+            launch_inverse_row_sum<float>(v.o, lv[l].irs, s, lv[l].st);
         }
     }
     NK_CHECK_LAUNCH();
@@ -565,8 +574,8 @@ static int coarse_cells_limit() {
     return limit;
 }
 
-// NK_COARSEST_SMEM=0 runs the coarsest level's sweeps as separate launches instead of one shared-memory block.
-static bool coarsest_in_shared_memory() {
+// NK_COARSEST_SMEM=0 runs the coarse levels as grid-wide launches instead of in one thread-block cluster.
+static bool coarse_levels_in_a_cluster() {
     static bool on = [] {
         const char* e = std::getenv("NK_COARSEST_SMEM");
         return !(e && std::atoi(e) == 0);
@@ -591,6 +600,21 @@ static bool use_graphs(const nk_problem* P) {
         return !(e && e[0] == '0');
     }();
     return on && !(P->sd.flags & NK_SOLVER_HOST_LOOP);
+}
+
+// Whether the levels from l down run in one cluster (k_coarse_cluster), and how: levels whose rows, split over the
+// cluster's CTAs, leave a thread at most two cells in FP32 (16384 cells on a level of enough rows) or one in FP64 (8192).
+// One cell more a thread spills; above the limit the grid-wide launches, which use every SM, are the faster ones.
+template <typename T>
+static bool plan_cluster(nk_problem* P, std::vector<Level<T>>& lv, int l, ClusterLevels<T>& C) {
+    if (P->sd.smoother != NK_SMOOTHER_POINT_JACOBI || !coarse_levels_in_a_cluster()) return false;
+    if (P->nlevels - l + 1 > MAX_COARSE_LEVELS) return false;
+    C = ClusterLevels<T>{};
+    C.n = P->nlevels - l + 1;
+    for (int k = 0; k < C.n; ++k) C.lv[k] = P->level_view(lv[l + k]);
+    C.sweeps = C.n > 1 ? P->sd.smoothing_sweeps : 1;   // a coarsest level alone takes no smoothing sweeps
+    C.coarsest = P->sd.coarsest_sweeps;
+    return cluster_plan<T>(C);
 }
 
 // Buffer that receives the first of `sweeps` point sweeps started from zero, so that the last lands in L.x.
@@ -657,17 +681,13 @@ static void v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* 
         return;
     }
     Level<T>& L = lv[l];
+    ClusterLevels<T> cluster;
+    if (!first_done && plan_cluster(P, lv, l, cluster)) {
+        launch_coarse_cluster<T>(cluster, done, s);
+        return;
+    }
     if (l == P->nlevels) {
-        int sweeps = P->sd.coarsest_sweeps;
-        LevelView<T> v = P->level_view(L);
-        int plane = (int)L.plane();
-        if (coarsest_in_shared_memory() && P->sd.smoother == NK_SMOOTHER_POINT_JACOBI && sweeps > 0 &&
-            coarsest_smem_fits<T>(v, plane)) {
-            if (first_done) launch_coarsest_smem<T>(v, plane, first_sweep_target(L, sweeps), sweeps - 1, 0, L.x, done, s);
-            else launch_coarsest_smem<T>(v, plane, nullptr, sweeps, 1, L.x, done, s);
-            return;
-        }
-        smooth(P, L, sweeps, true, done, first_done);
+        smooth(P, L, P->sd.coarsest_sweeps, true, done, first_done);
         return;
     }
     smooth(P, L, P->sd.smoothing_sweeps, true, done, first_done);
@@ -677,7 +697,7 @@ static void v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* 
     LevelView<T> c = P->level_view(N);
     bool fuse_first = (l + 1 != lc) && P->sd.smoother == NK_SMOOTHER_POINT_JACOBI;
     int next_sweeps = (l + 1 == P->nlevels) ? P->sd.coarsest_sweeps : P->sd.smoothing_sweeps;
-    fuse_first = fuse_first && next_sweeps > 0;
+    fuse_first = fuse_first && next_sweeps > 0 && !plan_cluster(P, lv, l + 1, cluster);
     launch_restrict<T>(c, v, L.q, N.b, fuse_first ? first_sweep_target(N, next_sweeps) : nullptr, done, s);
     v_cycle(P, lv, l + 1, done, fuse_first);
     launch_prolongate<T>(v, c, L.x, N.x, done, s);
@@ -1358,8 +1378,7 @@ static nk_status problem_create(nk_context* ctx, const nk_grid_desc* grid, const
         NK_CUDA(cudaEventCreate(&P->ev0));
         NK_CUDA(cudaEventCreate(&P->ev1));
         build(P);
-        configure_coarsest_smem<float>();   // shared-memory limit of the coarsest-level kernel, once, outside any capture
-        configure_coarsest_smem<double>();
+        if (P->precond == NK_PRECONDITIONER_MULTIGRID) configure_coarse_cluster();   // outside any capture
         P->gd.x_faces = nullptr; P->gd.y_faces = nullptr; P->gd.sigma_faces = nullptr;   // no pointer kept after the call
         NK_CUDA(cudaStreamSynchronize(P->stream));
     });

@@ -147,9 +147,42 @@ void launch_inverse_diagonal(const OpView<double>& o, double2* invd, cudaStream_
     k_inverse_diagonal<<<d.grid, d.block, 0, s>>>(o, invd); count_launch();
 }
 
+// The rows of -w A at (i, j), w = (1/rowsum)u, (1/rowsum)v: five own-component and four cross couplings of each
+// component (ssa_operator.jl:69-89 expanded by its operands; the metric quotients that cancel are left out).
+// Planes of Nx Ny records, dense: (uE, uW, uN, uS), (uC, vC, vN, vNW, vW) of the u row in st[0] and st[1] with vW in
+// st[4].x, the v row (vN, vS, vE, vW), (vC, uC, uE, uSE, uS) in st[2], st[3] and st[4].y, and w in st[4].zw.
 template <typename T>
-__global__ void k_inverse_row_sum(OpView<T> o, typename Vec2<T>::type* irs) {
-    NK_BATCH_ENTER(o.g, o, irs)
+__device__ __forceinline__ void stencil_rows(const OpView<T>& o, int i, int j, uint8_t m, typename Vec2<T>::type w,
+                                             typename Vec4<T>::type* st) {
+    using V4 = typename Vec4<T>::type;
+    const DevGrid<T>& g = o.g;
+    V4 rc = o.coef[g.idx(i, j)];
+    T etaw = eta_c(o, i - 1, j), etas = eta_c(o, i, j - 1);
+    T c00 = corner_factor(o, i, j) * rc.y, c01 = corner_factor(o, i, j + 1) * eta_ff(o, i, j + 1);
+    T c10 = corner_factor(o, i + 1, j) * eta_ff(o, i + 1, j);
+    T dxc = g.dxc[i], dyc = g.dyc[j], dxf = g.dxf[i], dyf = g.dyf[j];
+    T c00x = c00 * (dxf * g.rdyf[j]), c01x = c01 * (dxf * g.rdyf[j + 1]);
+    T c00y = c00 * (dyf * g.rdxf[i]), c10y = c10 * (dyf * g.rdxf[i + 1]);
+    T a1c = x_normal_diagonal(o, i, j), a1w = x_normal_diagonal(o, i - 1, j);
+    T a3c = y_normal_diagonal(o, i, j), a3s = y_normal_diagonal(o, i, j - 1);
+    T e2 = T(2) * rc.x, e2w = T(2) * etaw, e2s = T(2) * etas;
+    T wu = (m & U_IDENTITY) ? T(0) : w.x, wv = (m & V_IDENTITY) ? T(0) : w.y;   // an identity row has its centre alone
+    V4 a, b, f, h, r;
+    a.x = wu * a1c; a.y = wu * a1w; a.z = wu * c01x; a.w = wu * c00x;
+    b.x = (m & U_IDENTITY) ? -w.x : -wu * (dxf * dyc * rc.z + a1c + a1w + c01x + c00x);
+    b.y = -wu * (e2 + c00); b.z = wu * (e2 + c01); b.w = -wu * (e2w + c01);
+    f.x = wv * a3c; f.y = wv * a3s; f.z = wv * c10y; f.w = wv * c00y;
+    h.x = (m & V_IDENTITY) ? -w.y : -wv * (dxc * dyf * rc.w + a3c + a3s + c10y + c00y);
+    h.y = -wv * (e2 + c00); h.z = wv * (e2 + c10); h.w = -wv * (e2s + c10);
+    r.x = wu * (e2w + c00); r.y = wv * (e2s + c00); r.z = w.x; r.w = w.y;
+    const int n = g.Nx * g.Ny;
+    st += j * g.Nx + i;
+    st[0] = a; st[n] = b; st[2 * n] = f; st[3 * n] = h; st[4 * n] = r;
+}
+
+template <typename T>
+__global__ void k_inverse_row_sum(OpView<T> o, typename Vec2<T>::type* irs, typename Vec4<T>::type* st) {
+    NK_BATCH_ENTER(o.g, o, irs, st)
     int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y;
     if (i >= o.g.Nx || j >= o.g.Ny) return;
     uint8_t m = o.mask[o.g.idx(i, j)];
@@ -157,14 +190,15 @@ __global__ void k_inverse_row_sum(OpView<T> o, typename Vec2<T>::type* irs) {
     r.x = (m & U_DIRICHLET) ? T(0) : T(1) / x_row_sum(o, i, j, m);
     r.y = (m & V_DIRICHLET) ? T(0) : T(1) / y_row_sum(o, i, j, m);
     irs[o.g.idx(i, j)] = r;
+    if (st) stencil_rows(o, i, j, m, r, st);
 }
 template <typename T>
-void launch_inverse_row_sum(const OpView<T>& o, typename Vec2<T>::type* irs, cudaStream_t s) {
+void launch_inverse_row_sum(const OpView<T>& o, typename Vec2<T>::type* irs, cudaStream_t s, typename Vec4<T>::type* st) {
     LaunchDims d = dims2d(o.g.Nx, o.g.Ny);
-    k_inverse_row_sum<T><<<d.grid, d.block, 0, s>>>(o, irs); count_launch();
+    k_inverse_row_sum<T><<<d.grid, d.block, 0, s>>>(o, irs, st); count_launch();
 }
-template void launch_inverse_row_sum<double>(const OpView<double>&, double2*, cudaStream_t);
-template void launch_inverse_row_sum<float>(const OpView<float>&, float2*, cudaStream_t);
+template void launch_inverse_row_sum<double>(const OpView<double>&, double2*, cudaStream_t, double4*);
+template void launch_inverse_row_sum<float>(const OpView<float>&, float2*, cudaStream_t, float4*);
 
 // ---- conjugate gradients ------------------------------------------------------------------------------------
 __device__ __forceinline__ int read_done(const SolverScalars* sc) { return *(volatile const int*)&sc->done; }

@@ -40,3 +40,51 @@ def test_geometry_at_the_grounding_line_and_the_margin(oracle_cls, gpu_cls, nx, 
     for g, w in zip(got, want):
         assert np.max(np.abs(g - w)) <= 1e-12 * max(1.0, np.max(np.abs(w)))
     assert 0 < np.mean(want[0] == 1.0) < 1 and np.any(want[0] == 0.0)
+
+
+# The coarse levels' cluster kernel (all levels from the first of at most 16384 cells, in FP32 and in FP64) against the
+# oracle's V-cycle: one CTA and many, rows that do not divide by the CTAs, CTAs without rows, axes that stop halving
+# before the other, periodic seams inside and across CTAs, odd and even sweep counts, no coarse level at all, and a top
+# level one row beyond the limit.  FP64: the sums of products against the oracle's differences round at 1e-16 of
+# rowsum |x| in each of the ~50 sweeps, so 1e-12 of the largest entry; FP32: the same with 6e-8, so 1e-4.
+@gpu
+@pytest.mark.parametrize("precision, tol", [("fp64", 1e-12), ("mixed", 1e-4)])
+@pytest.mark.parametrize("nx, ny, topology, sweeps, coarsest, minimum", [
+    (16, 16, ("Bounded", "Bounded"), 2, 20, 4),
+    (64, 34, ("Bounded", "Bounded"), 2, 20, 16),
+    (96, 40, ("Periodic", "Bounded"), 1, 7, 2),
+    (40, 96, ("Bounded", "Periodic"), 3, 6, 4),
+    (72, 48, ("Periodic", "Periodic"), 2, 1, 3),
+    (75, 45, ("Bounded", "Bounded"), 2, 20, 4),
+    (128, 128, ("Bounded", "Bounded"), 2, 20, 32),
+    (128, 130, ("Bounded", "Bounded"), 2, 20, 32),
+    (512, 18, ("Bounded", "Bounded"), 2, 5, 9),
+])
+def test_coarse_levels_in_a_cluster(oracle_cls, gpu_cls, nx, ny, topology, sweeps, coarsest, minimum, precision, tol):
+    rng = np.random.default_rng(nx + ny)
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 1.5e3), topology=topology)
+    mg = nk.StressBalanceMultigridPreconditioner(smoothing_sweeps=sweeps, coarsest_sweeps=coarsest, minimum_coarse_size=minimum)
+
+    def vcycle(cls, precision):
+        solver = nk.StressBalanceSolver(preconditioner=mg, precision=precision)
+        P = cls(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                                          stress_balance=nk.DepthIntegrated(side_walls=nk.NoSlipWalls()), velocity_solver=solver))
+        H = np.clip(1000.0 + 400.0 * np.random.default_rng(1).standard_normal((ny, nx)), 0.0, None)
+        H[:, : nx // 8] = 0.0   # ice free: identity rows
+        for n, a in (("H", H), ("bed", 10.0), ("C", 1e9), ("A", 3e-24)):
+            P.set(n, a)
+        P.compute_geometry()
+        r = np.random.default_rng(2)
+        P.set("u", 1e-5 * r.standard_normal(P.shape("u")))
+        P.set("v", 1e-5 * r.standard_normal(P.shape("v")))
+        P.update_coefficients()
+        z = P.precondition(ru, rv)
+        P.close()
+        return z
+
+    fx, fy = grid.face_count(0), grid.face_count(1)
+    ru, rv = 1e10 * rng.standard_normal((ny, fx)), 1e10 * rng.standard_normal((fy, nx))
+    got, want = vcycle(gpu_cls, precision), vcycle(oracle_cls, "fp64")
+    for g, w in zip(got, want):
+        g, w = g[:ny, :nx], w[:ny, :nx]
+        assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
