@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <type_traits>
 
 #include "../../include/nunatak_gb300.h"
 
@@ -119,17 +120,15 @@ struct SolverScalars {
     double r0, tol, rnorm;
     double picard_dd, picard_xx;   // ||x - x_prev||^2, ||x||^2
     double reltol, abstol;
-    int it, done, done_next, status;
+    int it, done, status;
     int fixed, iterations, maxiter, flexible;
     unsigned int ticket;           // last-block counter of the fused reductions
-    unsigned int ticket2;
     // Picard (picard.jl:63-90), evaluated on the device between the conjugate-gradient solves
     double p_reltol, p_abstol, p_D, p_X;
     int p_fixed, p_iterations, p_maxiter, p_it;
     int p_done, it_total, cg_unconverged;
     int r32_exp;                   // mixed precision: the FP32 residual in the V-cycle is r 2^-r32_exp, z = z32 2^r32_exp
     int r32_exp_next;              // exponent the next k_cg_update scales its residual with (from the latest ‖r‖)
-    int zold_exp;                  // mixed precision: z_old = zold32 2^zold_exp (the exponent of the z32 it copies)
 };
 
 // Binary exponent that brings a residual of norm `norm` near 1 before it is rounded to FP32.  Scaling by a power of
@@ -137,8 +136,11 @@ struct SolverScalars {
 // but right-hand sides of any magnitude stay clear of FP32 overflow and of its subnormal range.  Evaluated by
 // one thread per kernel (it costs FP64 instructions); the cells apply it with scale_pow2.
 __device__ __forceinline__ int residual_exponent(double norm) {
+    const int ex = (int)(((unsigned)__double2hiint(norm) >> 20) & 0x7ffu);   // a norm carries no sign
+    if (ex > 0 && ex < 0x7ff) return ex - 1023;   // a normal number, without FP64 instructions
     return (norm > 0.0 && isfinite(norm)) ? ilogb(norm) : 0;
 }
+__device__ __forceinline__ bool finite_bits(double x) { return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u; }
 
 // x 2^k by an integer add to the exponent field (no FP64 instruction): exact for normal x and results.  Zeros,
 // infinities and NaNs pass through; subnormal x and results below the normal range flush to a signed zero,
@@ -154,6 +156,26 @@ __device__ __forceinline__ double scale_pow2(double x, int k) {
     return __longlong_as_double(b + ((long long)k << 52));
 }
 
+// f 2^k in FP64 on the integer units (an F2F conversion takes the FP64 pipe): exact, the bits of scale_pow2((double)f, k).
+__device__ __forceinline__ double widen_pow2(float f, int k) {
+    const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
+    const int ex = (int)(a >> 23), e = ex + 896 + k;   // 896 = 1023 - 127
+    if (ex != 0 && ex != 255 && e > 0 && e < 2047)
+        return __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + (unsigned)((896 + k) << 20))), (int)(a << 29));
+    if (a == 0) return __hiloint2double((int)u, 0);
+    return scale_pow2((double)f, k);
+}
+// (float)(x 2^k) on the integer units, rounded to nearest even: the bits of (float)scale_pow2(x, k)
+__device__ __forceinline__ float narrow_pow2(double x, int k) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int ex = (int)((hi >> 20) & 0x7ffu), e = ex - 896 + k;
+    if (ex != 0 && ex != 0x7ff && ex + k > 0 && ex + k < 0x7ff && e > 0 && e < 254) {
+        const unsigned m = ((unsigned)e << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29), rest = lo & 0x1fffffffu;
+        return __uint_as_float((hi & 0x80000000u) | (m + ((rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) ? 1u : 0u)));
+    }
+    return (float)scale_pow2(x, k);
+}
+
 // ---- warp / block reductions (fixed order, so results do not depend on scheduling) --------------------
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
@@ -162,68 +184,80 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
-// Sum over the block of up to two values; result valid in thread 0.  `sh` holds 2 * 32 doubles.
-__device__ __forceinline__ void block_sum2(double& a, double& b, double* sh) {
-    int lane = threadIdx.x + threadIdx.y * blockDim.x;
-    int w = lane >> 5, l = lane & 31;
-    int nw = (blockDim.x * blockDim.y + 31) >> 5;
-    a = warp_sum(a);
-    b = warp_sum(b);
-    if (l == 0) { sh[w] = a; sh[32 + w] = b; }
+// Sums over a block of at most 256 threads of NV values (1 or 2); the results are valid in every thread.  One FP64
+// instruction of a warp takes 64 cycles when nothing overlaps it and 19 of the SM's FP64 pipe otherwise, so the threads'
+// values meet in shared memory and one warp per value adds them, a lane eight of them and then five shuffles: 8 dependent
+// additions and 24 warp instructions for 256 threads and two values, where a butterfly in every warp takes 90.
+template <int NV>
+__device__ __forceinline__ void block_sum(double (&v)[NV]) {
+    const int tid = threadIdx.x + threadIdx.y * blockDim.x, lane = tid & 31, w = tid >> 5;
+    const int nw = (blockDim.x * blockDim.y) >> 5;
+    if (nw == 1) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) v[q] = warp_sum(v[q]);
+        return;
+    }
+    __shared__ double sh[NV][256], res[NV];
+    __syncthreads();   // a previous sum's results have been read
+#pragma unroll
+    for (int q = 0; q < NV; ++q) sh[q][tid] = v[q];
     __syncthreads();
-    if (w == 0) {
-        a = l < nw ? sh[l] : 0.0;
-        b = l < nw ? sh[32 + l] : 0.0;
-        a = warp_sum(a);
-        b = warp_sum(b);
+    if (w < NV) {
+        double a[8];   // by a tree: three dependent additions for eight warps
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a[k] = k < nw ? sh[w][lane + 32 * k] : 0.0;
+        double t = nw <= 2 ? a[0] + a[1] : (nw <= 4 ? (a[0] + a[1]) + (a[2] + a[3]) : ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7])));
+        t = warp_sum(t);
+        if (lane == 0) res[w] = t;
     }
     __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = res[q];
 }
 
-// Deterministic grid-wide reduction of two values: every block writes its partial sums, the last block
-// to arrive sums the partials in index order (fixed partition + fixed tree) and returns true in all its
-// threads with the totals in `ta`, `tb`.  `partials` holds 2 * gridDim entries.
-__device__ __forceinline__ bool grid_sum2(double a, double b, double2* partials, unsigned int* ticket,
-                                          double& ta, double& tb) {
-    __shared__ double sh[64];
+// Deterministic grid-wide sums: every block writes its partial sums, the last block to arrive adds the partials in index
+// order (fixed partition and tree) and returns true in all its threads with the totals in `v`.  `partials` holds one
+// double2 per block.
+template <int NV>
+__device__ __forceinline__ bool grid_sum(double (&v)[NV], double2* partials, unsigned int* ticket) {
+    static_assert(NV == 1 || NV == 2, "one or two values");
     __shared__ bool last;
-    block_sum2(a, b, sh);
-    int nblocks = gridDim.x * gridDim.y;
-    int bid = blockIdx.x + blockIdx.y * gridDim.x;
-    int tid = threadIdx.x + threadIdx.y * blockDim.x;
+    block_sum<NV>(v);
+    const int nblocks = gridDim.x * gridDim.y, bid = blockIdx.x + blockIdx.y * gridDim.x;
+    const int tid = threadIdx.x + threadIdx.y * blockDim.x, nt = blockDim.x * blockDim.y;
     if (tid == 0) {
-        partials[bid] = make_double2(a, b);
-        __threadfence();
-        unsigned int t = atomicAdd(ticket, 1u);
+        partials[bid] = make_double2(v[0], NV == 2 ? v[NV - 1] : 0.0);
+        // releases this block's partials, acquires those of the blocks that came before
+        unsigned int t;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(ticket) : "memory");
         last = (t == (unsigned int)nblocks - 1);
     }
     __syncthreads();
     if (!last) return false;
-    __threadfence();
-    int nt = blockDim.x * blockDim.y;
-    double sa = 0.0, sb = 0.0;
-    // k = tid, tid + nt, ... in order; eight L2 reads issued before their adds (the partials of the other blocks
-    // are not in this SM's L1, so __ldcg), which keeps the summation order and overlaps the read latencies
-    for (int base = tid; base < nblocks; base += 8 * nt) {
-        double2 p[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+    for (int q = 0; q < NV; ++q) v[q] = 0.0;
+    // k = tid, tid + nt, ... four at a time: the L2 reads (the partials of the other blocks are not in this SM's L1, so
+    // __ldcg) are issued before their adds, and a fixed tree adds them
+    for (int base = tid; base < nblocks; base += 4 * nt) {
+        double2 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
             int k = base + u * nt;
             p[u] = k < nblocks ? __ldcg(&partials[k]) : make_double2(0.0, 0.0);
         }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            if (base + u * nt < nblocks) {
-                sa += p[u].x;
-                sb += p[u].y;
-            }
-        }
+        v[0] += (p[0].x + p[1].x) + (p[2].x + p[3].x);
+        if (NV == 2) v[NV - 1] += (p[0].y + p[1].y) + (p[2].y + p[3].y);
     }
-    block_sum2(sa, sb, sh);
+    block_sum<NV>(v);
     if (tid == 0) { *ticket = 0u; }
-    ta = sa;
-    tb = sb;
-    return true;   // totals valid in thread 0
+    return true;
+}
+__device__ __forceinline__ bool grid_sum2(double a, double b, double2* partials, unsigned int* ticket, double& ta, double& tb) {
+    double v[2] = {a, b};
+    bool last = grid_sum<2>(v, partials, ticket);
+    ta = v[0];
+    tb = v[1];
+    return last;
 }
 
 // ---- batched launches ------------------------------------------------------------------------------------
@@ -288,14 +322,35 @@ long long launch_count();
 struct LaunchDims {
     dim3 grid, block;
 };
-// The per-iteration CG vector kernels give each thread VEC_ROWS cells of one column (rows j, j + BY, ...):
-// the thread sums its cells before the block reduction, whose FP64 butterfly then costs a quarter per cell.
-constexpr int VEC_ROWS = 4;
+constexpr int SM_COUNT = 152;
+// Shape of the conjugate-gradient vector kernels: a warp takes the row segments (32 columns of one row) t, t + warps of the
+// grid, ... and a block adds its sums once.  The FP64 pipe is one per SM: a small grid spreads one or two warps over every
+// SM, a large one has as many warps resident as hide its loads, each SM with the same work to its end.  k_cg_update:
+// 128 x 64 10.3 -> 7.6 us, 1024 x 512 22.6 us without and 18.4 us with the r.z_old of the flexible beta.
 inline LaunchDims vec_dims(int nx, int ny) {
+    const long long w = (long long)((nx + 31) / 32) * ny;
+    const int warps = w <= 2ll * SM_COUNT ? 1 : (w <= 4ll * SM_COUNT ? 2 : (w <= 8ll * SM_COUNT ? 4 : 8));
+    const long long blocks = (w + warps - 1) / warps, resident = 3ll * SM_COUNT;
     LaunchDims d;
-    d.block = dim3(BX, BY);
-    d.grid = dim3((nx + BX - 1) / BX, (ny + BY * VEC_ROWS - 1) / (BY * VEC_ROWS), batch_slots());
+    d.block = dim3(32, warps);
+    d.grid = dim3((unsigned)(blocks < resident ? blocks : resident), 1, batch_slots());
     return d;
+}
+// Calls body(k, ok) for the thread's cells, two row segments at a time: their indices k[2] and whether they exist, ok[2].
+template <typename F>
+__device__ __forceinline__ void for_each_cell_pair(int Nx, int Ny, int pitch, F&& body) {
+    const int across = (Nx + 31) / 32, n = across * Ny, step = (int)(gridDim.x * blockDim.y);
+    for (int t = (int)(threadIdx.y * gridDim.x + blockIdx.x); t < n; t += 2 * step) {
+        int k[2];
+        bool ok[2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            const int s = t + a * step, j = s / across, i = (s - j * across) * 32 + (int)threadIdx.x;
+            ok[a] = s < n && i < Nx;
+            k[a] = j * pitch + i;
+        }
+        body(k, ok);
+    }
 }
 inline LaunchDims dims2d(int nx, int ny) {
     LaunchDims d;

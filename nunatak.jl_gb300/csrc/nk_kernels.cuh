@@ -66,36 +66,34 @@ void launch_inverse_row_sum(const OpView<T>& o, typename Vec2<T>::type* irs, cud
 
 struct CGView {
     OpView<double> o;
-    double2* x; const double2* b; double2* r; double2* z; double2* p; double2* q; double2* zold;
+    double2* x; const double2* b; double2* r; double2* z; double2* q;
+    double2* pa; double2* pb;     // the search direction: step k (from 0) writes pa (k even) or pb (k odd), reads the other
     const double2* invd;          // Jacobi inverse diagonal or nullptr
     int precond;                  // NK_PRECONDITIONER_*
     SolverScalars* sc;
     double2* partials;
     unsigned long long cond;      // conditional-node handle of the conjugate-gradient while loop (0: none)
     float2* r32;                  // mixed precision: FP32 copy of r written for the V-cycle (or nullptr)
-    const float2* z32;            // mixed precision: FP32 V-cycle result read back as z (or nullptr)
-    float2* zold32;               // mixed precision: z_old kept as the FP32 z32 it equals exactly (or nullptr);
-                                  // z itself is then never stored: each kernel that needs it rescales z32
+    const float2* z32;            // mixed precision: the V-cycle's FP32 result, z = z32 2^r32_exp exactly (or nullptr);
+                                  // z is never stored, and until the next V-cycle it is the z_old of the flexible β
 };
 __device__ __forceinline__ void rebase(CGView& v, long long d) {
     rebase(v.o, d);
-    shift_ptr(v.x, d); shift_ptr(v.b, d); shift_ptr(v.r, d); shift_ptr(v.z, d); shift_ptr(v.p, d); shift_ptr(v.q, d);
-    shift_ptr(v.zold, d); shift_ptr(v.invd, d); shift_ptr(v.sc, d); shift_ptr(v.partials, d);
-    shift_ptr(v.r32, d); shift_ptr(v.z32, d); shift_ptr(v.zold32, d);
+    shift_ptr(v.x, d); shift_ptr(v.b, d); shift_ptr(v.r, d); shift_ptr(v.z, d); shift_ptr(v.q, d); shift_ptr(v.pa, d);
+    shift_ptr(v.pb, d); shift_ptr(v.invd, d); shift_ptr(v.sc, d); shift_ptr(v.partials, d);
+    shift_ptr(v.r32, d); shift_ptr(v.z32, d);
 }
-// r = b - A x; if the preconditioner is not multigrid also z = M r, p = z, rho = r.z; r0, tol, done
+// r = b - A x; if the preconditioner is not multigrid also z = M r, rho = r.z; r0, tol, done
 void launch_cg_init(const CGView& v, cudaStream_t s);
-// multigrid: after z = V(r): p = z, rho = r.z, done
+// multigrid: after z = V(r): rho = r.z
 void launch_cg_init_finish(const CGView& v, cudaStream_t s);
 void launch_cg_scale_r32(const CGView& v, cudaStream_t s);
-// q = A p, alpha = rho / p.q
+// p = z + beta p (p = z in the first step), q = A p, alpha = rho / p.q
 void launch_cg_apply(const CGView& v, cudaStream_t s);
-// x += alpha p, r -= alpha q (and z = M r for Jacobi / none); dots for beta and the stopping test
+// x += alpha p, r -= alpha q (and z = M r for Jacobi / none); the stopping decision, and the dots that beta needs
 void launch_cg_update(const CGView& v, cudaStream_t s);
-// multigrid: z = V(r) done; dots r.z (and r.z_old when flexible), beta
+// multigrid: z = V(r) done; r.z, beta
 void launch_cg_dots_after_precondition(const CGView& v, cudaStream_t s);
-// p = z + beta p, then commit the stopping decision of this step
-void launch_cg_xpby(const CGView& v, cudaStream_t s);
 // z = r * invd on the Nx x Ny range, z = r on the wall faces (unit diagonal)
 void launch_precondition_diagonal(const DevGrid<double>& g, double2* z, const double2* r, const double2* invd, cudaStream_t s);
 // Picard: xprev = x (over the Nx x Ny range)

@@ -63,6 +63,7 @@ int strip_rows(int nx, int ny, int elem_bytes, int kind) {
         return (r == 1 || r == 2 || r == 4 || r == 8) ? r : 0;
     }();
     if (forced) return elem_bytes == 8 ? std::min(forced, 4) : forced;
+    if (kind == STRIP_OPERATOR && elem_bytes == 8) return 0;   // operator_shape chooses
     if (kind != STRIP_OPERATOR) {
         std::lock_guard<std::mutex> g(tuned_mutex());
         auto it = tuned_rows().find(std::make_tuple(kind, nx, ny, elem_bytes));
@@ -73,7 +74,6 @@ int strip_rows(int nx, int ny, int elem_bytes, int kind) {
     // below 2^16 cells, two above; 1.48 -> 1.68 solves/s on the FP64 stream); FP32 and the FP64 operator kernels
     // keep two rows (four from 2^18 cells for the operator), which the concurrent mixed stream prefers
     if (elem_bytes == 8 && kind != STRIP_OPERATOR) return cells < (1 << 16) ? 1 : 2;
-    if (elem_bytes == 8) return cells >= (1 << 18) ? 4 : 2;
     return 2;
 }
 
@@ -193,7 +193,7 @@ struct nk_problem {
     double *H = nullptr, *bed = nullptr, *s = nullptr, *N = nullptr, *mu = nullptr, *phi = nullptr, *C = nullptr, *F2 = nullptr, *A2 = nullptr;
     double *A3 = nullptr, *T = nullptr, *eta_sigma = nullptr;
     double2 *phi_uv = nullptr, *tau = nullptr, *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *xprev = nullptr,
-            *zold = nullptr, *invd = nullptr, *bb = nullptr, *ub = nullptr, *usig = nullptr, *tmp_a = nullptr, *tmp_b = nullptr;
+            *p2 = nullptr, *invd = nullptr, *bb = nullptr, *ub = nullptr, *usig = nullptr, *tmp_a = nullptr, *tmp_b = nullptr;
     double* staging = nullptr;
     size_t staging_count = 0;
     double2* partials = nullptr;
@@ -297,8 +297,8 @@ struct nk_problem {
     CGView cg_view(const double2* b) const {
         CGView v;
         v.o = fine_op();
-        v.x = x; v.b = b; v.r = r; v.z = z; v.p = p; v.q = q;
-        v.zold = nullptr;
+        v.x = x; v.b = b; v.r = r; v.z = z; v.q = q;
+        v.pa = p; v.pb = p2;
         v.invd = invd;
         v.precond = precond;
         v.sc = sc;
@@ -307,7 +307,6 @@ struct nk_problem {
         bool fused = mixed && precond == NK_PRECONDITIONER_MULTIGRID;
         v.r32 = fused ? lv32[0].b : nullptr;
         v.z32 = fused ? lv32[0].x : nullptr;
-        v.zold32 = fused ? reinterpret_cast<float2*>(zold) : nullptr;   // flexible CG: z_old in FP32
         return v;
     }
 };
@@ -469,7 +468,7 @@ static void build(nk_problem* P, bool dry = false) {
     slots.push_back({(void**)&F.coef, A.reserve(pl * sizeof(double4))});
     slots.push_back({(void**)&F.mask, A.reserve(pl)});
     for (double** f : {&P->H, &P->bed, &P->s, &P->N, &P->mu, &P->phi, &P->C, &P->F2, &P->A2}) slots.push_back({(void**)f, A.reserve(d1)});
-    for (double2** f : {&P->phi_uv, &P->tau, &P->x, &P->r, &P->z, &P->p, &P->q, &P->xprev, &P->zold, &P->invd, &P->bb, &P->ub,
+    for (double2** f : {&P->phi_uv, &P->tau, &P->x, &P->r, &P->z, &P->p, &P->q, &P->xprev, &P->p2, &P->invd, &P->bb, &P->ub,
                         &P->tmp_a, &P->tmp_b})
         slots.push_back({(void**)f, A.reserve(d2)});
     slots.push_back({(void**)&P->eta_sigma, A.reserve(d1 * P->Ns)});
@@ -480,8 +479,9 @@ static void build(nk_problem* P, bool dry = false) {
     slots.push_back({(void**)&P->usig, A.reserve(d2 * P->Ns)});
     P->staging_count = (size_t)(P->Nx + 1) * (P->Ny + 1) * P->Ns;
     slots.push_back({(void**)&P->staging, A.reserve(P->staging_count * sizeof(double))});
-    LaunchDims big = dims2d(P->Nx + 1, P->Ny + 1), strips = strip_dims(P->Nx, P->Ny, STRIP_MIN_ROWS);
-    size_t nblocks = std::max((size_t)big.grid.x * big.grid.y, (size_t)strips.grid.x * strips.grid.y);
+    // the most blocks of a reduction: one a 2-D tile, or the resident blocks of operator_dims and vec_dims
+    LaunchDims big = dims2d(P->Nx + 1, P->Ny + 1);
+    size_t nblocks = std::max((size_t)big.grid.x * big.grid.y, (size_t)8 * SM_COUNT);
     slots.push_back({(void**)&P->partials, A.reserve(nblocks * sizeof(double2))});
     slots.push_back({(void**)&P->sc, A.reserve(sizeof(SolverScalars))});
     slots.push_back({(void**)&P->sig_tables, A.reserve((4 * P->Ns + 1 + (size_t)P->Ns * P->Ns) * sizeof(double))});
@@ -724,7 +724,7 @@ static void precondition_mg(nk_problem* P, const int* done, bool fused = false) 
 // so a solve needs no host round trip until it has finished:
 //
 //   picard_begin ─► WHILE(picard) { x⁻ = x ─► coefficient update ─► coarse coefficients ─► CG start
-//                                    ─► WHILE(cg) { apply ─► update ─► [V-cycle ─► dots] ─► xpby }
+//                                    ─► WHILE(cg) { apply ─► update ─► [V-cycle ─► dots] }
 //                                    ─► picard_end (Δ, X, stopping test) }
 static SolverScalars control_scalars(const nk_problem* P) {
     SolverScalars h{};
@@ -756,7 +756,6 @@ static void cg_step(nk_problem* P, const CGView& v) {
         precondition_mg(P, &P->sc->done, true);
         launch_cg_dots_after_precondition(v, s);
     }
-    launch_cg_xpby(v, s);
 }
 
 // conjugate_gradient!, conjugate_gradient.jl:165-171 (everything before the iteration loop)
@@ -2723,12 +2722,9 @@ nk_status nk_time_kernel(nk_problem* P, int32_t kernel, int32_t repeats, int64_t
             ev = energy_view(P, &q);
             NK_CUDA(cudaMemcpyAsync(const_cast<double*>(ev.E_old), P->thermal, (size_t)P->Ns * P->plane * sizeof(double), cudaMemcpyDeviceToDevice, s));
         }
-        if (kernel == NK_KERNEL_CG_UPDATE) {
-            // run the update with done = 0 so it is not skipped
-            P->sc_host->done = 0;
-            NK_CUDA(cudaMemcpyAsync(&P->sc->done, &P->sc_host->done, sizeof(int), cudaMemcpyHostToDevice, s));
-        }
         for (int rep = 0; rep < repeats; ++rep) {
+            if (kernel == NK_KERNEL_CG_UPDATE)   // every update with done = 0, which it may set itself, so none is skipped
+                NK_CUDA(cudaMemsetAsync(&P->sc->done, 0, sizeof(int), s));
             if (flush) NK_CUDA(cudaMemsetAsync(flush, rep & 0xff, (size_t)flush_bytes, s));
             NK_CUDA(cudaEventRecord(P->ev0, s));
             launch();

@@ -2,10 +2,9 @@
 //
 // Conjugate gradients restate src/Solvers/conjugate_gradient.jl:158-223 with the vector operations of
 // src/Solvers/velocity_vector.jl:48-141 fused into the kernels that produce their operands:
-//   step k:  apply   q = A p,  alpha = rho / p.q                       (one kernel + fused dot)
-//            update  x += alpha p, r -= alpha q [, z = r / diag], dots (one kernel + fused dots)
+//   step k:  apply   p = z + beta p, q = A p, alpha = rho / p.q          (one kernel + fused dot)
+//            update  x += alpha p, r -= alpha q [, z = r / diag], dots, the stopping decision (one kernel)
 //            [multigrid: z = V-cycle(r), then the r.z dot]
-//            xpby    p = z + beta p, commit the stopping decision        (one kernel)
 // Every dot is a deterministic two-stage reduction (fixed block partition and tree); its result stays
 // on the device, so no step needs a host synchronisation.  Every kernel of a step first reads the
 // device `done` flag and returns when the solve has stopped, so steps can be launched in batches (or
@@ -72,17 +71,28 @@ void launch_fill(double* dst, int count, double value, cudaStream_t s) {
 }
 
 // ---- operator, masks, diagonals ---------------------------------------------------------------------------
+// The operand of an FP64 operator kernel read from an array
+struct ReadPair {
+    const double2* p;
+    __device__ __forceinline__ double2 operator()(int k) const { return p[k]; }
+};
+struct SamePair {
+    __device__ __forceinline__ double2 operator()(const double2& x) const { return x; }
+};
+struct NoRead {
+    __device__ __forceinline__ NoExtra operator()(int) const { return NoExtra{}; }
+};
+static int forced_operator_rows() { return strip_rows(0, 0, 8); }   // NK_STRIP_ROWS, or 0
+
 template <int R>
-__global__ void __launch_bounds__(32 * STRIP_WARPS) k_apply(OpView<double> o, const double2* __restrict__ p, double2* __restrict__ q) {
-    int i, j0;
-    strip_origin<R>(i, j0);
-    if (j0 >= o.g.Ny) return;   // whole warp
-    strip_apply<R>(o, p, i, j0, [](int) { return NoExtra{}; }, [&](int k, double2 a, double2, NoExtra) { q[k] = a; });
+__global__ void __launch_bounds__(32 * STRIP_WARPS) k_apply(OpView<double> o, const double2* __restrict__ p, double2* __restrict__ q, int rows) {
+    for_each_strip(o.g.Nx, o.g.Ny, rows, [&](int i, int j0) {
+        strip_walk<R>(o, rows, ReadPair{p}, SamePair{}, i, j0, NoRead{}, [&](int k, double2 a, double2, NoExtra) { q[k] = a; });
+    });
 }
 void launch_apply(const OpView<double>& o, const double2* p, double2* q, cudaStream_t s) {
-    int rows = strip_rows(o.g.Nx, o.g.Ny, 8);
-    LaunchDims d = strip_dims(o.g.Nx, o.g.Ny, rows);
-    with_strip_rows(rows, [&](auto r) { k_apply<decltype(r)::value><<<d.grid, d.block, 0, s>>>(o, p, q); });
+    OperatorShape d = operator_shape(o.g.Nx, o.g.Ny, forced_operator_rows());
+    with_operator_rows(d.rows, [&](auto r, int rows) { k_apply<decltype(r)::value><<<d.d.grid, d.d.block, 0, s>>>(o, p, q, rows); });
     count_launch();
 }
 
@@ -203,21 +213,26 @@ template void launch_inverse_row_sum<float>(const OpView<float>&, float2*, cudaS
 // ---- conjugate gradients ------------------------------------------------------------------------------------
 __device__ __forceinline__ int read_done(const SolverScalars* sc) { return *(volatile const int*)&sc->done; }
 
-__device__ __forceinline__ int stop_after(const SolverScalars* sc, double rnorm, int it) {
-    if (!isfinite(rnorm)) return 1;
-    if (sc->fixed) return it >= sc->iterations;
-    return !(rnorm > sc->tol && it < sc->maxiter);
-}
+// The stopping rule's settings, read at a kernel's start so that the last block's decision waits for no load
+struct StopRule {
+    double tol;
+    int fixed, iterations, maxiter;
+    __device__ __forceinline__ explicit StopRule(const SolverScalars* sc)
+        : tol(sc->tol), fixed(sc->fixed), iterations(sc->iterations), maxiter(sc->maxiter) {}
+    __device__ __forceinline__ int stop(double rnorm, int it) const {
+        if (!finite_bits(rnorm)) return 1;
+        if (fixed) return it >= iterations;
+        return !(rnorm > tol && it < maxiter);
+    }
+};
 
 // conjugate_gradient!, conjugate_gradient.jl:165-171: r = b - A x, z = M r, p = z, rho = r.z
 template <int R>
-__global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_init(CGView v) {
+__global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_init(CGView v, int rows) {
     NK_BATCH_ENTER(v.o.g, v)
-    int i, j0;
-    strip_origin<R>(i, j0);
     double rz = 0.0, rr = 0.0;
-    if (j0 < v.o.g.Ny) {   // warps below the grid still take part in the block reduction
-        strip_apply<R>(v.o, (const double2*)v.x, i, j0, [&](int k) { return v.b[k]; }, [&](int k, double2 q, double2, const double2& b) {
+    for_each_strip(v.o.g.Nx, v.o.g.Ny, rows, [&](int i, int j0) {
+        strip_walk<R>(v.o, rows, ReadPair{v.x}, SamePair{}, i, j0, ReadPair{v.b}, [&](int k, double2 q, double2, const double2& b) {
             double2 r = make_double2(b.x - q.x, b.y - q.y);
             v.r[k] = r;   // the FP32 copy for the multigrid follows in k_cg_scale_r32, once ‖r0‖ is known
             rr += r.x * r.x + r.y * r.y;
@@ -228,11 +243,10 @@ __global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_init(CGView v) {
                     z = make_double2(r.x * d.x, r.y * d.y);
                 }
                 v.z[k] = z;
-                v.p[k] = z;
                 rz += r.x * z.x + r.y * z.y;
             }
         });
-    }
+    });
     double trz, trr;
     if (grid_sum2(rz, rr, v.partials, &v.sc->ticket, trz, trr) && threadIdx.x == 0 && threadIdx.y == 0) {
         SolverScalars* sc = v.sc;
@@ -249,14 +263,12 @@ __global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_init(CGView v) {
         int done = sc->fixed ? (sc->iterations <= 0) : !(r0 > sc->tol && 0 < sc->maxiter);
         if (!isfinite(r0)) done = 1;
         sc->done = done;
-        sc->done_next = done;
         if (v.cond && v.precond != NK_PRECONDITIONER_MULTIGRID) cudaGraphSetConditional(v.cond, done ? 0u : 1u);
     }
 }
 void launch_cg_init(const CGView& v, cudaStream_t s) {
-    int rows = strip_rows(v.o.g.Nx, v.o.g.Ny, 8);
-    LaunchDims d = strip_dims(v.o.g.Nx, v.o.g.Ny, rows);
-    with_strip_rows(rows, [&](auto r) { k_cg_init<decltype(r)::value><<<d.grid, d.block, 0, s>>>(v); });
+    OperatorShape d = operator_shape(v.o.g.Nx, v.o.g.Ny, forced_operator_rows());
+    with_operator_rows(d.rows, [&](auto r, int rows) { k_cg_init<decltype(r)::value><<<d.d.grid, d.d.block, 0, s>>>(v, rows); });
     count_launch();
 }
 
@@ -268,7 +280,7 @@ __global__ void k_cg_scale_r32(CGView v) {
     if (i < v.o.g.Nx && j < v.o.g.Ny) {
         int k = v.o.g.idx(i, j);
         double2 r = v.r[k];
-        v.r32[k] = make_float2((float)scale_pow2(r.x, -e), (float)scale_pow2(r.y, -e));
+        v.r32[k] = make_float2(narrow_pow2(r.x, -e), narrow_pow2(r.y, -e));
     }
 }
 void launch_cg_scale_r32(const CGView& v, cudaStream_t s) {
@@ -276,34 +288,27 @@ void launch_cg_scale_r32(const CGView& v, cudaStream_t s) {
     k_cg_scale_r32<<<d.grid, d.block, 0, s>>>(v); count_launch();
 }
 
-// multigrid start: p = z, rho = r.z (and z_old = z for flexible conjugate gradients)
-__global__ void k_cg_init_finish(CGView v) {
+// z at k: the FP64 z, or the V-cycle's FP32 result scaled by 2^ze (the conversion and the scaling are exact)
+__device__ __forceinline__ double2 cg_z(const CGView& v, int k, int ze) {
+    if (!v.z32) return v.z[k];
+    float2 f = v.z32[k];
+    return make_double2(widen_pow2(f.x, ze), widen_pow2(f.y, ze));
+}
+// multigrid start: rho = r.z
+__global__ void __launch_bounds__(256) k_cg_init_finish(CGView v) {
     NK_BATCH_ENTER(v.o.g, v)
-    int i = blockIdx.x * BX + threadIdx.x, j0 = blockIdx.y * BY * VEC_ROWS + threadIdx.y;
-    double rz = 0.0;
+    const int ze = v.sc->r32_exp;
+    double rz[1] = {0.0};
+    for_each_cell_pair(v.o.g.Nx, v.o.g.Ny, v.o.g.pitch, [&](const int* k, const bool* ok) {
 #pragma unroll
-    for (int row = 0; row < VEC_ROWS; ++row) {
-        int j = j0 + row * BY;
-        if (i < v.o.g.Nx && j < v.o.g.Ny) {
-            int k = v.o.g.idx(i, j);
-            double2 z, r = v.r[k];
-            if (v.z32) {
-                float2 f = v.z32[k];
-                int ze = v.sc->r32_exp;
-                z = make_double2(scale_pow2((double)f.x, ze), scale_pow2((double)f.y, ze));
-                if (v.zold32) v.zold32[k] = f;
-            } else {
-                z = v.z[k];
+        for (int a = 0; a < 2; ++a)
+            if (ok[a]) {
+                double2 z = cg_z(v, k[a], ze), r = v.r[k[a]];
+                rz[0] = fma(r.x, z.x, fma(r.y, z.y, rz[0]));
             }
-            v.p[k] = z;
-            if (v.zold) v.zold[k] = z;
-            rz += r.x * z.x + r.y * z.y;
-        }
-    }
-    double trz, dummy;
-    if (grid_sum2(rz, 0.0, v.partials, &v.sc->ticket, trz, dummy) && threadIdx.x == 0 && threadIdx.y == 0) {
-        v.sc->rho = trz;
-        v.sc->zold_exp = v.sc->r32_exp;   // the exponent of the z32 now in zold32
+    });
+    if (grid_sum<1>(rz, v.partials, &v.sc->ticket) && threadIdx.x == 0 && threadIdx.y == 0) {
+        v.sc->rho = rz[0];
         if (v.cond) cudaGraphSetConditional(v.cond, v.sc->done ? 0u : 1u);
     }
 }
@@ -312,89 +317,121 @@ void launch_cg_init_finish(const CGView& v, cudaStream_t s) {
     k_cg_init_finish<<<d.grid, d.block, 0, s>>>(v); count_launch();
 }
 
-// conjugate_gradient_step!, conjugate_gradient.jl:209-212: q = A p, alpha = rho / p.q (0 if p.q = 0)
+// conjugate_gradient_step!, conjugate_gradient.jl:209-212 and the xpby! of the step before (:220): p = z + beta p where
+// the operand is loaded, q = A p, alpha = rho / p.q (0 if p.q = 0).  Bound by the FP64 pipe.  The rows above and below a
+// walk and the columns beside a strip form their p twice, 3.2 FP64 instructions a cell instead of a pass of its own
+// over z and p (10 us of launch and traffic at 1024 x 512, 5 us at 128 x 64); a cell's p is written to the buffer that this
+// step's readers do not read.
 template <int R>
-__global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_apply(CGView v) {
+__global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_apply(CGView v, int rows) {
     NK_BATCH_ENTER(v.o.g, v)
     if (read_done(v.sc)) return;
-    int i, j0;
-    strip_origin<R>(i, j0);
-    double pq = 0.0;
-    if (j0 < v.o.g.Ny) {   // warps below the grid still take part in the block reduction
-        strip_apply<R>(v.o, (const double2*)v.p, i, j0, [](int) { return NoExtra{}; }, [&](int k, double2 q, double2 p, NoExtra) {
+    const int it = v.sc->it, ze = v.sc->r32_exp;
+    const double beta = v.sc->beta;
+    double2* p_out = (it & 1) ? v.pb : v.pa;
+    const double2* p_in = (it & 1) ? v.pa : v.pb;
+    const bool first = it == 0;
+    const double rho = v.sc->rho;
+    const int status = v.sc->status;
+    double pq[1] = {0.0};
+    struct Operand { double2 z, p; float2 z32; };
+    auto load = [&](int k) {
+        Operand a;
+        if (v.z32) a.z32 = v.z32[k]; else a.z = v.z[k];
+        if (!first) a.p = p_in[k];
+        return a;
+    };
+    auto value = [&](const Operand& a) {
+        double2 z = v.z32 ? make_double2(widen_pow2(a.z32.x, ze), widen_pow2(a.z32.y, ze)) : a.z;
+        return first ? z : make_double2(z.x + beta * a.p.x, z.y + beta * a.p.y);
+    };
+    for_each_strip(v.o.g.Nx, v.o.g.Ny, rows, [&](int i, int j0) {
+        strip_walk<R>(v.o, rows, load, value, i, j0, NoRead{}, [&](int k, double2 q, double2 p, NoExtra) {
             v.q[k] = q;
-            pq += p.x * q.x + p.y * q.y;
+            p_out[k] = p;
+            pq[0] = fma(p.x, q.x, fma(p.y, q.y, pq[0]));
         });
-    }
-    double tpq, dummy;
-    if (grid_sum2(pq, 0.0, v.partials, &v.sc->ticket, tpq, dummy) && threadIdx.x == 0 && threadIdx.y == 0) {
+    });
+    if (grid_sum<1>(pq, v.partials, &v.sc->ticket) && threadIdx.x == 0 && threadIdx.y == 0) {
         SolverScalars* sc = v.sc;
-        sc->pq = tpq;
-        sc->alpha = (tpq == 0.0) ? 0.0 : sc->rho / tpq;
-        if (tpq < 0.0 && sc->status == NK_OK) sc->status = NK_BREAKDOWN;
+        sc->pq = pq[0];
+        sc->alpha = (pq[0] == 0.0) ? 0.0 : rho / pq[0];
+        if (pq[0] < 0.0 && status == NK_OK) sc->status = NK_BREAKDOWN;
     }
 }
 void launch_cg_apply(const CGView& v, cudaStream_t s) {
-    int rows = strip_rows(v.o.g.Nx, v.o.g.Ny, 8);
-    LaunchDims d = strip_dims(v.o.g.Nx, v.o.g.Ny, rows);
-    with_strip_rows(rows, [&](auto r) { k_cg_apply<decltype(r)::value><<<d.grid, d.block, 0, s>>>(v); });
+    OperatorShape d = operator_shape(v.o.g.Nx, v.o.g.Ny, forced_operator_rows());
+    with_operator_rows(d.rows, [&](auto r, int rows) { k_cg_apply<decltype(r)::value><<<d.d.grid, d.d.block, 0, s>>>(v, rows); });
     count_launch();
 }
 
-// conjugate_gradient_step!, conjugate_gradient.jl:214-219 and the stopping test of :193-197
-__global__ void k_cg_update(CGView v) {
+// conjugate_gradient_step!, conjugate_gradient.jl:214-219 and the stopping test of :193-197.  With the multigrid in
+// FP32 also r_new.z_old of the flexible beta, whose z_old is still the V-cycle's last result.  The last block takes the
+// stopping decision, so the V-cycle after the last step is skipped.
+__global__ void __launch_bounds__(256, 3) k_cg_update(CGView v) {
     NK_BATCH_ENTER(v.o.g, v)
     if (read_done(v.sc)) return;
-    int i = blockIdx.x * BX + threadIdx.x, j0 = blockIdx.y * BY * VEC_ROWS + threadIdx.y;
-    double alpha = v.sc->alpha;
-    // FP32 copy of the new residual scaled by the exponent of the previous norm (read before the last block
-    // replaces it)
-    int r32_exp = v.sc->r32_exp_next;
-    double rz = 0.0, rr = 0.0;
+    const double alpha = v.sc->alpha;
+    // FP32 copy of the new residual scaled by the exponent of the previous norm, z_old by its own (both read before the
+    // last block replaces them)
+    const int r32_exp = v.sc->r32_exp_next, ze = v.sc->r32_exp;
+    const int it0 = v.sc->it;
+    const double rho = v.sc->rho;
+    const StopRule rule(v.sc);
+    const double2* pp = (it0 & 1) ? v.pb : v.pa;
+    const bool jacobi = v.precond == NK_PRECONDITIONER_DIAGONAL, mg = v.precond == NK_PRECONDITIONER_MULTIGRID;
+    double t[2] = {0.0, 0.0};   // r.r, and r.z (Jacobi, none) or r.z_old (mixed)
+    for_each_cell_pair(v.o.g.Nx, v.o.g.Ny, v.o.g.pitch, [&](const int* k, const bool* ok) {
+        double2 p[2], q[2], x[2], r[2], d[2];
+        float2 zo[2];
 #pragma unroll
-    for (int row = 0; row < VEC_ROWS; ++row) {
-        int j = j0 + row * BY;
-        if (i < v.o.g.Nx && j < v.o.g.Ny) {
-            int k = v.o.g.idx(i, j);
-            double2 p = v.p[k], q = v.q[k], x = v.x[k], r = v.r[k];
-            x.x = x.x + alpha * p.x;
-            x.y = x.y + alpha * p.y;
-            r.x = r.x + (-alpha) * q.x;
-            r.y = r.y + (-alpha) * q.y;
-            v.x[k] = x;
-            v.r[k] = r;
-            if (v.r32) v.r32[k] = make_float2((float)scale_pow2(r.x, -r32_exp), (float)scale_pow2(r.y, -r32_exp));
-            rr += r.x * r.x + r.y * r.y;
-            if (v.precond != NK_PRECONDITIONER_MULTIGRID) {
-                double2 z = r;
-                if (v.precond == NK_PRECONDITIONER_DIAGONAL) {
-                    double2 d = v.invd[k];
-                    z = make_double2(r.x * d.x, r.y * d.y);
-                }
-                v.z[k] = z;
-                rz += r.x * z.x + r.y * z.y;
+        for (int a = 0; a < 2; ++a)   // every read before any write
+            if (ok[a]) {
+                p[a] = pp[k[a]]; q[a] = v.q[k[a]]; x[a] = v.x[k[a]]; r[a] = v.r[k[a]];
+                if (jacobi) d[a] = v.invd[k[a]];
+                if (v.z32) zo[a] = v.z32[k[a]];
             }
-        }
-    }
-    double trz, trr;
-    if (grid_sum2(rz, rr, v.partials, &v.sc->ticket, trz, trr) && threadIdx.x == 0 && threadIdx.y == 0) {
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+            if (ok[a]) {
+                double2 xx = x[a], rr = r[a];
+                xx.x = xx.x + alpha * p[a].x;
+                xx.y = xx.y + alpha * p[a].y;
+                rr.x = rr.x + (-alpha) * q[a].x;
+                rr.y = rr.y + (-alpha) * q[a].y;
+                v.x[k[a]] = xx;
+                v.r[k[a]] = rr;
+                if (v.r32) v.r32[k[a]] = make_float2(narrow_pow2(rr.x, -r32_exp), narrow_pow2(rr.y, -r32_exp));
+                t[0] = fma(rr.x, rr.x, fma(rr.y, rr.y, t[0]));
+                if (!mg) {
+                    double2 z = rr;
+                    if (jacobi) z = make_double2(rr.x * d[a].x, rr.y * d[a].y);
+                    v.z[k[a]] = z;
+                    t[1] = fma(rr.x, z.x, fma(rr.y, z.y, t[1]));
+                } else if (v.z32) {
+                    t[1] = fma(rr.x, widen_pow2(zo[a].x, ze), fma(rr.y, widen_pow2(zo[a].y, ze), t[1]));
+                }
+            }
+    });
+    if (grid_sum<2>(t, v.partials, &v.sc->ticket) && threadIdx.x == 0 && threadIdx.y == 0) {
         SolverScalars* sc = v.sc;
-        sc->rr = trr;
-        double rn = sqrt(trr);
+        sc->rr = t[0];
+        const double rn = sqrt(t[0]);
+        const int it = it0 + 1, stop = rule.stop(rn, it);
+        if (!mg) {
+            sc->beta = (rho == 0.0) ? 0.0 : t[1] / rho;
+            sc->rho = t[1];
+        } else {
+            sc->rz_old = t[1];
+        }
         sc->r32_exp = r32_exp;
         sc->r32_exp_next = residual_exponent(rn);
         sc->rnorm = rn;
-        int it = sc->it + 1;
         sc->it = it;
-        if (v.precond != NK_PRECONDITIONER_MULTIGRID) {
-            double rho = sc->rho;
-            sc->beta = (rho == 0.0) ? 0.0 : trz / rho;
-            sc->rho = trz;
-        }
-        if (!isfinite(rn)) sc->status = NK_NONFINITE;
-        int stop = stop_after(sc, rn, it);
-        sc->done_next = stop;
-        if (stop && !sc->fixed && !(rn <= sc->tol)) sc->cg_unconverged += 1;
+        if (!finite_bits(rn)) sc->status = NK_NONFINITE;
+        if (stop && !rule.fixed && !(rn <= rule.tol)) sc->cg_unconverged += 1;
+        sc->done = stop;
+        if (v.cond) cudaGraphSetConditional(v.cond, stop ? 0u : 1u);
     }
 }
 void launch_cg_update(const CGView& v, cudaStream_t s) {
@@ -404,94 +441,31 @@ void launch_cg_update(const CGView& v, cudaStream_t s) {
 
 // after z = V-cycle(r): rho_new = r.z; beta = rho_new / rho, or the flexible (Polak-Ribière) form
 // beta = (r.z - r.z_old) / rho when the preconditioner varies between steps
-__global__ void k_cg_dots_after_precondition(CGView v) {
+__global__ void __launch_bounds__(256) k_cg_dots_after_precondition(CGView v) {
     NK_BATCH_ENTER(v.o.g, v)
     if (read_done(v.sc)) return;
-    int i = blockIdx.x * BX + threadIdx.x, j0 = blockIdx.y * BY * VEC_ROWS + threadIdx.y;
-    double rz = 0.0, rzo = 0.0;
+    const int ze = v.sc->r32_exp, flexible = v.sc->flexible;
+    const double rho = v.sc->rho, rz_old = v.sc->rz_old;
+    double rz[1] = {0.0};
+    for_each_cell_pair(v.o.g.Nx, v.o.g.Ny, v.o.g.pitch, [&](const int* k, const bool* ok) {
+        double2 z[2], r[2];
 #pragma unroll
-    for (int row = 0; row < VEC_ROWS; ++row) {
-        int j = j0 + row * BY;
-        if (i < v.o.g.Nx && j < v.o.g.Ny) {
-            int k = v.o.g.idx(i, j);
-            double2 r = v.r[k], z;
-            if (v.z32) {
-                float2 f = v.z32[k];
-                int ze = v.sc->r32_exp;
-                z = make_double2(scale_pow2((double)f.x, ze), scale_pow2((double)f.y, ze));
-            } else {
-                z = v.z[k];
-            }
-            rz += r.x * z.x + r.y * z.y;
-            if (v.zold32) {
-                float2 fo = v.zold32[k];
-                int zo_e = v.sc->zold_exp;
-                double2 zo = make_double2(scale_pow2((double)fo.x, zo_e), scale_pow2((double)fo.y, zo_e));
-                rzo += r.x * zo.x + r.y * zo.y;
-            } else if (v.zold) {
-                double2 zo = v.zold[k];
-                rzo += r.x * zo.x + r.y * zo.y;
-            }
-        }
-    }
-    double trz, trzo;
-    if (grid_sum2(rz, rzo, v.partials, &v.sc->ticket, trz, trzo) && threadIdx.x == 0 && threadIdx.y == 0) {
+        for (int a = 0; a < 2; ++a)
+            if (ok[a]) { z[a] = cg_z(v, k[a], ze); r[a] = v.r[k[a]]; }
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+            if (ok[a]) rz[0] = fma(r[a].x, z[a].x, fma(r[a].y, z[a].y, rz[0]));
+    });
+    if (grid_sum<1>(rz, v.partials, &v.sc->ticket) && threadIdx.x == 0 && threadIdx.y == 0) {
         SolverScalars* sc = v.sc;
-        double rho = sc->rho;
-        double num = sc->flexible ? (trz - trzo) : trz;
+        const double num = flexible ? (rz[0] - rz_old) : rz[0];
         sc->beta = (rho == 0.0) ? 0.0 : num / rho;
-        sc->rho = trz;
-        sc->rz_old = trzo;
+        sc->rho = rz[0];
     }
 }
 void launch_cg_dots_after_precondition(const CGView& v, cudaStream_t s) {
     LaunchDims d = vec_dims(v.o.g.Nx, v.o.g.Ny);
     k_cg_dots_after_precondition<<<d.grid, d.block, 0, s>>>(v); count_launch();
-}
-
-// xpby!(z, beta, p), conjugate_gradient.jl:220; the last block commits the stopping decision
-__global__ void k_cg_xpby(CGView v) {
-    NK_BATCH_ENTER(v.o.g, v)
-    if (read_done(v.sc)) return;
-    int i = blockIdx.x * BX + threadIdx.x, j0 = blockIdx.y * BY * VEC_ROWS + threadIdx.y;
-    double beta = v.sc->beta;
-    int ze = v.sc->r32_exp;
-#pragma unroll
-    for (int row = 0; row < VEC_ROWS; ++row) {
-        int j = j0 + row * BY;
-        if (i < v.o.g.Nx && j < v.o.g.Ny) {
-            int k = v.o.g.idx(i, j);
-            double2 z, p = v.p[k];
-            if (v.z32) {   // z = z32 2^e, as k_cg_dots_after_precondition formed it; z_old keeps z32 itself
-                float2 f = v.z32[k];
-                z = make_double2(scale_pow2((double)f.x, ze), scale_pow2((double)f.y, ze));
-                if (v.zold32) v.zold32[k] = f;
-            } else {
-                z = v.z[k];
-            }
-            p.x = z.x + beta * p.x;
-            p.y = z.y + beta * p.y;
-            v.p[k] = p;
-            if (v.zold) v.zold[k] = z;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        __threadfence();
-        unsigned int n = gridDim.x * gridDim.y;
-        unsigned int t = atomicAdd(&v.sc->ticket2, 1u);
-        if (t == n - 1) {
-            v.sc->ticket2 = 0u;
-            v.sc->zold_exp = v.sc->r32_exp;   // the exponent of the z32 now in zold32
-            int d = v.sc->done_next;
-            v.sc->done = d;
-            if (v.cond) cudaGraphSetConditional(v.cond, d ? 0u : 1u);
-        }
-    }
-}
-void launch_cg_xpby(const CGView& v, cudaStream_t s) {
-    LaunchDims d = vec_dims(v.o.g.Nx, v.o.g.Ny);
-    k_cg_xpby<<<d.grid, d.block, 0, s>>>(v); count_launch();
 }
 
 // precondition!(z, ::StressBalanceDiagonalPreconditioner, r, ...) over size(z.u), size(z.v)

@@ -20,7 +20,7 @@
 namespace nk {
 
 constexpr int STRIP_COLS = 30;   // columns written per warp (lanes 1..30)
-constexpr int STRIP_WARPS = 4;   // warps per block, stacked in y
+constexpr int STRIP_WARPS = 4;   // most warps per block, stacked in y
 
 // Launch shape of a strip kernel whose warps walk `rows` rows each.
 inline LaunchDims strip_dims(int nx, int ny, int rows) {
@@ -29,7 +29,6 @@ inline LaunchDims strip_dims(int nx, int ny, int rows) {
     d.grid = dim3((nx + STRIP_COLS - 1) / STRIP_COLS, (ny + rows * STRIP_WARPS - 1) / (rows * STRIP_WARPS), batch_slots());
     return d;
 }
-
 // Rows per warp for an nx x ny grid of `elem_bytes`-byte values (host side; nk_problem.cu).  Long walks
 // amortise the two priming rows on large grids; short ones keep enough warps in flight on small grids.
 // `kind` names the kernel: the multigrid sweeps and residuals write one value per cell with no reduction, so
@@ -37,7 +36,6 @@ inline LaunchDims strip_dims(int nx, int ny, int rows) {
 // entry (nk_problem.cu); the FP64 operator kernels carry block reductions and keep the fixed rule.
 enum StripKernel { STRIP_OPERATOR = 0, STRIP_SMOOTH = 1, STRIP_RESIDUAL = 2 };
 int strip_rows(int nx, int ny, int elem_bytes, int kind = STRIP_OPERATOR);
-constexpr int STRIP_MIN_ROWS = 1;
 
 // Calls f(std::integral_constant<int, R>) for the supported walk lengths R.
 template <typename F>
@@ -91,7 +89,9 @@ struct NoExtra {};
 // extra(k) returned.  Every lane of the warp must call this (shuffles); lanes with nothing to do pass through.
 // IU / IV: the mask bits of the identity rows (q = p).  A caller whose own rule already fixes the prescribed rows
 // may pass U_INACTIVE / V_INACTIVE, the bits of the strain-rate reads, which then serve both tests.
-template <int R, uint8_t IU = U_IDENTITY, uint8_t IV = V_IDENTITY, typename T, typename Src, typename Extra, typename Emit>
+// UNI: on a regular square grid (DevGrid::h != 0) the metric factors cancel as in strip_apply_uniform, whose expressions
+// it then uses, and no metric is loaded.
+template <int R, bool UNI, uint8_t IU = U_IDENTITY, uint8_t IV = V_IDENTITY, typename T, typename Src, typename Extra, typename Emit>
 __device__ __forceinline__ void strip_apply_general(const OpView<T>& o, Src&& src, int i, int j0, Extra&& extra, Emit&& emit) {
     using V2 = typename Vec2<T>::type;
     using V4 = typename Vec4<T>::type;
@@ -103,11 +103,14 @@ __device__ __forceinline__ void strip_apply_general(const OpView<T>& o, Src&& sr
     const bool own_col = lane >= 1 && lane <= STRIP_COLS && i < g.Nx;
     T rdxc_i = T(0), dxc_i = T(0), rdxf_i = T(0), dxf_i = T(0);
     int cxi = 0, fxi = 0;
+    const T h2 = UNI ? g.h * g.h : T(0);
     if (col_ok) {
-        rdxc_i = g.rdxc[i];
-        dxc_i = g.dxc[i];
-        rdxf_i = g.rdxf[i];
-        dxf_i = g.dxf[i];
+        if (!UNI) {
+            rdxc_i = g.rdxc[i];
+            dxc_i = g.dxc[i];
+            rdxf_i = g.rdxf[i];
+            dxf_i = g.dxf[i];
+        }
         cxi = g.cx(i);
         fxi = g.fx(i);
     }
@@ -128,15 +131,17 @@ __device__ __forceinline__ void strip_apply_general(const OpView<T>& o, Src&& sr
         V4 z;
         z.x = T(0); z.y = T(0); z.z = T(0); z.w = T(0);
         rec[r] = okc ? o.coef[g.idx(cxi, g.cy(jc))] : z;
-        rdyc[r] = okc ? g.rdyc[jc] : T(0);
-        dyc[r] = okc ? g.dyc[jc] : T(0);
         cff[r] = okf ? o.coef[g.idx(fxi, g.fy(jf))].y : T(0);
-        rdyf[r] = okf ? g.rdyf[jf] : T(0);
+        if (!UNI) {
+            rdyc[r] = okc ? g.rdyc[jc] : T(0);
+            dyc[r] = okc ? g.dyc[jc] : T(0);
+            rdyf[r] = okf ? g.rdyf[jf] : T(0);
+        }
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         int j = j0 + r;
-        dyf[r] = (col_ok && j <= g.Ny) ? g.dyf[j] : T(0);
+        if (!UNI) dyf[r] = (col_ok && j <= g.Ny) ? g.dyf[j] : T(0);
         if (own_col && j < g.Ny) ex[r] = extra(g.idx(i, j));
     }
 
@@ -144,6 +149,12 @@ __device__ __forceinline__ void strip_apply_general(const OpView<T>& o, Src&& sr
     auto centre = [&](int a, int c, T& sxx, T& syy) {
         T mu = row[a].mu(), mv = row[a].mv(), mvn = row[a + 1].mv();
         T mue = __shfl_down_sync(full, mu, 1);
+        if (UNI) {
+            T du = mue - mu, dv = mvn - mv;
+            sxx = rec[c].x * (T(2) * du + dv);
+            syy = rec[c].x * (T(2) * dv + du);
+            return;
+        }
         T exx = (mue - mu) * rdxc_i;
         T eyy = (mvn - mv) * rdyc[c];
         T eta = rec[c].x;
@@ -154,6 +165,11 @@ __device__ __forceinline__ void strip_apply_general(const OpView<T>& o, Src&& sr
     auto corner = [&](int a, int c, int j) -> T {
         T mu = row[a].mu(), mus = row[a - 1].mu(), mv = row[a].mv();
         T mvw = __shfl_up_sync(full, mv, 1);
+        if (UNI) {
+            T e = cff[c] * ((mu - mus) + (mv - mvw));
+            if (per_ff_x || g.out_y(j) || g.out_y(j - 1)) e = o.wall_factor * e;
+            return e;
+        }
         T dudy = (mu - mus) * rdyf[c];
         T dvdx = (mv - mvw) * rdxf_i;
         // 2 η̄Hᶠᶠ ε̇xy with ε̇xy = (dudy + dvdx) / 2 (× the wall factor), written as η̄Hᶠᶠ (dudy + dvdx): the
@@ -178,11 +194,18 @@ __device__ __forceinline__ void strip_apply_general(const OpView<T>& o, Src&& sr
         if (own_col && j < g.Ny) {
             const V4& c = rec[r + 1];             // the record of (i, j) itself: cx(i) = i, cy(j) = j here
             const V2& x = row[r + 1].raw;
-            T divu = (sxx - sxx_w) + (dxf_i * t_n - dxf_i * t_c);
-            T divv = (syy - syy_s) + (dyf[r] * t_e - dyf[r] * t_c);
             V2 q;
-            q.x = (row[r + 1].m & IU) ? x.x : (dxf_i * dyc[r + 1]) * c.z * x.x - divu;
-            q.y = (row[r + 1].m & IV) ? x.y : (dxc_i * dyf[r]) * c.w * x.y - divv;
+            if (UNI) {
+                T divu = T(2) * (sxx - sxx_w) + (t_n - t_c);
+                T divv = T(2) * (syy - syy_s) + (t_e - t_c);
+                q.x = (row[r + 1].m & IU) ? x.x : h2 * c.z * x.x - divu;
+                q.y = (row[r + 1].m & IV) ? x.y : h2 * c.w * x.y - divv;
+            } else {
+                T divu = (sxx - sxx_w) + (dxf_i * t_n - dxf_i * t_c);
+                T divv = (syy - syy_s) + (dyf[r] * t_e - dyf[r] * t_c);
+                q.x = (row[r + 1].m & IU) ? x.x : (dxf_i * dyc[r + 1]) * c.z * x.x - divu;
+                q.y = (row[r + 1].m & IV) ? x.y : (dxc_i * dyf[r]) * c.w * x.y - divv;
+            }
             emit(g.idx(i, j), q, x, ex[r]);
         }
         syy_s = syy;
@@ -316,13 +339,13 @@ __device__ __forceinline__ void strip_apply_uniform(const OpView<T>& o, Src&& sr
     auto mv = [&](int a) { return (msk[a] & V_INACTIVE) ? T(0) : raw[a].y; };
     auto cff = [&](int c) { return c < R ? rec[c + 1].y : cffR; };
 
+    // η̄H (2 Δu + Δv) and η̄H (2 Δv + Δu): half the stresses, whose doubling joins the divergence (exact)
     auto centre = [&](int a, int c, T& sxx, T& syy) {
         T u0 = mu(a), v0 = mv(a), vn = mv(a + 1);
         T ue = __shfl_down_sync(full, u0, 1);
         T du = ue - u0, dv = vn - v0;
-        T e2 = T(2) * rec[c].x;
-        sxx = e2 * (T(2) * du + dv);
-        syy = e2 * (T(2) * dv + du);
+        sxx = rec[c].x * (T(2) * du + dv);
+        syy = rec[c].x * (T(2) * dv + du);
     };
     auto corner = [&](int a, int c) -> T {   // Δx × the corner shear (= Δy × it)
         T u0 = mu(a), us = mu(a - 1), v0 = mv(a);
@@ -343,8 +366,8 @@ __device__ __forceinline__ void strip_apply_uniform(const OpView<T>& o, Src&& sr
         if (own_col) {
             const V4& c = rec[r + 1];
             const V2& x = raw[r + 1];
-            T divu = (sxx - sxx_w) + (t_n - t_c);
-            T divv = (syy - syy_s) + (t_e - t_c);
+            T divu = T(2) * (sxx - sxx_w) + (t_n - t_c);
+            T divv = T(2) * (syy - syy_s) + (t_e - t_c);
             V2 q;
             q.x = (msk[r + 1] & IU) ? x.x : h2 * c.z * x.x - divu;
             q.y = (msk[r + 1] & IV) ? x.y : h2 * c.w * x.y - divv;
@@ -363,7 +386,8 @@ __device__ __forceinline__ void strip_apply_src(const OpView<T>& o, Src&& src, i
     const bool interior = i_first >= 1 && i_first + 31 <= o.g.Nx - 2 && j0 - 1 >= 1 && j0 + R <= o.g.Ny - 2;
     if (interior && o.g.h != decltype(o.g.h)(0)) strip_apply_uniform<R, IU, IV>(o, src, i, j0, extra, emit);
     else if (interior) strip_apply_interior<R, IU, IV>(o, src, i, j0, extra, emit);
-    else strip_apply_general<R, IU, IV>(o, src, i, j0, extra, emit);
+    else if (o.g.h != decltype(o.g.h)(0)) strip_apply_general<R, true, IU, IV>(o, src, i, j0, extra, emit);
+    else strip_apply_general<R, false, IU, IV>(o, src, i, j0, extra, emit);
 }
 
 // strip_apply_src with the operand read from an array.
@@ -373,11 +397,201 @@ __device__ __forceinline__ void strip_apply(const OpView<T>& o, const typename V
     strip_apply_src<R, IU, IV>(o, [p](int k, int, int) { return p[k]; }, i, j0, extra, emit);
 }
 
+// ---- long walks -------------------------------------------------------------------------------------------------
+// The same walk over any number of rows, one row of operands ahead of the arithmetic, with the previous row in registers:
+// the two rows that a walk reads besides its own are shared by all of them, where the unrolled walks of R rows share them
+// by R.  For the FP64 kernels of large grids, which the FP64 pipe binds: k_cg_apply at 1024 x 512 takes 41 us, 30 FP64
+// instructions a cell, against 58 us and 34 with walks of 4 rows.
+//
+// One lane's column of the walk: push(row j + 1) returns the divergence of row j.
+template <typename T, bool UNI>
+struct StripColumn {
+    const DevGrid<T>& g;
+    T wall_factor, rdxc, dxc, rdxf, dxf;
+    bool wall_x;
+    T mu, mv, sy, t;           // the last row pushed, Δx Tyy of the centre below it and the shear of its corner
+    __device__ __forceinline__ StripColumn(const OpView<T>& o, int i, bool col_ok)
+        : g(o.g), wall_factor(o.wall_factor), rdxc(T(0)), dxc(T(0)), rdxf(T(0)), dxf(T(0)), mu(T(0)), mv(T(0)), sy(T(0)), t(T(0)) {
+        wall_x = g.out_x(i) || g.out_x(i - 1);
+        if (!UNI && col_ok) {
+            rdxc = g.rdxc[i]; dxc = g.dxc[i]; rdxf = g.rdxf[i]; dxf = g.dxf[i];
+        }
+    }
+    // (un, vn): masked velocities of row j + 1; eta: η̄H of centre (i, j); cff: η̄Hᶠᶠ of corner (i, j + 1); jm: the metric
+    // index of row j (j itself, wrapped where a walk runs over a periodic edge)
+    __device__ __forceinline__ void push(int j, int jm, T un, T vn, T eta, T cff, T& divu, T& divv) {
+        const unsigned full = 0xffffffffu;
+        const T ue = __shfl_down_sync(full, mu, 1), vw = __shfl_up_sync(full, vn, 1);
+        const bool wall = wall_x || g.out_y(j + 1) || g.out_y(j);
+        T sx, syn, tn;
+        if (UNI) {
+            const T du = ue - mu, dv = vn - mv;
+            sx = eta * (T(2) * du + dv);
+            syn = eta * (T(2) * dv + du);
+            tn = cff * ((un - mu) + (vn - vw));
+            if (__any_sync(full, wall)) tn = wall ? wall_factor * tn : tn;   // a warp off the walls issues no product
+        } else {
+            const bool in = jm >= -1 && jm <= g.Ny - 1;
+            const T rdyc = in ? g.rdyc[jm] : T(0), dyc = in ? g.dyc[jm] : T(0), rdyf = in ? g.rdyf[jm + 1] : T(0);
+            const T exx = (ue - mu) * rdxc, eyy = (vn - mv) * rdyc;
+            sx = dyc * (T(2) * eta * (T(2) * exx + eyy));
+            syn = dxc * (T(2) * eta * (T(2) * eyy + exx));
+            T e = (un - mu) * rdyf + (vn - vw) * rdxf;
+            if (wall) e = wall_factor * e;
+            tn = cff * e;
+        }
+        const T sxw = __shfl_up_sync(full, sx, 1), te = __shfl_down_sync(full, t, 1);
+        if (UNI) {
+            divu = T(2) * (sx - sxw) + (tn - t);
+            divv = T(2) * (syn - sy) + (te - t);
+        } else {
+            const T dyf = jm >= 0 && jm < g.Ny ? g.dyf[jm] : T(0);
+            divu = (sx - sxw) + (dxf * tn - dxf * t);
+            divv = (syn - sy) + (dyf * te - dyf * t);
+        }
+        mu = un; mv = vn; sy = syn; t = tn;
+    }
+};
+
+// q = A p over rows j0 .. j1 - 1 of one warp strip; `load(k)` issues the reads of the operand at k, `value(loaded)` forms
+// it, `extra` and `emit` as in strip_apply_general.
+template <bool UNI, uint8_t IU = U_IDENTITY, uint8_t IV = V_IDENTITY, typename T, typename Load, typename Value, typename Extra, typename Emit>
+__device__ __forceinline__ void strip_march(const OpView<T>& o, Load&& load, Value&& value, int i, int j0, int j1, Extra&& extra, Emit&& emit) {
+    using V2 = typename Vec2<T>::type;
+    using V4 = typename Vec4<T>::type;
+    using L = decltype(load(0));
+    using E = decltype(extra(0));
+    const DevGrid<T>& g = o.g;
+    const int lane = threadIdx.x & 31;
+    const bool col_ok = i <= g.Nx, own_col = lane >= 1 && lane <= STRIP_COLS && i < g.Nx;
+    const bool ucol = g.px || (i >= 0 && i <= g.Nx), vcol = !g.out_x(i);
+    const int cxi = col_ok ? g.cx(i) : 0, fxi = col_ok ? g.fx(i) : 0, iw = col_ok ? (g.px ? g.wrap(i, g.Nx) : (i < 0 ? 0 : i)) : 0;
+    const T h2 = UNI ? g.h * g.h : T(0);
+    StripColumn<T, UNI> col(o, i, col_ok);
+    struct Row { L l; V4 rec; T cff; uint8_t m; bool u, v; };
+    auto fetch = [&](int j) {   // row j of the lane's column; every index is within the stored plane
+        Row r;
+        r.m = 0;
+        r.cff = T(0);
+        r.rec.x = r.rec.y = r.rec.z = r.rec.w = T(0);
+        const bool row_ok = col_ok && j <= g.Ny;
+        r.u = row_ok && ucol && !g.out_y(j);
+        r.v = row_ok && vcol && (g.py || j >= 0);
+        if (row_ok) {
+            r.rec = o.coef[g.idx(cxi, g.cy(j))];
+            r.cff = o.coef[g.idx(fxi, g.fy(j))].y;
+        }
+        if (r.u || r.v) {
+            const int k = g.idx(iw, g.py ? g.wrap(j, g.Ny) : j);
+            r.m = __ldg(o.mask + k);
+            r.l = load(k);
+        }
+        return r;
+    };
+    auto pair = [&](const Row& r) {
+        V2 x;
+        x.x = x.y = T(0);
+        if (r.u || r.v) x = value(r.l);
+        return x;
+    };
+    Row cur = fetch(j0 - 1), nxt = fetch(j0);
+    V2 x = pair(cur);
+    col.mu = (cur.u && !(cur.m & U_INACTIVE)) ? x.x : T(0);
+    col.mv = (cur.v && !(cur.m & V_INACTIVE)) ? x.y : T(0);
+    E ex{};
+    for (int j = j0 - 1; j < j1; ++j) {   // the first turn, row j0 - 1, only fills sy and t
+        Row pre = fetch(j + 2);
+        E exn{};
+        if (own_col && j + 1 < j1) exn = extra(g.idx(i, j + 1));
+        const V2 xn = pair(nxt);
+        const T un = (nxt.u && !(nxt.m & U_INACTIVE)) ? xn.x : T(0), vn = (nxt.v && !(nxt.m & V_INACTIVE)) ? xn.y : T(0);
+        T divu, divv;
+        col.push(j, j, un, vn, cur.rec.x, nxt.cff, divu, divv);
+        if (own_col && j >= j0) {
+            V2 q;
+            const T au = UNI ? h2 : g.dxf[i] * g.dyc[j], av = UNI ? h2 : g.dxc[i] * g.dyf[j];
+            q.x = (cur.m & IU) ? x.x : au * cur.rec.z * x.x - divu;
+            q.y = (cur.m & IV) ? x.y : av * cur.rec.w * x.y - divv;
+            emit(g.idx(i, j), q, x, ex);
+        }
+        cur = nxt;
+        nxt = pre;
+        x = xn;
+        ex = exn;
+    }
+}
+
+// Launch shape of the FP64 operator kernels: rows per walk, warps per block, blocks.  rows > 0: unrolled walks
+// (strip_apply); rows < 0: long walks (strip_march) of -rows rows.
+struct OperatorShape {
+    int rows;
+    LaunchDims d;
+};
+inline OperatorShape operator_shape(int nx, int ny, int forced) {
+    OperatorShape s;
+    const long long across = (nx + STRIP_COLS - 1) / STRIP_COLS;
+    int rows = forced, warps;
+    long long tasks;
+    if (!forced && across * ny > 20ll * SM_COUNT) {
+        // Long walks, the number of rows that finishes the busiest SM first: a walk costs its rows and one and a half
+        // more, an SM takes the walks in turn, and four to twelve warps keep its FP64 pipe busy.
+        double best = 0;
+        for (int r = 4; r <= 64; ++r) {
+            const long long n = across * ((ny + r - 1) / r), per = (n + SM_COUNT - 1) / SM_COUNT;
+            if (r > 4 && per < 4) break;
+            const double cost = (double)per * (r + 1.5) * (per > 12 ? 1.05 : 1.0);
+            if (r == 4 || cost < best) { best = cost; rows = -r; }
+        }
+        tasks = across * ((ny - rows - 1) / -rows);
+        warps = 2;
+    } else {
+        // Unrolled walks: one row while that leaves a warp an SM quarter to itself, so that the serial chain of FP64
+        // instructions (64 cycles each) is the shortest (256 x 128: 10.3 us, 10.9 with two rows and 13.9 with four), else two.
+        if (!forced) rows = across * ny <= 8ll * SM_COUNT ? 1 : 2;
+        tasks = across * ((ny + rows - 1) / rows);
+        warps = tasks <= 2ll * SM_COUNT ? 1 : (tasks <= 4ll * SM_COUNT ? 2 : STRIP_WARPS);
+    }
+    const long long resident = 8ll * SM_COUNT;
+    long long blocks = (tasks + warps - 1) / warps;
+    s.rows = rows;
+    s.d.block = dim3(32, warps);
+    s.d.grid = dim3((unsigned)(blocks < resident ? blocks : resident), 1, batch_slots());
+    return s;
+}
+// Calls walk(i, j0) for every strip of R rows of the calling warp in a launch of operator_shape
+template <typename F>
+__device__ __forceinline__ void for_each_strip(int Nx, int Ny, int R, F&& walk) {
+    const int across = (Nx + STRIP_COLS - 1) / STRIP_COLS, n = across * ((Ny + R - 1) / R);
+    for (int t = (int)(threadIdx.y * gridDim.x + blockIdx.x); t < n; t += (int)(gridDim.x * blockDim.y)) {
+        const int row = t / across;
+        walk((t - row * across) * STRIP_COLS - 1 + (int)threadIdx.x, row * R);
+    }
+}
+// q = A p over rows j0 .. min(j0 + R, Ny) - 1 by the walk that operator_shape chose: R > 0 unrolled, R = 0 a long walk of `rows`.
+template <int R, uint8_t IU = U_IDENTITY, uint8_t IV = V_IDENTITY, typename T, typename Load, typename Value, typename Extra, typename Emit>
+__device__ __forceinline__ void strip_walk(const OpView<T>& o, int rows, Load&& load, Value&& value, int i, int j0, Extra&& extra, Emit&& emit) {
+    if constexpr (R > 0) {
+        strip_apply_src<R, IU, IV>(o, [&](int k, int, int) { return value(load(k)); }, i, j0, extra, emit);
+    } else {
+        const int j1 = j0 + rows < o.g.Ny ? j0 + rows : o.g.Ny;
+        if (o.g.h != decltype(o.g.h)(0)) strip_march<true, IU, IV>(o, load, value, i, j0, j1, extra, emit);
+        else strip_march<false, IU, IV>(o, load, value, i, j0, j1, extra, emit);
+    }
+}
+// Calls f(std::integral_constant<int, R>, rows): R = 0 for long walks of `rows` rows
+template <typename F>
+inline void with_operator_rows(int rows, F&& f) {
+    if (rows < 0) f(std::integral_constant<int, 0>{}, -rows);
+    else if (rows == 1) f(std::integral_constant<int, 1>{}, 1);
+    else if (rows == 2) f(std::integral_constant<int, 2>{}, 2);
+    else f(std::integral_constant<int, 4>{}, 4);
+}
+
 // Column and first row of the calling thread in a strip launch of R rows per warp (strip_dims).
 template <int R>
 __device__ __forceinline__ void strip_origin(int& i, int& j0) {
     i = blockIdx.x * STRIP_COLS - 1 + (int)threadIdx.x;
-    j0 = (blockIdx.y * STRIP_WARPS + (int)threadIdx.y) * R;
+    j0 = (blockIdx.y * blockDim.y + (int)threadIdx.y) * R;
 }
 
 }  // namespace nk

@@ -88,3 +88,69 @@ def test_coarse_levels_in_a_cluster(oracle_cls, gpu_cls, nx, ny, topology, sweep
     for g, w in zip(got, want):
         g, w = g[:ny, :nx], w[:ny, :nx]
         assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
+
+
+# The conjugate-gradient kernels at the sizes where their launch shapes change: one row a walk (up to 8 strip rows an SM),
+# two rows, long walks (more than 20 strip rows an SM) with a remainder of rows, blocks of 1, 2 and more warps, widths of
+# 30 k and 32 k columns and one beside, a periodic seam, faces that are not square.  Ten steps from rest against the
+# oracle's: the operator's sums round at 1e-16 of their terms, ten steps carry that to 1e-12 of the largest velocity.
+@gpu
+@pytest.mark.parametrize("nx, ny, topology, stretch", [
+    (30, 9, ("Bounded", "Bounded"), 1.0),
+    (33, 40, ("Periodic", "Bounded"), 1.0),
+    (61, 64, ("Bounded", "Periodic"), 1.0),
+    (128, 61, ("Bounded", "Bounded"), 1.25),
+    (301, 131, ("Bounded", "Bounded"), 1.0),
+    (420, 215, ("Periodic", "Periodic"), 1.0),
+    (481, 203, ("Bounded", "Bounded"), 1.0),
+    (513, 190, ("Periodic", "Bounded"), 0.8),
+])
+def test_cg_steps_at_the_launch_shapes_edges(oracle_cls, gpu_cls, nx, ny, topology, stretch):
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 2e3 * stretch), topology=topology)
+    solver = nk.StressBalanceSolver(linear_iteration_control=nk.FixedIterations(10), picard_iteration_control=nk.FixedIterations(1))
+    desc = nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                               stress_balance=nk.DepthIntegrated(side_walls=nk.NoSlipWalls()), velocity_solver=solver)
+    H = np.clip(1000.0 + 300.0 * np.random.default_rng(nx).standard_normal((ny, nx)), 0.0, None)
+    H[ny // 3: ny // 3 + 2] = 0.0
+    out = []
+    for cls in (gpu_cls, oracle_cls):
+        P = cls(grid, desc)
+        for n, a in (("H", H), ("bed", 10.0), ("C", 1e9), ("A", 3e-24)):
+            P.set(n, a)
+        P.compute_geometry()
+        st = P.picard_solve()
+        out.append((P.get("u"), P.get("v")))
+        assert st.linear_iterations_total == 10
+        P.close()
+    for g, w in zip(*out):
+        assert np.max(np.abs(g - w)) <= 1e-12 * np.max(np.abs(w))
+
+
+# The FP64 <-> FP32 conversions on the integer units are the hardware conversions' bits, so a mixed solve keeps its
+# residuals' scale: right-hand sides far outside the FP32 range (2^-400 to 2^400, whose squared norms FP64 still holds)
+# converge in the same steps, to the same digits, as those near one.
+@gpu
+@pytest.mark.parametrize("exponent", [-400, -300, 300, 400])
+def test_mixed_solve_scales_with_its_right_hand_side(gpu_cls, exponent):
+    nx, ny = 64, 40
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 2e3))
+    solver = nk.StressBalanceSolver(linear_iteration_control=nk.Convergence(reltol=1e-12, maxiter=200), precision="mixed",
+                                    preconditioner=nk.StressBalanceMultigridPreconditioner(minimum_coarse_size=8))
+    P = gpu_cls(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                                          velocity_solver=solver))
+    for n, a in (("H", 1000.0), ("bed", 10.0), ("C", 1e9), ("A", 3e-24), ("u", 1e-6), ("v", 0.0)):
+        P.set(n, a)
+    P.compute_geometry()
+    P.update_coefficients()
+    rng = np.random.default_rng(5)
+    bu, bv = rng.standard_normal(P.shape("u")), rng.standard_normal(P.shape("v"))
+    res = []
+    for scale in (1.0, 2.0 ** exponent):
+        P.set("u", 0.0)
+        P.set("v", 0.0)
+        st = P.linear_solve(bu * scale, bv * scale)
+        res.append((P.get("u") / scale, P.get("v") / scale, st.linear_iterations_total, st.status))
+    P.close()
+    assert res[0][2:] == res[1][2:]
+    for a, b in zip(res[0][:2], res[1][:2]):
+        assert np.array_equal(a, b)
