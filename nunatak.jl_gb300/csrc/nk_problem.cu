@@ -1724,13 +1724,11 @@ static void check_thickness_step(nk_problem* P, double dt) {
 // the stage's thickness, sets H = max(0, H_start + Δτ G(H)), the last adds its clip and advances a front; then the
 // geometry (rk_substep! and update_state! without the velocity solve, time_stepping.jl:15-25).
 static void thickness_stage(nk_problem* P, double dt, int st, int coupling) {
-    const bool bounded = P->advection.scheme == NK_ADVECTION_WENO && P->advection.bounded;
     ThicknessView v = thickness_view(P, coupling != 0);
     if (st == 0) NK_CUDA(cudaMemcpyAsync((double*)v.H0, P->H, P->plane * sizeof(double), cudaMemcpyDeviceToDevice, P->stream));
     const double stages[3] = {1.0 / 3, 1.0 / 2, 1.0};     // SplitRungeKutta3 (Wicker-Skamarock) fractions
     NK_CUDA(cudaMemcpyAsync((double*)v.Hs, P->H, P->plane * sizeof(double), cudaMemcpyDeviceToDevice, P->stream));
     if (v.fx) launch_thickness_faces(v, P->stream);
-    if (bounded) launch_thickness_limiter(v, P->stream);
     launch_thickness_stage(v, stages[st] * dt, st == 2, P->stream);
     if (st == 2 && P->front.enabled)   // rk_substep!: advance_front! after the final stage (time_stepping.jl:23)
         launch_advance_front(front_view(P, coupling != 0), P->front.passes, stages[st] * dt, P->plane, P->stream);
@@ -2283,7 +2281,6 @@ struct TimeGradient {
         NK_CUDA(cudaMemcpyAsync((double*)tv.Hs, P->H, pl * sizeof(double), cudaMemcpyDeviceToDevice, s));
         NK_CUDA(cudaMemcpyAsync((double*)tv.H0, tape(3 * k), pl * sizeof(double), cudaMemcpyDeviceToDevice, s));
         if (tv.fx) launch_thickness_faces(tv, s);
-        if (P->advection.scheme == NK_ADVECTION_WENO && P->advection.bounded) launch_thickness_limiter(tv, s);
         NK_CUDA(cudaMemsetAsync(lamx_stage, 0, pl * sizeof(double2), s));
         StageAdjointView a;
         a.t = tv;
@@ -2322,7 +2319,6 @@ struct TimeGradient {
         NK_CUDA(cudaMemcpyAsync((double*)tv.Hs, P->H, pl * sizeof(double), cudaMemcpyDeviceToDevice, s));
         NK_CUDA(cudaMemcpyAsync((double*)tv.H0, tape(3 * k), pl * sizeof(double), cudaMemcpyDeviceToDevice, s));
         if (tv.fx) launch_thickness_faces(tv, s);
-        if (P->advection.scheme == NK_ADVECTION_WENO && P->advection.bounded) launch_thickness_limiter(tv, s);
         launch_thickness_stage(tv, last * d.dt, 1, s);   // P->H = the output before the front (the clip is restored at the end)
         NK_CUDA(cudaMemcpyAsync(h3pre, P->H, pl * sizeof(double), cudaMemcpyDeviceToDevice, s));
         // the advance again on copies, recorded pass by pass
@@ -2684,9 +2680,7 @@ nk_status nk_time_kernel(nk_problem* P, int32_t kernel, int32_t repeats, int64_t
                 launch_cg_update(v, s);
             } else if (kernel == NK_KERNEL_THICKNESS_STAGE) {
                 launch_thickness_stage(tv, 1.0, 0, s);
-            } else if (kernel == NK_KERNEL_THICKNESS_LIMITER) {
-                launch_thickness_limiter(tv, s);
-            } else if (kernel == NK_KERNEL_THICKNESS_FACES) {
+            } else if (kernel == NK_KERNEL_THICKNESS_FACES || kernel == NK_KERNEL_THICKNESS_LIMITER) {   // one kernel for both
                 launch_thickness_faces(tv, s);
             } else if (kernel == NK_KERNEL_STEP_ENTHALPY) {
                 launch_step_enthalpy(ev, 1.0, s);
@@ -2703,19 +2697,17 @@ nk_status nk_time_kernel(nk_problem* P, int32_t kernel, int32_t repeats, int64_t
         // (a WENO stage reads the face reconstructions, one pair per x and per y face of the cell, instead of the stencils)
         else if (kernel == NK_KERNEL_THICKNESS_STAGE)
             bytes = cells * (8 + 8 + 8 + 8 + 16 + 8 + (P->pd.grounding ? 8 : 0) + (bounded ? 8 : 0) + (weno ? 32 : 0));
-        else if (kernel == NK_KERNEL_THICKNESS_LIMITER) bytes = cells * (8 + 8 + 32);
-        else if (kernel == NK_KERNEL_THICKNESS_FACES) bytes = cells * (8 + 32);
+        else if (kernel == NK_KERNEL_THICKNESS_FACES || kernel == NK_KERNEL_THICKNESS_LIMITER) bytes = cells * (8 + 32 + (bounded ? 8 : 0));
         // per column: H, Hⁿ, φ, m, mᵍ, G, Tₛ, Tₒ, H_w, (u, v), (uᵇ, vᵇ) and the drag; per layer E_old, η, (uσ, vσ) read and E,
         // T, ω, Φ written
         else if (kernel == NK_KERNEL_STEP_ENTHALPY) bytes = cells * 8 * (11 + 8.0 * P->Ns);
         if (kernel == NK_KERNEL_THICKNESS_STAGE || kernel == NK_KERNEL_THICKNESS_LIMITER || kernel == NK_KERNEL_THICKNESS_FACES) {
             tv = thickness_view(P, false);
-            if (kernel == NK_KERNEL_THICKNESS_FACES && !tv.fx) bad("the face reconstructions belong to the WENO schemes");
+            if (kernel != NK_KERNEL_THICKNESS_STAGE && !tv.fx) bad("the face reconstructions belong to the WENO schemes");
             NK_CUDA(cudaMemcpyAsync((double*)tv.Hs, P->H, P->plane * sizeof(double), cudaMemcpyDeviceToDevice, s));
             NK_CUDA(cudaMemcpyAsync((double*)tv.H0, P->H, P->plane * sizeof(double), cudaMemcpyDeviceToDevice, s));
             if (tv.fx) launch_thickness_faces(tv, s);
             if (kernel == NK_KERNEL_THICKNESS_STAGE && !bounded) tv.bounded = 0;
-            if (kernel == NK_KERNEL_THICKNESS_STAGE && bounded) launch_thickness_limiter(tv, s);
         } else if (kernel == NK_KERNEL_STEP_ENTHALPY) {
             if (P->pd.rate_factor_layout != NK_RATE_FACTOR_SIGMA || P->Ns > ENERGY_MAX_LAYERS) bad("the energy step needs the sigma rate factor");
             nk_energy_params q = default_energy_params();

@@ -26,23 +26,33 @@ __device__ __forceinline__ void stencil_y(const DevGrid<double>& g, const double
 }
 // WENO-5: the three third-order candidates, their Jiang-Shu smoothness indicators and the WENO-Z weights
 // α_k = d_k (1 + τ / (β_k + ε)), τ = |β₀ - β₂|, ε = 1e-8, d = (1, 6, 3) / 10 (Jiang and Shu 1996; Borges et al. 2008,
-// exponent 1).
+// exponent 1).  Both reconstructions of one cell from s[m + 2] = its neighbours m = -2..2: `plus` at the face towards
+// m > 0 and `minus` at the other.  The two share their indicators (mirrored: β₀ and β₂ change places), the weights'
+// numerators over the common denominator Π(β_k + ε) and, over the product of the weights' sums, one division; the
+// candidates are differences from the cell, so that all of it is 68 FP64 instructions a pair, 162 when each face's two
+// reconstructions were evaluated by themselves.
+__device__ __forceinline__ void weno5_cell(const double* s, double& plus, double& minus) {
+    const double c = s[2];
+    const double d1 = s[1] - s[0], d2 = c - s[1], d3 = s[3] - c, d4 = s[4] - s[3];
+    const double D0 = d2 - d1, D1 = d3 - d2, D2 = d4 - d3;                       // second differences
+    const double B0 = fma(2.0, d2, D0), B1 = d2 + d3, B2 = fma(-2.0, d3, D2);    // a - 4b + 3c, d - b, 3c - 4d + e
+    const double eps = 1e-8, w13 = 13.0 / 12;
+    const double e0 = fma(w13, D0 * D0, fma(0.25, B0 * B0, eps)), e1 = fma(w13, D1 * D1, fma(0.25, B1 * B1, eps)),
+                 e2 = fma(w13, D2 * D2, fma(0.25, B2 * B2, eps));
+    const double tau = fabs(e0 - e2);
+    const double p0 = (e0 + tau) * (e1 * e2), p1 = (e1 + tau) * (e0 * e2), p2 = (e2 + tau) * (e0 * e1);
+    const double p16 = 6 * p1, q0 = 3 * p0, q2 = 3 * p2;
+    const double S = p0 + p16 + q2, M = p2 + p16 + q0;                           // the weights' sums, times 10
+    const double g0 = fma(5.0, d2, -2.0 * d1), g1 = fma(2.0, d3, d2), g2 = fma(4.0, d3, -d4);   // 6 (candidate - c)
+    const double h0 = fma(5.0, d3, -2.0 * d4), h1 = fma(2.0, d2, d3), h2 = fma(4.0, d2, -d1);   // 6 (c - candidate)
+    const double r = (1.0 / 6) / (S * M);
+    plus = fma(fma(p0, g0, fma(p16, g1, q2 * g2)) * M, r, c);
+    minus = fma(-(fma(p2, h0, fma(p16, h1, q0 * h2)) * S), r, c);
+}
 __device__ __forceinline__ double weno5_face(const double* s) {
-    const double a = s[0], b = s[1], c = s[2], d = s[3], e = s[4];
-    const double sixth = 1.0 / 6;
-    double q0 = (2 * a - 7 * b + 11 * c) * sixth;
-    double q1 = (-b + 5 * c + 2 * d) * sixth;
-    double q2 = (2 * c + 5 * d - e) * sixth;
-    double b0 = 13.0 / 12 * (a - 2 * b + c) * (a - 2 * b + c) + 0.25 * (a - 4 * b + 3 * c) * (a - 4 * b + 3 * c);
-    double b1 = 13.0 / 12 * (b - 2 * c + d) * (b - 2 * c + d) + 0.25 * (b - d) * (b - d);
-    double b2 = 13.0 / 12 * (c - 2 * d + e) * (c - 2 * d + e) + 0.25 * (3 * c - 4 * d + e) * (3 * c - 4 * d + e);
-    const double eps = 1e-8;
-    double tau = fabs(b0 - b2);
-    // αₖ = dₖ (1 + τ / (βₖ + ε)) over the common denominator Π(βₖ + ε): one FP64 division per face instead of four
-    // (the weights' ratio is unchanged; the rounding differs from the separate quotients in the last bits)
-    double e0 = b0 + eps, e1 = b1 + eps, e2 = b2 + eps;
-    double a0 = 0.1 * (e0 + tau) * (e1 * e2), a1 = 0.6 * (e1 + tau) * (e0 * e2), a2 = 0.3 * (e2 + tau) * (e0 * e1);
-    return (a0 * q0 + a1 * q1 + a2 * q2) / (a0 + a1 + a2);
+    double plus, minus;
+    weno5_cell(s, plus, minus);
+    return plus;
 }
 __device__ __forceinline__ double face_value(const ThicknessView& v, const double* s) {
     if (v.scheme == NK_ADVECTION_WENO) return weno5_face(s);

@@ -154,3 +154,38 @@ def test_mixed_solve_scales_with_its_right_hand_side(gpu_cls, exponent):
     assert res[0][2:] == res[1][2:]
     for a, b in zip(res[0][:2], res[1][:2]):
         assert np.array_equal(a, b)
+
+
+# The thickness stages with each cell's WENO reconstructions and limiter in one kernel: axes shorter and longer than a
+# stencil's wrap, widths beside 32, both periodic seams, no bounds, bounds out of reach (no division) and bounds that the
+# reconstructions pass (the limiter divides), an ice-free margin.  Reconstructions round at 1e-16 of the thickness, the
+# shared denominators at a few more; three stages carry that to 1e-12 of the largest thickness.
+@gpu
+@pytest.mark.parametrize("bounds", [None, (0.0, 1e5), (200.0, 900.0)])
+@pytest.mark.parametrize("nx, ny, topology", [(5, 7, ("Periodic", "Periodic")), (33, 9, ("Bounded", "Periodic")), (31, 40, ("Periodic", "Bounded")),
+                                              (64, 33, ("Bounded", "Bounded"))])
+def test_weno_faces_and_limiter(oracle_cls, gpu_cls, nx, ny, topology, bounds):
+    rng = np.random.default_rng(nx + 7 * ny)
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 1e3), y=(0.0, ny * 1.3e3), topology=topology, halo=(4, 4))
+    desc = nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                               grounding=nk.SubgridGroundedFraction())
+    H = 550.0 + 340.0 * np.tanh(rng.standard_normal((ny, nx)))
+    if bounds != (200.0, 900.0):
+        H[: max(1, ny // 4), : max(1, nx // 4)] = 0.0
+    out = []
+    for cls in (gpu_cls, oracle_cls):
+        P = cls(grid, desc)
+        r = np.random.default_rng(3)
+        P.set("H", H)
+        P.set("bed", -450.0)
+        P.set("u", 1e-5 * r.standard_normal(P.shape("u")))
+        P.set("v", 1e-5 * r.standard_normal(P.shape("v")))
+        P.energy_set("surface_mass_balance", 1e-8)
+        P.energy_set("basal_melt_rate", 2e-8)
+        P.set_thickness_advection(nk.WENO(order=5, bounds=bounds))
+        P.compute_geometry()
+        P.step_thickness(5e6)
+        out.append([P.get(n) for n in ("H", "tau_u", "tau_v")] + [P.energy_get("clipped_thickness")])
+        P.close()
+    for g, w in zip(*out):
+        assert np.max(np.abs(g - w)) <= 1e-12 * max(np.max(np.abs(w)), 1.0)
