@@ -401,6 +401,13 @@ struct CoarseLevels {
 };
 template <typename T>
 void launch_coarse_vcycle(const CoarseLevels<T>& C, const int* done, cudaStream_t s);
+// One half of a V-cycle's visit to a level in one pass (nk_vcycle.cu; two sweeps each way, both axes halved).  Down:
+// x2 = two sweeps from zero on L.b, C.b = R (L.b - A x2).  Up: xout = two sweeps on x2 + P xc.
+template <typename T>
+void launch_vcycle_down(const LevelView<T>& L, const LevelView<T>& C, typename Vec2<T>::type* x2, const int* done, cudaStream_t s);
+template <typename T>
+void launch_vcycle_up(const LevelView<T>& L, const LevelView<T>& C, const typename Vec2<T>::type* x2, const typename Vec2<T>::type* xc,
+                      typename Vec2<T>::type* xout, const int* done, cudaStream_t s);
 // The levels from lv[0] down to the coarsest, lv[n - 1], run by one thread-block cluster (nk_cluster.cu).
 template <typename T>
 struct ClusterLevels {

@@ -587,6 +587,44 @@ inline void with_operator_rows(int rows, F&& f) {
     else f(std::integral_constant<int, 4>{}, 4);
 }
 
+// One stage of a walk: push(row j + 1) gives the divergence of row j (cff: η̄Hᶠᶠ of corner (i, j + 1) times the wall
+// factor).
+template <typename T, bool UNI>
+struct Stage {
+    const DevGrid<T>& g;
+    T mu, mv, sy, t, rdxc, dxc, rdxf, dxf;
+    __device__ __forceinline__ Stage(const DevGrid<T>& grid, int iw) : g(grid), mu(T(0)), mv(T(0)), sy(T(0)), t(T(0)) {
+        if (!UNI) {
+            rdxc = g.rdxc[iw]; dxc = g.dxc[iw]; rdxf = g.rdxf[iw]; dxf = g.dxf[iw];
+        }
+    }
+    __device__ __forceinline__ void push(int jm, T un, T vn, T eta, T cff, T& divu, T& divv) {   // jm: the stored row of j
+        const unsigned full = 0xffffffffu;
+        const T ue = __shfl_down_sync(full, mu, 1), vw = __shfl_up_sync(full, vn, 1);
+        const T du = ue - mu, dv = vn - mv;
+        T sx, syn, tn;
+        if (UNI) {
+            sx = eta * (T(2) * du + dv);
+            syn = eta * (T(2) * dv + du);
+            tn = cff * ((un - mu) + (vn - vw));
+        } else {
+            const T exx = du * rdxc, eyy = dv * g.rdyc[jm], e2 = T(2) * eta;
+            sx = g.dyc[jm] * (e2 * (T(2) * exx + eyy));
+            syn = dxc * (e2 * (T(2) * eyy + exx));
+            tn = cff * ((un - mu) * g.rdyf[jm + 1] + (vn - vw) * rdxf);
+        }
+        const T sxw = __shfl_up_sync(full, sx, 1), te = __shfl_down_sync(full, t, 1);
+        if (UNI) {
+            divu = T(2) * (sx - sxw) + (tn - t);
+            divv = T(2) * (syn - sy) + (te - t);
+        } else {
+            divu = (sx - sxw) + dxf * (tn - t);
+            divv = (syn - sy) + g.dyf[jm] * (te - t);
+        }
+        mu = un; mv = vn; sy = syn; t = tn;
+    }
+};
+
 // Column and first row of the calling thread in a strip launch of R rows per warp (strip_dims).
 template <int R>
 __device__ __forceinline__ void strip_origin(int& i, int& j0) {

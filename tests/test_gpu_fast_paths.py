@@ -90,6 +90,45 @@ def test_coarse_levels_in_a_cluster(oracle_cls, gpu_cls, nx, ny, topology, sweep
         assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
 
 
+# One pass down and one up a level (FP32 levels above the cluster's 16384 cells, two sweeps, both axes halved): widths at
+# and beside multiples of the 26 and 28 columns that a warp writes, rows that do not divide by a walk, one and two such
+# levels, periodic seams, faces that are not square, walls with shear, ice-free cells.  Tolerance as above.
+@gpu
+@pytest.mark.parametrize("nx, ny, topology, stretch", [
+    (260, 66, ("Bounded", "Bounded"), 1.0),
+    (280, 62, ("Periodic", "Bounded"), 1.0),
+    (262, 90, ("Bounded", "Periodic"), 1.5),
+    (150, 130, ("Periodic", "Periodic"), 1.0),
+    (364, 210, ("Bounded", "Bounded"), 0.7),
+    (416, 224, ("Bounded", "Bounded"), 1.0),
+])
+def test_vcycle_halves(oracle_cls, gpu_cls, nx, ny, topology, stretch):
+    rng = np.random.default_rng(nx + ny)
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 2e3 * stretch), topology=topology)
+    mg = nk.StressBalanceMultigridPreconditioner(minimum_coarse_size=20)
+    H = np.clip(1000.0 + 400.0 * np.random.default_rng(1).standard_normal((ny, nx)), 0.0, None)
+    H[:, : nx // 8] = 0.0
+    H[ny // 2, :] = 0.0
+    ru, rv = 1e10 * rng.standard_normal((ny, grid.face_count(0))), 1e10 * rng.standard_normal((grid.face_count(1), nx))
+    z = []
+    for cls, precision in ((gpu_cls, "mixed"), (oracle_cls, "fp64")):
+        P = cls(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                                          stress_balance=nk.DepthIntegrated(side_walls=nk.NoSlipWalls()),
+                                          velocity_solver=nk.StressBalanceSolver(preconditioner=mg, precision=precision)))
+        for n, a in (("H", H), ("bed", 10.0), ("C", 1e9), ("A", 3e-24)):
+            P.set(n, a)
+        P.compute_geometry()
+        r = np.random.default_rng(2)
+        P.set("u", 1e-5 * r.standard_normal(P.shape("u")))
+        P.set("v", 1e-5 * r.standard_normal(P.shape("v")))
+        P.update_coefficients()
+        z.append(P.precondition(ru, rv))
+        P.close()
+    for g, w in zip(*z):
+        g, w = g[:ny, :nx], w[:ny, :nx]
+        assert np.max(np.abs(g - w)) <= 1e-4 * np.max(np.abs(w))
+
+
 # The conjugate-gradient kernels at the sizes where their launch shapes change: one row a walk (up to 8 strip rows an SM),
 # two rows, long walks (more than 20 strip rows an SM) with a remainder of rows, blocks of 1, 2 and more warps, widths of
 # 30 k and 32 k columns and one beside, a periodic seam, faces that are not square.  Ten steps from rest against the
