@@ -84,15 +84,16 @@ struct NoRead {
 };
 static int forced_operator_rows() { return strip_rows(0, 0, 8); }   // NK_STRIP_ROWS, or 0
 
-template <int R>
-__global__ void __launch_bounds__(32 * STRIP_WARPS) k_apply(OpView<double> o, const double2* __restrict__ p, double2* __restrict__ q, int rows) {
-    for_each_strip(o.g.Nx, o.g.Ny, rows, [&](int i, int j0) {
-        strip_walk<R>(o, rows, ReadPair{p}, SamePair{}, i, j0, NoRead{}, [&](int k, double2 a, double2, NoExtra) { q[k] = a; });
+template <bool UNI>
+__global__ void __launch_bounds__(64) k_apply(OpView<double> o, const double2* __restrict__ p, double2* __restrict__ q, int rows) {
+    for_each_strip(o.g.Nx, o.g.Ny, rows, [&](int i, int j0, int j1) {
+        strip_march<UNI>(o, ReadPair{p}, SamePair{}, i, j0, j1, NoRead{}, [&](int k, double2 a, double2, NoExtra) { q[k] = a; });
     });
 }
 void launch_apply(const OpView<double>& o, const double2* p, double2* q, cudaStream_t s) {
     OperatorShape d = operator_shape(o.g.Nx, o.g.Ny, forced_operator_rows());
-    with_operator_rows(d.rows, [&](auto r, int rows) { k_apply<decltype(r)::value><<<d.d.grid, d.d.block, 0, s>>>(o, p, q, rows); });
+    if (o.g.h != 0.0) k_apply<true><<<d.d.grid, d.d.block, 0, s>>>(o, p, q, d.rows);
+    else k_apply<false><<<d.d.grid, d.d.block, 0, s>>>(o, p, q, d.rows);
     count_launch();
 }
 
@@ -227,12 +228,12 @@ struct StopRule {
 };
 
 // conjugate_gradient!, conjugate_gradient.jl:165-171: r = b - A x, z = M r, p = z, rho = r.z
-template <int R>
-__global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_init(CGView v, int rows) {
+template <bool UNI>
+__global__ void __launch_bounds__(64) k_cg_init(CGView v, int rows) {
     NK_BATCH_ENTER(v.o.g, v)
     double rz = 0.0, rr = 0.0;
-    for_each_strip(v.o.g.Nx, v.o.g.Ny, rows, [&](int i, int j0) {
-        strip_walk<R>(v.o, rows, ReadPair{v.x}, SamePair{}, i, j0, ReadPair{v.b}, [&](int k, double2 q, double2, const double2& b) {
+    for_each_strip(v.o.g.Nx, v.o.g.Ny, rows, [&](int i, int j0, int j1) {
+        strip_march<UNI>(v.o, ReadPair{v.x}, SamePair{}, i, j0, j1, ReadPair{v.b}, [&](int k, double2 q, double2, const double2& b) {
             double2 r = make_double2(b.x - q.x, b.y - q.y);
             v.r[k] = r;   // the FP32 copy for the multigrid follows in k_cg_scale_r32, once ‖r0‖ is known
             rr += r.x * r.x + r.y * r.y;
@@ -268,7 +269,8 @@ __global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_init(CGView v, int rows
 }
 void launch_cg_init(const CGView& v, cudaStream_t s) {
     OperatorShape d = operator_shape(v.o.g.Nx, v.o.g.Ny, forced_operator_rows());
-    with_operator_rows(d.rows, [&](auto r, int rows) { k_cg_init<decltype(r)::value><<<d.d.grid, d.d.block, 0, s>>>(v, rows); });
+    if (v.o.g.h != 0.0) k_cg_init<true><<<d.d.grid, d.d.block, 0, s>>>(v, d.rows);
+    else k_cg_init<false><<<d.d.grid, d.d.block, 0, s>>>(v, d.rows);
     count_launch();
 }
 
@@ -322,8 +324,8 @@ void launch_cg_init_finish(const CGView& v, cudaStream_t s) {
 // walk and the columns beside a strip form their p twice, 3.2 FP64 instructions a cell instead of a pass of its own
 // over z and p (10 us of launch and traffic at 1024 x 512, 5 us at 128 x 64); a cell's p is written to the buffer that this
 // step's readers do not read.
-template <int R>
-__global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_apply(CGView v, int rows) {
+template <bool UNI>
+__global__ void __launch_bounds__(64) k_cg_apply(CGView v, int rows) {
     NK_BATCH_ENTER(v.o.g, v)
     if (read_done(v.sc)) return;
     const int it = v.sc->it, ze = v.sc->r32_exp;
@@ -345,8 +347,8 @@ __global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_apply(CGView v, int row
         double2 z = v.z32 ? make_double2(widen_pow2(a.z32.x, ze), widen_pow2(a.z32.y, ze)) : a.z;
         return first ? z : make_double2(z.x + beta * a.p.x, z.y + beta * a.p.y);
     };
-    for_each_strip(v.o.g.Nx, v.o.g.Ny, rows, [&](int i, int j0) {
-        strip_walk<R>(v.o, rows, load, value, i, j0, NoRead{}, [&](int k, double2 q, double2 p, NoExtra) {
+    for_each_strip(v.o.g.Nx, v.o.g.Ny, rows, [&](int i, int j0, int j1) {
+        strip_march<UNI>(v.o, load, value, i, j0, j1, NoRead{}, [&](int k, double2 q, double2 p, NoExtra) {
             v.q[k] = q;
             p_out[k] = p;
             pq[0] = fma(p.x, q.x, fma(p.y, q.y, pq[0]));
@@ -361,7 +363,8 @@ __global__ void __launch_bounds__(32 * STRIP_WARPS) k_cg_apply(CGView v, int row
 }
 void launch_cg_apply(const CGView& v, cudaStream_t s) {
     OperatorShape d = operator_shape(v.o.g.Nx, v.o.g.Ny, forced_operator_rows());
-    with_operator_rows(d.rows, [&](auto r, int rows) { k_cg_apply<decltype(r)::value><<<d.d.grid, d.d.block, 0, s>>>(v, rows); });
+    if (v.o.g.h != 0.0) k_cg_apply<true><<<d.d.grid, d.d.block, 0, s>>>(v, d.rows);
+    else k_cg_apply<false><<<d.d.grid, d.d.block, 0, s>>>(v, d.rows);
     count_launch();
 }
 

@@ -397,196 +397,10 @@ __device__ __forceinline__ void strip_apply(const OpView<T>& o, const typename V
     strip_apply_src<R, IU, IV>(o, [p](int k, int, int) { return p[k]; }, i, j0, extra, emit);
 }
 
-// ---- long walks -------------------------------------------------------------------------------------------------
-// The same walk over any number of rows, one row of operands ahead of the arithmetic, with the previous row in registers:
-// the two rows that a walk reads besides its own are shared by all of them, where the unrolled walks of R rows share them
-// by R.  For the FP64 kernels of large grids, which the FP64 pipe binds: k_cg_apply at 1024 x 512 takes 41 us, 30 FP64
-// instructions a cell, against 58 us and 34 with walks of 4 rows.
+// ---- rolling walks ------------------------------------------------------------------------------------------------
+// The same walk over any number of rows with the previous row in registers: the two rows that a walk reads besides its own
+// are shared by all of them, where the unrolled walks of R rows share them by R.
 //
-// One lane's column of the walk: push(row j + 1) returns the divergence of row j.
-template <typename T, bool UNI>
-struct StripColumn {
-    const DevGrid<T>& g;
-    T wall_factor, rdxc, dxc, rdxf, dxf;
-    bool wall_x;
-    T mu, mv, sy, t;           // the last row pushed, Δx Tyy of the centre below it and the shear of its corner
-    __device__ __forceinline__ StripColumn(const OpView<T>& o, int i, bool col_ok)
-        : g(o.g), wall_factor(o.wall_factor), rdxc(T(0)), dxc(T(0)), rdxf(T(0)), dxf(T(0)), mu(T(0)), mv(T(0)), sy(T(0)), t(T(0)) {
-        wall_x = g.out_x(i) || g.out_x(i - 1);
-        if (!UNI && col_ok) {
-            rdxc = g.rdxc[i]; dxc = g.dxc[i]; rdxf = g.rdxf[i]; dxf = g.dxf[i];
-        }
-    }
-    // (un, vn): masked velocities of row j + 1; eta: η̄H of centre (i, j); cff: η̄Hᶠᶠ of corner (i, j + 1); jm: the metric
-    // index of row j (j itself, wrapped where a walk runs over a periodic edge)
-    __device__ __forceinline__ void push(int j, int jm, T un, T vn, T eta, T cff, T& divu, T& divv) {
-        const unsigned full = 0xffffffffu;
-        const T ue = __shfl_down_sync(full, mu, 1), vw = __shfl_up_sync(full, vn, 1);
-        const bool wall = wall_x || g.out_y(j + 1) || g.out_y(j);
-        T sx, syn, tn;
-        if (UNI) {
-            const T du = ue - mu, dv = vn - mv;
-            sx = eta * (T(2) * du + dv);
-            syn = eta * (T(2) * dv + du);
-            tn = cff * ((un - mu) + (vn - vw));
-            if (__any_sync(full, wall)) tn = wall ? wall_factor * tn : tn;   // a warp off the walls issues no product
-        } else {
-            const bool in = jm >= -1 && jm <= g.Ny - 1;
-            const T rdyc = in ? g.rdyc[jm] : T(0), dyc = in ? g.dyc[jm] : T(0), rdyf = in ? g.rdyf[jm + 1] : T(0);
-            const T exx = (ue - mu) * rdxc, eyy = (vn - mv) * rdyc;
-            sx = dyc * (T(2) * eta * (T(2) * exx + eyy));
-            syn = dxc * (T(2) * eta * (T(2) * eyy + exx));
-            T e = (un - mu) * rdyf + (vn - vw) * rdxf;
-            if (wall) e = wall_factor * e;
-            tn = cff * e;
-        }
-        const T sxw = __shfl_up_sync(full, sx, 1), te = __shfl_down_sync(full, t, 1);
-        if (UNI) {
-            divu = T(2) * (sx - sxw) + (tn - t);
-            divv = T(2) * (syn - sy) + (te - t);
-        } else {
-            const T dyf = jm >= 0 && jm < g.Ny ? g.dyf[jm] : T(0);
-            divu = (sx - sxw) + (dxf * tn - dxf * t);
-            divv = (syn - sy) + (dyf * te - dyf * t);
-        }
-        mu = un; mv = vn; sy = syn; t = tn;
-    }
-};
-
-// q = A p over rows j0 .. j1 - 1 of one warp strip; `load(k)` issues the reads of the operand at k, `value(loaded)` forms
-// it, `extra` and `emit` as in strip_apply_general.
-template <bool UNI, uint8_t IU = U_IDENTITY, uint8_t IV = V_IDENTITY, typename T, typename Load, typename Value, typename Extra, typename Emit>
-__device__ __forceinline__ void strip_march(const OpView<T>& o, Load&& load, Value&& value, int i, int j0, int j1, Extra&& extra, Emit&& emit) {
-    using V2 = typename Vec2<T>::type;
-    using V4 = typename Vec4<T>::type;
-    using L = decltype(load(0));
-    using E = decltype(extra(0));
-    const DevGrid<T>& g = o.g;
-    const int lane = threadIdx.x & 31;
-    const bool col_ok = i <= g.Nx, own_col = lane >= 1 && lane <= STRIP_COLS && i < g.Nx;
-    const bool ucol = g.px || (i >= 0 && i <= g.Nx), vcol = !g.out_x(i);
-    const int cxi = col_ok ? g.cx(i) : 0, fxi = col_ok ? g.fx(i) : 0, iw = col_ok ? (g.px ? g.wrap(i, g.Nx) : (i < 0 ? 0 : i)) : 0;
-    const T h2 = UNI ? g.h * g.h : T(0);
-    StripColumn<T, UNI> col(o, i, col_ok);
-    struct Row { L l; V4 rec; T cff; uint8_t m; bool u, v; };
-    auto fetch = [&](int j) {   // row j of the lane's column; every index is within the stored plane
-        Row r;
-        r.m = 0;
-        r.cff = T(0);
-        r.rec.x = r.rec.y = r.rec.z = r.rec.w = T(0);
-        const bool row_ok = col_ok && j <= g.Ny;
-        r.u = row_ok && ucol && !g.out_y(j);
-        r.v = row_ok && vcol && (g.py || j >= 0);
-        if (row_ok) {
-            r.rec = o.coef[g.idx(cxi, g.cy(j))];
-            r.cff = o.coef[g.idx(fxi, g.fy(j))].y;
-        }
-        if (r.u || r.v) {
-            const int k = g.idx(iw, g.py ? g.wrap(j, g.Ny) : j);
-            r.m = __ldg(o.mask + k);
-            r.l = load(k);
-        }
-        return r;
-    };
-    auto pair = [&](const Row& r) {
-        V2 x;
-        x.x = x.y = T(0);
-        if (r.u || r.v) x = value(r.l);
-        return x;
-    };
-    Row cur = fetch(j0 - 1), nxt = fetch(j0);
-    V2 x = pair(cur);
-    col.mu = (cur.u && !(cur.m & U_INACTIVE)) ? x.x : T(0);
-    col.mv = (cur.v && !(cur.m & V_INACTIVE)) ? x.y : T(0);
-    E ex{};
-    for (int j = j0 - 1; j < j1; ++j) {   // the first turn, row j0 - 1, only fills sy and t
-        Row pre = fetch(j + 2);
-        E exn{};
-        if (own_col && j + 1 < j1) exn = extra(g.idx(i, j + 1));
-        const V2 xn = pair(nxt);
-        const T un = (nxt.u && !(nxt.m & U_INACTIVE)) ? xn.x : T(0), vn = (nxt.v && !(nxt.m & V_INACTIVE)) ? xn.y : T(0);
-        T divu, divv;
-        col.push(j, j, un, vn, cur.rec.x, nxt.cff, divu, divv);
-        if (own_col && j >= j0) {
-            V2 q;
-            const T au = UNI ? h2 : g.dxf[i] * g.dyc[j], av = UNI ? h2 : g.dxc[i] * g.dyf[j];
-            q.x = (cur.m & IU) ? x.x : au * cur.rec.z * x.x - divu;
-            q.y = (cur.m & IV) ? x.y : av * cur.rec.w * x.y - divv;
-            emit(g.idx(i, j), q, x, ex);
-        }
-        cur = nxt;
-        nxt = pre;
-        x = xn;
-        ex = exn;
-    }
-}
-
-// Launch shape of the FP64 operator kernels: rows per walk, warps per block, blocks.  rows > 0: unrolled walks
-// (strip_apply); rows < 0: long walks (strip_march) of -rows rows.
-struct OperatorShape {
-    int rows;
-    LaunchDims d;
-};
-inline OperatorShape operator_shape(int nx, int ny, int forced) {
-    OperatorShape s;
-    const long long across = (nx + STRIP_COLS - 1) / STRIP_COLS;
-    int rows = forced, warps;
-    long long tasks;
-    if (!forced && across * ny > 20ll * SM_COUNT) {
-        // Long walks, the number of rows that finishes the busiest SM first: a walk costs its rows and one and a half
-        // more, an SM takes the walks in turn, and four to twelve warps keep its FP64 pipe busy.
-        double best = 0;
-        for (int r = 4; r <= 64; ++r) {
-            const long long n = across * ((ny + r - 1) / r), per = (n + SM_COUNT - 1) / SM_COUNT;
-            if (r > 4 && per < 4) break;
-            const double cost = (double)per * (r + 1.5) * (per > 12 ? 1.05 : 1.0);
-            if (r == 4 || cost < best) { best = cost; rows = -r; }
-        }
-        tasks = across * ((ny - rows - 1) / -rows);
-        warps = 2;
-    } else {
-        // Unrolled walks: one row while that leaves a warp an SM quarter to itself, so that the serial chain of FP64
-        // instructions (64 cycles each) is the shortest (256 x 128: 10.3 us, 10.9 with two rows and 13.9 with four), else two.
-        if (!forced) rows = across * ny <= 8ll * SM_COUNT ? 1 : 2;
-        tasks = across * ((ny + rows - 1) / rows);
-        warps = tasks <= 2ll * SM_COUNT ? 1 : (tasks <= 4ll * SM_COUNT ? 2 : STRIP_WARPS);
-    }
-    const long long resident = 8ll * SM_COUNT;
-    long long blocks = (tasks + warps - 1) / warps;
-    s.rows = rows;
-    s.d.block = dim3(32, warps);
-    s.d.grid = dim3((unsigned)(blocks < resident ? blocks : resident), 1, batch_slots());
-    return s;
-}
-// Calls walk(i, j0) for every strip of R rows of the calling warp in a launch of operator_shape
-template <typename F>
-__device__ __forceinline__ void for_each_strip(int Nx, int Ny, int R, F&& walk) {
-    const int across = (Nx + STRIP_COLS - 1) / STRIP_COLS, n = across * ((Ny + R - 1) / R);
-    for (int t = (int)(threadIdx.y * gridDim.x + blockIdx.x); t < n; t += (int)(gridDim.x * blockDim.y)) {
-        const int row = t / across;
-        walk((t - row * across) * STRIP_COLS - 1 + (int)threadIdx.x, row * R);
-    }
-}
-// q = A p over rows j0 .. min(j0 + R, Ny) - 1 by the walk that operator_shape chose: R > 0 unrolled, R = 0 a long walk of `rows`.
-template <int R, uint8_t IU = U_IDENTITY, uint8_t IV = V_IDENTITY, typename T, typename Load, typename Value, typename Extra, typename Emit>
-__device__ __forceinline__ void strip_walk(const OpView<T>& o, int rows, Load&& load, Value&& value, int i, int j0, Extra&& extra, Emit&& emit) {
-    if constexpr (R > 0) {
-        strip_apply_src<R, IU, IV>(o, [&](int k, int, int) { return value(load(k)); }, i, j0, extra, emit);
-    } else {
-        const int j1 = j0 + rows < o.g.Ny ? j0 + rows : o.g.Ny;
-        if (o.g.h != decltype(o.g.h)(0)) strip_march<true, IU, IV>(o, load, value, i, j0, j1, extra, emit);
-        else strip_march<false, IU, IV>(o, load, value, i, j0, j1, extra, emit);
-    }
-}
-// Calls f(std::integral_constant<int, R>, rows): R = 0 for long walks of `rows` rows
-template <typename F>
-inline void with_operator_rows(int rows, F&& f) {
-    if (rows < 0) f(std::integral_constant<int, 0>{}, -rows);
-    else if (rows == 1) f(std::integral_constant<int, 1>{}, 1);
-    else if (rows == 2) f(std::integral_constant<int, 2>{}, 2);
-    else f(std::integral_constant<int, 4>{}, 4);
-}
-
 // One stage of a walk: push(row j + 1) gives the divergence of row j (cff: η̄Hᶠᶠ of corner (i, j + 1) times the wall
 // factor).
 template <typename T, bool UNI>
@@ -624,6 +438,114 @@ struct Stage {
         mu = un; mv = vn; sy = syn; t = tn;
     }
 };
+
+// q = A p over rows j0 .. j1 - 1 of one warp strip, for the FP64 operator kernels.  `load(k)` issues the reads of the operand
+// at k, `value(loaded)` forms it, `extra` and `emit` as in strip_apply_general.  k_cg_apply, against unrolled walks of 1 row
+// (128 x 64), 2 (512 x 256) and long walks with range tests (1280 x 160, 1024 x 512): 9.3 -> 8.1, 23.1 -> 17.8,
+// 22.8 -> 20.2 and 41.0 -> 40.5 us; unrolled walks of 4 rows took 58 us at 1024 x 512.  Rows and columns beyond a Bounded edge are
+// read at the nearest stored point (0 .. N, whose last row and column are walls) and flagged inactive below 0, where the
+// stored mask does not say so, so that no read carries a range test; no row that is written depends on the coefficients
+// there.  The reads run three rows ahead of the arithmetic in four slots.
+template <bool UNI, uint8_t IU = U_IDENTITY, uint8_t IV = V_IDENTITY, typename T, typename Load, typename Value, typename Extra, typename Emit>
+__device__ __forceinline__ void strip_march(const OpView<T>& o, Load&& load, Value&& value, int i, int j0, int j1, Extra&& extra, Emit&& emit) {
+    using V2 = typename Vec2<T>::type;
+    using V4 = typename Vec4<T>::type;
+    using L = decltype(load(0));
+    using E = decltype(extra(0));
+    const DevGrid<T>& g = o.g;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool own = lane >= 1 && lane <= STRIP_COLS && i < g.Nx;
+    const int iw = g.px ? (i < 0 ? i + g.Nx : (i >= g.Nx ? (i - g.Nx) % g.Nx : i)) : (i < 0 ? 0 : (i > g.Nx ? g.Nx : i));
+    const unsigned low = !g.px && i < 0 ? U_INACTIVE | V_INACTIVE : 0u;
+    const bool wall_x = !g.px && (i <= 0 || i >= g.Nx), any_wall = __any_sync(full, wall_x);
+    const T h2 = g.h * g.h;
+    auto row = [&](int j) {
+        if (g.py) return j < 0 ? j + g.Ny : (j >= g.Ny ? (j - g.Ny) % g.Ny : j);
+        return j < 0 ? 0 : (j > g.Ny ? g.Ny : j);
+    };
+    struct Row { L l; E ex; V4 c; V2 x; unsigned m; };
+    auto fetch = [&](Row& r, int j) {
+        const int k = row(j) * g.pitch + iw;
+        r.c = o.coef[k];
+        r.l = load(k);
+        r.ex = extra(k);
+        r.m = __ldg(o.mask + k);
+    };
+    auto settle = [&](Row& r, int j) {
+        r.x = value(r.l);
+        const bool wall_y = !g.py && (j <= 0 || j >= g.Ny);
+        if (any_wall || wall_y) {   // uniform: a warp off the walls issues no product
+            if (wall_x || wall_y) r.c.y = o.wall_factor * r.c.y;
+        }
+        r.m |= low | (!g.py && j < 0 ? U_INACTIVE | V_INACTIVE : 0u);
+    };
+    Stage<T, UNI> s(g, iw);
+    Row ring[4];
+    fetch(ring[0], j0 - 1);
+    fetch(ring[1], j0);
+    fetch(ring[2], j0 + 1);
+    settle(ring[0], j0 - 1);
+    s.mu = (ring[0].m & U_INACTIVE) ? T(0) : ring[0].x.x;
+    s.mv = (ring[0].m & V_INACTIVE) ? T(0) : ring[0].x.y;
+    auto step = [&](int j, Row& cur, Row& nxt, Row& far) {
+        if (j + 3 <= j1) fetch(far, j + 3);
+        settle(nxt, j + 1);
+        T du, dv;
+        s.push(UNI ? 0 : row(j), (nxt.m & U_INACTIVE) ? T(0) : nxt.x.x, (nxt.m & V_INACTIVE) ? T(0) : nxt.x.y, cur.c.x, nxt.c.y, du, dv);
+        if (own && j >= j0) {
+            const T au = UNI ? h2 : g.dxf[i] * g.dyc[j], av = UNI ? h2 : g.dxc[i] * g.dyf[j];
+            V2 q;
+            q.x = (cur.m & IU) ? cur.x.x : au * cur.c.z * cur.x.x - du;
+            q.y = (cur.m & IV) ? cur.x.y : av * cur.c.w * cur.x.y - dv;
+            emit(g.idx(i, j), q, cur.x, cur.ex);
+        }
+    };
+    for (int j = j0 - 1; j < j1; j += 4) {   // the first turn, row j0 - 1, only fills the stage
+        step(j, ring[0], ring[1], ring[3]);
+        if (j + 1 >= j1) break;
+        step(j + 1, ring[1], ring[2], ring[0]);
+        if (j + 2 >= j1) break;
+        step(j + 2, ring[2], ring[3], ring[1]);
+        if (j + 3 >= j1) break;
+        step(j + 3, ring[3], ring[0], ring[2]);
+    }
+}
+
+// Launch shape of the FP64 operator kernels: rows per walk, warps per block, blocks.
+struct OperatorShape {
+    int rows;
+    LaunchDims d;
+};
+inline OperatorShape operator_shape(int nx, int ny, int forced) {
+    OperatorShape s;
+    const long long across = (nx + STRIP_COLS - 1) / STRIP_COLS;
+    // The rows that finish the busiest SM first.  Its FP64 pipe takes 24 instructions of 19 cycles for each row of each of
+    // its walks, and a walk alone takes about 2500 cycles a row (dependent instructions of 64 cycles, shuffles); a walk
+    // costs one more row than it writes.
+    double best = 0;
+    s.rows = forced;
+    for (int r = 1; !forced && r <= 64 && r <= ny; ++r) {
+        const long long n = across * ((ny + r - 1) / r), per = (n + SM_COUNT - 1) / SM_COUNT;
+        const double pipe = (double)per * (r + 1.2) * 460, chain = (r + 1) * 2500.0, cost = pipe > chain ? pipe : chain;
+        if (r == 1 || cost < best) { best = cost; s.rows = r; }
+    }
+    const long long tasks = across * ((ny + s.rows - 1) / s.rows);
+    const int warps = tasks <= 2ll * SM_COUNT ? 1 : 2;
+    const long long resident = 8ll * SM_COUNT, blocks = (tasks + warps - 1) / warps;
+    s.d.block = dim3(32, warps);
+    s.d.grid = dim3((unsigned)(blocks < resident ? blocks : resident), 1, batch_slots());
+    return s;
+}
+// Calls walk(i, j0, j1) for every strip of `rows` rows of the calling warp in a launch of operator_shape
+template <typename F>
+__device__ __forceinline__ void for_each_strip(int Nx, int Ny, int rows, F&& walk) {
+    const int across = (Nx + STRIP_COLS - 1) / STRIP_COLS, n = across * ((Ny + rows - 1) / rows);
+    for (int t = (int)(threadIdx.y * gridDim.x + blockIdx.x); t < n; t += (int)(gridDim.x * blockDim.y)) {
+        const int row = t / across, j0 = row * rows;
+        walk((t - row * across) * STRIP_COLS - 1 + (int)threadIdx.x, j0, j0 + rows < Ny ? j0 + rows : Ny);
+    }
+}
 
 // Column and first row of the calling thread in a strip launch of R rows per warp (strip_dims).
 template <int R>
