@@ -622,10 +622,22 @@ void launch_thickness_stage(const ThicknessView& v, double dtau, int final_stage
 }
 
 // ---- the energy step ----------------------------------------------------------------------------------------
+// b < a ? b : a and a < b ? b : a; against zero the sign decides, on the integer units (a comparison takes the FP64 pipe)
 __device__ __forceinline__ double dmin(double a, double b) { return b < a ? b : a; }
 __device__ __forceinline__ double dmax(double a, double b) { return a < b ? b : a; }
+__device__ __forceinline__ bool negative(double x) {   // x <= -0.0, infinities included, NaN excluded
+    const unsigned h = (unsigned)__double2hiint(x);
+    return h >= 0x80000000u && (h < 0xfff00000u || (h == 0xfff00000u && __double2loint(x) == 0));
+}
+__device__ __forceinline__ double at_least_zero(double x) { return negative(x) ? 0.0 : x; }
+// clamp(x, 0, 1)
+__device__ __forceinline__ double clamp01(double x) {
+    const unsigned h = (unsigned)__double2hiint(x);
+    if (negative(x)) return 0.0;
+    return h >= 0x3ff00000u && h <= 0x7ff00000u && !(h == 0x7ff00000u && __double2loint(x) != 0) ? 1.0 : x;
+}
 // unit_ramp(x, w) = clamp(x / w, 0, 1), src/Thermodynamics/enthalpy_conversions.jl:69
-__device__ __forceinline__ double unit_ramp(double x, double w) { return dmin(dmax(x / w, 0.0), 1.0); }
+__device__ __forceinline__ double unit_ramp(double x, double w) { return clamp01(x / w); }
 
 // step_thermodynamics! (src/Thermodynamics/column_energy_solve.jl:26-78) for one column (i, j), one thread:
 // 1. the strain heating Φₖ = 4 ηₖ ε̇ₑ² (+ τᵇ² w₂ₖ / Δζₖ / ηₖ for the DIVA), strain_heating.jl:43-56;
@@ -640,9 +652,24 @@ __device__ __forceinline__ double unit_ramp(double x, double w) { return dmin(dm
 // 6. T = min(T_pm, T_r + E / c) and ω = max(0, E - E_pm) / L on every layer.
 // Columns thinner than the minimum thickness hold the surface enthalpy.  E_old is a copy of E: the neighbours'
 // old enthalpy is read while this column writes its new one.
+// Bound by the FP64 pipe.  Steps 2 and 4 go up the column together, so that a layer's four volume fluxes serve its mass and
+// its enthalpy and no flux is stored; the layers' geometric quotients come from shared memory, once a block; signs are
+// tested on the integer units.  700 x 350, 10 layers: 881 -> 623 us.
 __global__ void __launch_bounds__(128) k_step_enthalpy(EnergyView v, double dt) {
     const DevGrid<double>& g = v.g;
     int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
+    // face kf = k + 1 above layer k: θ = (zf - zm) / (zp - zm), zf - zm, zp - zf; and w₂ₖ / Δζₖ
+    __shared__ double s_theta[ENERGY_MAX_LAYERS + 1], s_lo[ENERGY_MAX_LAYERS + 1], s_hi[ENERGY_MAX_LAYERS + 1], s_w2[ENERGY_MAX_LAYERS + 1];
+    for (int k = threadIdx.y * 32 + threadIdx.x + 1; k <= v.sig.N; k += 128) {
+        s_w2[k] = v.sig.w2[k - 1] / v.sig.dz[k - 1];
+        if (k < v.sig.N) {
+            const double zf = v.sig.zf[k], zm = v.sig.zc[k - 1], zp = v.sig.zc[k];
+            s_theta[k] = (zf - zm) / (zp - zm);
+            s_lo[k] = zf - zm;
+            s_hi[k] = zp - zf;
+        }
+    }
+    __syncthreads();
     if (i >= g.Nx || j >= g.Ny) return;
     const EnergyConstants& q = v.q;
     const SigmaTable& sg = v.sig;
@@ -654,11 +681,11 @@ __global__ void __launch_bounds__(128) k_step_enthalpy(EnergyView v, double dt) 
     // through the column are inverted once and each layer's diffusivity is evaluated once (the results differ from
     // the quotients of the formulas in the last bits only).
     const double r_L = 1 / q.L, r_c = 1 / q.c, r_blend = 1 / q.blend, r_dt = 1 / dt, k_c = q.k / q.c;
-    auto ramp = [](double x, double rw) { return dmin(dmax(x * rw, 0.0), 1.0); };   // unit_ramp with 1/w
+    auto ramp = [](double x, double rw) { return clamp01(x * rw); };   // unit_ramp with 1/w
     auto Tpm = [&](double p) { return q.T0 - q.beta * p; };
     auto Epm = [&](double p) { return q.c * (Tpm(p) - q.Tr); };
     auto enthalpy = [&](double T, double p) { return q.c * (dmin(T, Tpm(p)) - q.Tr) + 0.0 * q.L; };
-    auto water_fraction = [&](double E, double p) { return dmax(0.0, E - Epm(p)) * r_L; };
+    auto water_fraction = [&](double E, double p) { return at_least_zero(E - Epm(p)) * r_L; };
     auto thickness = [&](double h) { return dmax(h, q.min_thickness); };
     auto layer_pressure = [&](int k) { return rho * ga * H * (1 - sg.zc[k - 1]); };
     auto Eold = [&](int k, int ii, int jj) { return v.E_old[(k - 1) * P + g.c_idx(ii, jj)]; };
@@ -680,40 +707,29 @@ __global__ void __launch_bounds__(128) k_step_enthalpy(EnergyView v, double dt) 
     for (int k = 1; k <= Ns; ++k) {
         double eta = v.eta_sigma[(k - 1) * P + c];
         double ph = 4 * eta * e2;
-        if (v.diva) ph += tb2 * sg.w2[k - 1] / (sg.dz[k - 1] * (eta == 0.0 ? INFINITY : eta));
+        if (v.diva) ph += tb2 * s_w2[k] / (eta == 0.0 ? INFINITY : eta);
         v.Phi[(k - 1) * P + c] = ph;
     }
 
-    // 2. layer volume fluxes
-    auto layer_u = [&](int f, int k) { return g.peripheral_fc(f, j) ? 0.0 : v.usig[(k - 1) * P + g.u_idx(f, j)].x; };
-    auto layer_v = [&](int f, int k) { return g.peripheral_cf(i, f) ? 0.0 : v.usig[(k - 1) * P + g.v_idx(i, f)].y; };
-    auto xvol = [&](int f, int k) {
-        double u = layer_u(f, k);
-        return g.dyc[j] * u * (u > 0 ? v.Hn[g.c_idx(f - 1, j)] : v.Hn[g.c_idx(f, j)]);
+    // 2. layer fluxes: the volumes that leave layer k through its four faces (upwind Hⁿ) and the enthalpy they carry
+    const double Hw_ = v.Hn[g.c_idx(i - 1, j)], He_ = v.Hn[g.c_idx(i + 1, j)], Hs_ = v.Hn[g.c_idx(i, j - 1)], Hn_ = v.Hn[g.c_idx(i, j + 1)];
+    const int iw = g.c_idx(i - 1, j), ie = g.c_idx(i + 1, j), is = g.c_idx(i, j - 1), in = g.c_idx(i, j + 1);
+    const int fw = g.u_idx(i, j), fe = g.u_idx(i + 1, j), fs = g.v_idx(i, j), fn = g.v_idx(i, j + 1);
+    const bool ww = g.peripheral_fc(i, j), we = g.peripheral_fc(i + 1, j), ws = g.peripheral_cf(i, j), wn = g.peripheral_cf(i, j + 1);
+    const double rx = g.rdxc[i], ry = g.rdyc[j];
+    auto layer_fluxes = [&](int k, double Ek, double& vol, double& enth) {   // divergence of both, per area
+        const long long o = (k - 1) * P;
+        const double uw = ww ? 0.0 : v.usig[o + fw].x, ue = we ? 0.0 : v.usig[o + fe].x;
+        const double us = ws ? 0.0 : v.usig[o + fs].y, un = wn ? 0.0 : v.usig[o + fn].y;
+        const bool pw = positive(uw), pe = positive(ue), ps = positive(us), pn = positive(un);
+        const double qw = uw * (pw ? Hw_ : Hn), qe = ue * (pe ? Hn : He_), qs = us * (ps ? Hs_ : Hn), qn = un * (pn ? Hn : Hn_);
+        vol = fma(qe - qw, rx, (qn - qs) * ry);
+        const double xe = qe * (pe ? Ek : v.E_old[o + ie]), xw = qw * (pw ? v.E_old[o + iw] : Ek);
+        const double yn = qn * (pn ? Ek : v.E_old[o + in]), ys = qs * (ps ? v.E_old[o + is] : Ek);
+        enth = fma(xe - xw, rx, (yn - ys) * ry);
     };
-    auto yvol = [&](int f, int k) {
-        double w = layer_v(f, k);
-        return g.dxc[i] * w * (w > 0 ? v.Hn[g.c_idx(i, f - 1)] : v.Hn[g.c_idx(i, f)]);
-    };
-    auto xenth = [&](int f, int k) {
-        double u = v.usig[(k - 1) * P + g.u_idx(f, j)].x;
-        return xvol(f, k) * (u > 0 ? Eold(k, f - 1, j) : Eold(k, f, j));
-    };
-    auto yenth = [&](int f, int k) {
-        double w = v.usig[(k - 1) * P + g.v_idx(i, f)].y;
-        return yvol(f, k) * (w > 0 ? Eold(k, i, f - 1) : Eold(k, i, f));
-    };
-    const double Az = g.Az_cc(i, j), r_Az = 1 / Az;
-    double W[ENERGY_MAX_LAYERS + 1];
-    {
-        double dHdt = (thickness(H) - thickness(Hn)) * r_dt;
-        double m = v.grounding ? (1 - v.phi[c]) * v.melt[c] : v.melt[c];
-        W[0] = -m - (q.coupled ? v.gmelt[c] : 0.0);
-        for (int k = 1; k <= Ns; ++k) {
-            double div = (xvol(i + 1, k) - xvol(i, k) + yvol(j + 1, k) - yvol(j, k)) * r_Az;
-            W[k] = W[k - 1] - sg.dz[k - 1] * (dHdt + div);
-        }
-    }
+    const double dHdt = (thickness(H) - thickness(Hn)) * r_dt;
+    const double W0 = -(v.grounding ? (1 - v.phi[c]) * v.melt[c] : v.melt[c]) - (q.coupled ? v.gmelt[c] : 0.0);
 
     // 3. basal state
     const double Ht = thickness(H), Hnt = thickness(Hn);
@@ -741,42 +757,45 @@ __global__ void __launch_bounds__(128) k_step_enthalpy(EnergyView v, double dt) 
     const double Es = enthalpy(v.Ts[c], 0.0);
     const double chi = phi_g * r * (1 - sb);
     const double Eo = enthalpy(v.To[c], pb);
-    const double Fb = rho * W[0];
-    const double Lam = D * (chi + 1 - phi_g) + dmax(-Fb, 0.0);
-    const double S = (1 - r) * qg + D * (chi * Epm_b + (1 - phi_g) * Eo) + dmax(Fb, 0.0) * Epm_b;
-    const double Fs = rho * W[Ns];
-    const double kapN = Ns == 1 ? kap1 : diffusivity(Ns);
-    const double Ks = kapN / (Ht * (1 - sg.zc[Ns - 1]));
-    const double Ds = Ks + dmax(Fs, 0.0), Ss = (Ks + dmax(-Fs, 0.0)) * Es;
-    // interior face kf = 2..Nσ between layers of diffusivities km (below) and kp (above)
-    auto couplings = [&](int kf, double km, double kp, double& lower, double& upper) {
-        double zf = sg.zf[kf - 1], zm = sg.zc[kf - 2], zp = sg.zc[kf - 1];
-        double theta = (zf - zm) / (zp - zm);
-        double Fk = rho * W[kf - 1];
-        double cond = km * kp / (Ht * ((zf - zm) * kp + (zp - zf) * km));   // 1 / (Ht ((zf - zm) / km + (zp - zf) / kp))
-        double Dk = dmax(cond, dmax(dmax(Fk, 0.0) * theta, dmax(-Fk, 0.0) * (1 - theta)));
+    const double Fb = rho * W0;
+    const double Lam = D * (chi + 1 - phi_g) + at_least_zero(-Fb);
+    const double S = (1 - r) * qg + D * (chi * Epm_b + (1 - phi_g) * Eo) + at_least_zero(Fb) * Epm_b;
+    const double r_Ht = 1 / Ht;
+    // the face above layer k, between layers of diffusivities km (below) and kp (above), volume flux Wk through it
+    auto couplings = [&](int k, double Wk, double km, double kp, double& lower, double& upper) {
+        const double theta = s_theta[k], Fk = rho * Wk;
+        const double cond = km * kp * r_Ht / (s_lo[k] * kp + s_hi[k] * km);   // 1 / (Ht ((zf - zm) / km + (zp - zf) / kp))
+        const double Dk = dmax(cond, negative(Fk) ? -Fk * (1 - theta) : Fk * theta);
         lower = -Fk * (1 - theta) - Dk;
         upper = Fk * theta - Dk;
     };
     double t[ENERGY_MAX_LAYERS + 1], e[ENERGY_MAX_LAYERS + 1];
-    double lower_m = 0, upper_m = 0, prev_a = 0, prev_c = 0, rpiv = 1;
-    double kap_k = kap1;
+    double upper_m = 0, prev_a = 0, prev_c = 0, rpiv = 1;
+    double kap_k = kap1, Wk = W0, Ek = Eold(1, i, j);
     for (int k = 1; k <= Ns; ++k) {
-        double dz = sg.dz[k - 1];
-        double lower_p = 0, upper_p = 0;
+        const double dz = sg.dz[k - 1];
+        double vol, enth;
+        layer_fluxes(k, Ek, vol, enth);
+        Wk -= dz * (dHdt + vol);
+        double lower_p = 0, upper_p = 0, Enext = 0, diag_p, forcing = k == 1 ? S : 0.0;
         if (k < Ns) {
-            double kap_n = k + 1 == Ns ? kapN : diffusivity(k + 1);
-            couplings(k + 1, kap_k, kap_n, lower_p, upper_p);
+            Enext = Eold(k + 1, i, j);
+            const double w = ramp(Enext - Epm(layer_pressure(k + 1)) + q.blend, r_blend), kap_n = k_c * (1 - w + w * q.temperate_ratio);
+            couplings(k, Wk, kap_k, kap_n, lower_p, upper_p);
             kap_k = kap_n;
+            diag_p = -lower_p;
+        } else {   // the surface
+            const double Fs = rho * Wk, Ks = kap_k / (Ht * (1 - sg.zc[Ns - 1]));
+            diag_p = Ks + at_least_zero(Fs);
+            forcing += (Ks + at_least_zero(-Fs)) * Es;
         }
-        double diag_m = k == 1 ? Lam : -upper_m;
-        double diag_p = k == Ns ? Ds : -lower_p;
-        double forcing = (k == 1 ? S : 0.0) + (k == Ns ? Ss : 0.0);
-        double transport = rho * dz * ((xenth(i + 1, k) - xenth(i, k) + yenth(j + 1, k) - yenth(j, k)) * r_Az);
+        const double diag_m = k == 1 ? Lam : -upper_m;
+        const double transport = rho * dz * enth;
         double ak = mu ? lower_p : 0.0;
         double ck = mu ? upper_p : 0.0;
-        double bk = mu ? rho * Ht * dz * r_dt + diag_m + diag_p : 1.0;
-        double fk = mu ? rho * Hnt * dz * Eold(k, i, j) * r_dt - transport + Ht * dz * v.Phi[(k - 1) * P + c] + forcing : Es;
+        const double store = rho * dz * r_dt;
+        double bk = mu ? store * Ht + diag_m + diag_p : 1.0;
+        double fk = mu ? store * Hnt * Ek - transport + Ht * dz * v.Phi[(k - 1) * P + c] + forcing : Es;
         if (k == 1) {
             rpiv = 1 / bk;
             e[1] = fk * rpiv;
@@ -786,7 +805,8 @@ __global__ void __launch_bounds__(128) k_step_enthalpy(EnergyView v, double dt) 
             e[k] = (fk - prev_a * e[k - 1]) * rpiv;
         }
         prev_a = ak; prev_c = ck;
-        lower_m = lower_p; upper_m = upper_p;
+        upper_m = upper_p;
+        Ek = Enext;
     }
     for (int k = Ns - 1; k >= 1; --k) e[k] -= t[k + 1] * e[k + 1];
 
@@ -799,9 +819,9 @@ __global__ void __launch_bounds__(128) k_step_enthalpy(EnergyView v, double dt) 
         for (int k = 1; k <= Ns; ++k) {
             double w = water_fraction(e[k], layer_pressure(k));
             double x = w * r_drain;
-            double rate = q.max_drainage_rate * (dmin(dmax(x - 1, 0.0), 1.0) + 9 * dmin(dmax(x - 2, 0.0), 1.0)) * 0.1;
-            double dw = dmin(dt * rate, dmax(w - q.drainage_fraction, 0.0));
-            dw = mu ? dw : 0.0;
+            if (negative(x - 1) || !mu) continue;   // no layer drains below the fraction that starts it
+            double rate = q.max_drainage_rate * (clamp01(x - 1) + 9 * clamp01(x - 2)) * 0.1;
+            double dw = dmin(dt * rate, at_least_zero(w - q.drainage_fraction));
             e[k] -= q.L * dw;
             drained += Ht * sg.dz[k - 1] * dw;
         }
