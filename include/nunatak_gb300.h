@@ -580,7 +580,7 @@ typedef struct nk_time_gradient_stats {
 } nk_time_gradient_stats;
 
 /* Device memory: the checkpoints and one segment's stage states, (⌈steps / K⌉ + 3K + 2) states of 3 planes (DIVA:
- * 6 + Nσ; a front: 2 more, 3 with von Mises calving) plus about 25 planes of adjoints, allocated for the call and freed
+ * 6 + Nσ; a front: 2 more, 3 with von Mises calving) plus about 50 planes of adjoints, allocated for the call and freed
  * before it returns.
  * After an error the problem's fields are those of whichever step the sweep had reached. */
 nk_status nk_checkpointed_gradient(nk_problem* problem, const nk_time_gradient_desc* desc, nk_cost_fn cost, void* user,

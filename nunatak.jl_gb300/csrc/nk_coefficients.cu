@@ -291,13 +291,6 @@ void launch_velocity_profile(const PhysView& ph, int diva, const double2* x, con
 
 // ---- geometry ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ double nonzero(double x) { return x == 0.0 ? 1.0 : x; }
-// The sign of a flotation by its high word, on the integer units: a finite x >= +0, and a finite x < 0 of normal size.
-// Neither holds for -0, subnormal negatives, infinities and NaN, which take the general expressions.
-__device__ __forceinline__ bool surely_grounded(double x) { return (unsigned)__double2hiint(x) < 0x7ff00000u; }
-__device__ __forceinline__ bool surely_floating(double x) {
-    unsigned h = (unsigned)__double2hiint(x);
-    return h >= 0x80100000u && h < 0xfff00000u;
-}
 // x > 0 of a finite x, and a + b == 0, on the integer units (the sum itself where one is negative)
 __device__ __forceinline__ bool positive(double x) { return surely_grounded(x) && __double_as_longlong(x) != 0; }
 __device__ __forceinline__ bool sum_is_zero(double a, double b) {

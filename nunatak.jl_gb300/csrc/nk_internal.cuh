@@ -176,6 +176,14 @@ __device__ __forceinline__ float narrow_pow2(double x, int k) {
     return (float)scale_pow2(x, k);
 }
 
+// The sign of a flotation by its high word, on the integer units: a finite x >= +0, and a finite x < 0 of normal size.
+// Neither holds for -0, subnormal negatives, infinities and NaN, which take the general expressions.
+__device__ __forceinline__ bool surely_grounded(double x) { return (unsigned)__double2hiint(x) < 0x7ff00000u; }
+__device__ __forceinline__ bool surely_floating(double x) {
+    unsigned h = (unsigned)__double2hiint(x);
+    return h >= 0x80100000u && h < 0xfff00000u;
+}
+
 // ---- warp / block reductions (fixed order, so results do not depend on scheduling) --------------------
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {

@@ -245,14 +245,6 @@ __device__ __forceinline__ double2 recon_adjoint_y(const StageAdjointView& a, in
     return r;
 }
 
-// The distinct faces (x faces when `n` is Nx) whose five-cell stencils can hold cell `i`: i-3 .. i+3, within 0..n on
-// a Bounded axis, wrapped on a Periodic one (every face when the axis is shorter than the seven).
-struct FaceRange { int lo, hi; bool all; };
-__device__ __forceinline__ FaceRange stencil_faces(int i, int n, int periodic) {
-    if (periodic) return n <= 7 ? FaceRange{0, n - 1, true} : FaceRange{i - 3, i + 3, false};
-    return FaceRange{i - 3 < 0 ? 0 : i - 3, i + 3 > n ? n : i + 3, false};
-}
-
 // ∂/∂(f1, f2, f3) of triangle_fraction (nk_coefficients.cu): one floating corner 1 - a² / ((b - a)(c - a)),
 // one grounded corner c² / ((c - a)(c - b)), a ≤ b ≤ c the sorted flotations; zero when all three agree in sign.
 __device__ __forceinline__ void triangle_fraction_partials(double f1, double f2, double f3, double* d) {
@@ -311,62 +303,97 @@ __device__ __forceinline__ void centre_fraction_partials(const double f[3][3], d
     }
 }
 
+// Every reconstruction's and every grounded fraction's reverse once: a cell's two reconstructions along an axis share its
+// five-cell stencil, so the cell writes what they send to the five cells (planes 0..4 along x, 5..9 along y), and what its
+// fraction sends to its 3 x 3 (planes 10..18); k_stage_adjoint_stencils gathers them.  Bound by the FP64 pipe.  250 x 125:
+// 825 us when every cell evaluated the up to twenty reconstructions and nine fractions that read it, 87 us (72 and 15) this way.
+__global__ void k_stage_adjoint_recon(StageAdjointView a) {
+    const ThicknessView& v = a.t;
+    const DevGrid<double>& g = v.g;
+    const int axis = blockIdx.z;
+    int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y;
+    if (i >= g.Nx || j >= g.Ny) return;
+    const double* __restrict__ Hs = v.Hs;
+    const int me = g.idx(i, j);
+    if (axis == 2) {   // what the cell's centre grounded fraction sends to the 3 x 3 flotations it reads
+        const double lp = v.grounding ? a.lam_phi[me] : 0.0;
+        if (lp == 0.0) return;   // not gathered
+        double f[3][3], d[3][3];
+        // nine flotations of one sign: every triangle is 0 or 1 and its partials zero
+        bool grounded = true, floating = true;
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+#pragma unroll
+            for (int y = 0; y < 3; ++y) {
+                const int k = g.c_idx(i + x - 1, j + y - 1);
+                f[x][y] = Hs[k] + a.rw_ri * a.bed[k];
+                d[x][y] = 0.0;
+                grounded = grounded && surely_grounded(f[x][y]);
+                floating = floating && surely_floating(f[x][y]);
+            }
+        if (!(grounded || floating)) centre_fraction_partials(f, d);
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+#pragma unroll
+            for (int y = 0; y < 3; ++y) a.recon[(size_t)(10 + 3 * x + y) * a.plane + me] = lp * d[x][y];
+        return;
+    }
+    // λ of the reconstruction towards the next cell (at face + 1) and towards the previous one (at the cell's own face)
+    const double plus = axis == 0 ? recon_adjoint_x(a, g.px && i + 1 == g.Nx ? 0 : i + 1, j).x
+                                  : recon_adjoint_y(a, i, g.py && j + 1 == g.Ny ? 0 : j + 1).x;
+    const double minus = axis == 0 ? recon_adjoint_x(a, i, j).y : recon_adjoint_y(a, i, j).y;
+    double s[5], r[5], J[5], out[5] = {0, 0, 0, 0, 0};
+    if (plus != 0.0 || minus != 0.0) {
+#pragma unroll
+        for (int m = -2; m <= 2; ++m)
+            s[m + 2] = axis == 0 ? Hs[j * g.pitch + wide_map(i + m, g.Nx, g.px)] : Hs[wide_map(j + m, g.Ny, g.py) * g.pitch + i];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) r[m] = s[4 - m];
+        if (plus != 0.0) {
+            face_value_gradient(v, s, J);
+#pragma unroll
+            for (int m = 0; m < 5; ++m) out[m] += J[m] * plus;
+        }
+        if (minus != 0.0) {
+            face_value_gradient(v, r, J);
+#pragma unroll
+            for (int m = 0; m < 5; ++m) out[4 - m] += J[m] * minus;
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 5; ++m) a.recon[(size_t)(5 * axis + m) * a.plane + me] = out[m];
+}
+// What the stencils of one axis send to cell c of n: `at(k, m)` is what cell k's stencil sends to its neighbour m - 2.  On a
+// Bounded axis a stencil beyond the edge reads the edge cell; a periodic axis shorter than the stencil reads cells twice.
+template <typename At>
+__device__ __forceinline__ double gather_stencils(int c, int n, int periodic, At&& at) {
+    double acc = 0.0;
+    if (periodic && n < 5) {
+        for (int k = 0; k < n; ++k)
+            for (int m = 0; m < 5; ++m)
+                if (wide_map(k + m - 2, n, 1) == c) acc += at(k, m);
+        return acc;
+    }
+    for (int q = c - 2; q <= c + 2; ++q) {
+        if (!periodic && (q < 0 || q >= n)) continue;
+        const int k = periodic ? wide_map(q, n, 1) : q;
+        acc += at(k, c - q + 2);
+        if (periodic) continue;
+        if (c == 0)
+            for (int m = 0; m < 2 - q; ++m) acc += at(k, m);
+        if (c == n - 1)
+            for (int m = n - q + 2; m < 5; ++m) acc += at(k, m);
+    }
+    return acc;
+}
+
 __global__ void k_stage_adjoint_stencils(StageAdjointView a) {
     const ThicknessView& v = a.t;
     const DevGrid<double>& g = v.g;
     int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y;
     if (i >= g.Nx || j >= g.Ny) return;
-    const double* __restrict__ Hs = v.Hs;
-    double acc = 0.0, s[5], J[5];
-    int cols[5];
-    FaceRange fr = stencil_faces(i, g.Nx, g.px);
-    int row = g.cy(j) * g.pitch;
-    for (int q = fr.lo; q <= fr.hi; ++q) {
-        int f = (g.px && !fr.all) ? wide_map(q, g.Nx, 1) : q;
-        double2 r = recon_adjoint_x(a, f, j);
-#pragma unroll
-        for (int side = 0; side < 2; ++side) {
-            double lr = side == 0 ? r.x : r.y;
-            if (lr == 0.0) continue;
-            bool hit = false;
-#pragma unroll
-            for (int m = -2; m <= 2; ++m) {
-                cols[m + 2] = wide_map(side == 0 ? f - 1 + m : f - m, g.Nx, g.px);
-                hit |= cols[m + 2] == i;
-            }
-            if (!hit) continue;
-#pragma unroll
-            for (int m = 0; m < 5; ++m) s[m] = Hs[row + cols[m]];
-            face_value_gradient(v, s, J);
-#pragma unroll
-            for (int m = 0; m < 5; ++m)
-                if (cols[m] == i) acc += J[m] * lr;
-        }
-    }
-    fr = stencil_faces(j, g.Ny, g.py);
-    int col = g.cx(i);
-    for (int q = fr.lo; q <= fr.hi; ++q) {
-        int f = (g.py && !fr.all) ? wide_map(q, g.Ny, 1) : q;
-        double2 r = recon_adjoint_y(a, i, f);
-#pragma unroll
-        for (int side = 0; side < 2; ++side) {
-            double lr = side == 0 ? r.x : r.y;
-            if (lr == 0.0) continue;
-            bool hit = false;
-#pragma unroll
-            for (int m = -2; m <= 2; ++m) {
-                cols[m + 2] = wide_map(side == 0 ? f - 1 + m : f - m, g.Ny, g.py);
-                hit |= cols[m + 2] == j;
-            }
-            if (!hit) continue;
-#pragma unroll
-            for (int m = 0; m < 5; ++m) s[m] = Hs[cols[m] * g.pitch + col];
-            face_value_gradient(v, s, J);
-#pragma unroll
-            for (int m = 0; m < 5; ++m)
-                if (cols[m] == j) acc += J[m] * lr;
-        }
-    }
+    double acc = gather_stencils(i, g.Nx, g.px, [&](int k, int m) { return a.recon[(size_t)m * a.plane + g.idx(k, j)]; });
+    acc += gather_stencils(j, g.Ny, g.py, [&](int k, int m) { return a.recon[(size_t)(5 + m) * a.plane + g.idx(i, k)]; });
     // the centre grounded fractions whose 3 x 3 flotations read this cell (φ of the melt source)
     if (v.grounding) {
         const int me = g.idx(i, j);
@@ -384,27 +411,13 @@ __global__ void k_stage_adjoint_stencils(StageAdjointView a) {
             int cj = (g.py && !yall) ? g.wrap(qy, g.Ny) : qy;
             for (int qx = xlo; qx <= xhi; ++qx) {
                 int ci = (g.px && !xall) ? g.wrap(qx, g.Nx) : qx;
-                double lp = a.lam_phi[g.idx(ci, cj)];
-                if (lp == 0.0) continue;
-                double f[3][3], d[3][3];
-                int kk[3][3];
-                bool hit = false;
-#pragma unroll
-                for (int x = 0; x < 3; ++x)
-#pragma unroll
-                    for (int y = 0; y < 3; ++y) {
-                        int k = g.c_idx(ci + x - 1, cj + y - 1);
-                        kk[x][y] = k;
-                        f[x][y] = Hs[k] + a.rw_ri * a.bed[k];
-                        hit |= k == me;
-                    }
-                if (!hit) continue;
-                centre_fraction_partials(f, d);
+                const int q = g.idx(ci, cj);
+                if (a.lam_phi[q] == 0.0) continue;
 #pragma unroll
                 for (int x = 0; x < 3; ++x)
 #pragma unroll
                     for (int y = 0; y < 3; ++y)
-                        if (kk[x][y] == me) acc += lp * d[x][y];
+                        if (g.c_idx(ci + x - 1, cj + y - 1) == me) acc += a.recon[(size_t)(10 + 3 * x + y) * a.plane + q];
             }
         }
     }
@@ -417,6 +430,7 @@ void launch_stage_adjoint(const StageAdjointView& a, cudaStream_t s) {
     k_stage_adjoint_cells<<<dc.grid, dc.block, 0, s>>>(a); count_launch();
     k_stage_adjoint_faces<<<df.grid, df.block, 0, s>>>(a); count_launch();
     k_stage_adjoint_limiter<<<dc.grid, dc.block, 0, s>>>(a); count_launch();
+    k_stage_adjoint_recon<<<dim3(dc.grid.x, dc.grid.y, a.t.grounding ? 3 : 2), dc.block, 0, s>>>(a); count_launch();
     k_stage_adjoint_stencils<<<dc.grid, dc.block, 0, s>>>(a); count_launch();
 }
 

@@ -62,45 +62,32 @@ __device__ __forceinline__ double face_value(const ThicknessView& v, const doubl
 
 // ∂(face value)/∂s[m], m = 0..4, of the reconstructions above, for the reverse of the stage.  WENO-5 by the chain rule
 // through its candidates qₖ, smoothness indicators βₖ and weights: with αₖ = dₖ (1 + τ / (βₖ + ε)), S = Σ αₖ and
-// q = Σ αₖ qₖ / S, ∂q = Σ (αₖ ∂qₖ + (qₖ - q) ∂αₖ) / S, ∂αₖ = dₖ (∂τ / (βₖ + ε) - τ ∂βₖ / (βₖ + ε)²) and
-// ∂τ = sign(β₀ - β₂) (∂β₀ - ∂β₂).
+// q = Σ αₖ qₖ / S, ∂q = Σ αₖ/S ∂qₖ + Σ bₖ ∂βₖ, where gₖ = dₖ (qₖ - q) / S gives b through ∂αₖ = dₖ (∂τ / (βₖ + ε) -
+// τ ∂βₖ / (βₖ + ε)²) and ∂τ = sign(β₀ - β₂) (∂β₀ - ∂β₂).  Four divisions; a quotient for every term and neighbour took
+// thirty-two.
 __device__ __forceinline__ void weno5_face_gradient(const double* s, double* J) {
     const double a = s[0], b = s[1], c = s[2], d = s[3], e = s[4];
     const double sixth = 1.0 / 6;
-    const double q[3] = {(2 * a - 7 * b + 11 * c) * sixth, (-b + 5 * c + 2 * d) * sixth, (2 * c + 5 * d - e) * sixth};
-    const double dq[3][5] = {{2 * sixth, -7 * sixth, 11 * sixth, 0, 0}, {0, -sixth, 5 * sixth, 2 * sixth, 0},
-                             {0, 0, 2 * sixth, 5 * sixth, -sixth}};
+    const double q0 = (2 * a - 7 * b + 11 * c) * sixth, q1 = (-b + 5 * c + 2 * d) * sixth, q2 = (2 * c + 5 * d - e) * sixth;
     const double A0 = a - 2 * b + c, B0 = a - 4 * b + 3 * c;
     const double A1 = b - 2 * c + d, B1 = b - d;
     const double A2 = c - 2 * d + e, B2 = 3 * c - 4 * d + e;
-    const double beta[3] = {13.0 / 12 * A0 * A0 + 0.25 * B0 * B0, 13.0 / 12 * A1 * A1 + 0.25 * B1 * B1,
-                            13.0 / 12 * A2 * A2 + 0.25 * B2 * B2};
+    const double b0 = 13.0 / 12 * A0 * A0 + 0.25 * B0 * B0, b1 = 13.0 / 12 * A1 * A1 + 0.25 * B1 * B1, b2 = 13.0 / 12 * A2 * A2 + 0.25 * B2 * B2;
+    const double eps = 1e-8, r0 = 1 / (b0 + eps), r1 = 1 / (b1 + eps), r2 = 1 / (b2 + eps);
+    const double tau = fabs(b0 - b2), sg = b0 >= b2 ? 1.0 : -1.0;
+    const double a0 = 0.1 * (1 + tau * r0), a1 = 0.6 * (1 + tau * r1), a2 = 0.3 * (1 + tau * r2);
+    const double rS = 1 / (a0 + a1 + a2), val = (a0 * q0 + a1 * q1 + a2 * q2) * rS;
+    const double g0 = 0.1 * (q0 - val) * rS * r0, g1 = 0.6 * (q1 - val) * rS * r1, g2 = 0.3 * (q2 - val) * rS * r2;
+    const double G = sg * (g0 + g1 + g2);
+    const double c0 = G - tau * g0 * r0, c1 = -tau * g1 * r1, c2 = -G - tau * g2 * r2;   // ∂q/∂βₖ
     const double k13 = 13.0 / 6;
-    const double db[3][5] = {{k13 * A0 + 0.5 * B0, -2 * k13 * A0 - 2 * B0, k13 * A0 + 1.5 * B0, 0, 0},
-                             {0, k13 * A1 + 0.5 * B1, -2 * k13 * A1, k13 * A1 - 0.5 * B1, 0},
-                             {0, 0, k13 * A2 + 1.5 * B2, -2 * k13 * A2 - 2 * B2, k13 * A2 + 0.5 * B2}};
-    const double eps = 1e-8, dk[3] = {0.1, 0.6, 0.3};
-    const double tau = fabs(beta[0] - beta[2]), sg = beta[0] >= beta[2] ? 1.0 : -1.0;
-    double al[3], S = 0, num = 0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        al[k] = dk[k] * (1 + tau / (beta[k] + eps));
-        S += al[k];
-        num += al[k] * q[k];
-    }
-    const double val = num / S, rS = 1 / S;
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-        const double dtau = sg * (db[0][m] - db[2][m]);
-        double acc = 0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const double ek = beta[k] + eps;
-            const double dal = dk[k] * (dtau / ek - tau * db[k][m] / (ek * ek));
-            acc += al[k] * dq[k][m] + (q[k] - val) * dal;
-        }
-        J[m] = acc * rS;
-    }
+    const double u0 = c0 * k13 * A0, v0 = c0 * 0.5 * B0, u1 = c1 * k13 * A1, v1 = c1 * 0.5 * B1, u2 = c2 * k13 * A2, v2 = c2 * 0.5 * B2;
+    const double w0 = a0 * rS * sixth, w1 = a1 * rS * sixth, w2 = a2 * rS * sixth;
+    J[0] = 2 * w0 + u0 + v0;
+    J[1] = -7 * w0 - w1 - 2 * u0 - 4 * v0 + u1 + v1;
+    J[2] = 11 * w0 + 5 * w1 + 2 * w2 + u0 + 3 * v0 - 2 * u1 + u2 + 3 * v2;
+    J[3] = 2 * w1 + 5 * w2 + u1 - v1 - 2 * u2 - 4 * v2;
+    J[4] = -w2 + u2 + v2;
 }
 __device__ __forceinline__ void face_value_gradient(const ThicknessView& v, const double* s, double* J) {
     if (v.scheme == NK_ADVECTION_WENO) { weno5_face_gradient(s, J); return; }

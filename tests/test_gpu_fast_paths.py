@@ -228,3 +228,48 @@ def test_weno_faces_and_limiter(oracle_cls, gpu_cls, nx, ny, topology, bounds):
         P.close()
     for g, w in zip(*out):
         assert np.max(np.abs(g - w)) <= 1e-12 * max(np.max(np.abs(w)), 1.0)
+
+
+# The reverse of a stage on axes where a stencil reaches past both edges, reads a cell twice or only just wraps: the
+# gradient of a weighted sum of the thickness after two steps against centred differences of the steps themselves.  One
+# FP64 step's rounding over the difference 2 x 1e-3 m leaves 1e-9 of a weight; the difference's own second-order error and
+# the limiter's kinks are kept below by a smooth field, so 1e-6 of the largest entry.
+@gpu
+@pytest.mark.parametrize("scheme", [nk.WENO(order=5, bounds=(0.0, 1e5)), nk.UpwindBiased(order=3)])
+@pytest.mark.parametrize("nx, ny, topology", [(4, 9, ("Periodic", "Bounded")), (5, 6, ("Periodic", "Periodic")), (9, 4, ("Bounded", "Bounded"))])
+def test_stage_reverse_on_short_axes(gpu_cls, nx, ny, topology, scheme):
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 1e3), y=(0.0, ny * 1e3), topology=topology, halo=(4, 4))
+    desc = nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(), grounding=nk.SubgridGroundedFraction())
+    x = (np.arange(nx)[None, :] + 0.5) / nx
+    y = (np.arange(ny)[:, None] + 0.5) / ny
+    H0 = 800.0 + 60.0 * np.sin(2 * np.pi * x + 0.3) + 45.0 * np.cos(2 * np.pi * y + 0.7) + 20.0 * np.sin(2 * np.pi * (x + y))
+    weight = np.random.default_rng(1).random((ny, nx)) + 0.5
+    r = np.random.default_rng(2)
+    P = gpu_cls(grid, desc)
+    P.set("bed", -300.0)
+    u, v = 1e-5 * (1 + 0.3 * r.standard_normal(P.shape("u"))), 1e-5 * (-1 + 0.3 * r.standard_normal(P.shape("v")))
+    P.set_thickness_advection(scheme)
+    P.energy_set("surface_mass_balance", 1e-8)
+    dt = 4e6
+
+    def start(H):
+        P.set("H", H)
+        P.set("u", u)
+        P.set("v", v)
+        P.compute_geometry()
+
+    def forward(H):
+        start(H)
+        for _ in range(2):
+            P.step_thickness(dt)
+        return P.get("H")
+
+    start(H0)
+    g = P.checkpointed_gradient(lambda step, H, *_: (float(np.sum(weight * H)), weight, None, None) if step == 2 else None, dt, 2,
+                                velocity_solves=False)["H"]
+    for j, i in ((0, 0), (ny - 1, nx - 1), (ny // 2, 0), (0, nx // 2), (ny // 2, nx - 1)):
+        d = np.zeros_like(H0)
+        d[j, i] = 1e-3
+        diff = np.sum(weight * (forward(H0 + d) - forward(H0 - d))) / 2e-3
+        assert abs(g[j, i] - diff) <= 1e-6 * np.max(np.abs(g))
+    P.close()
