@@ -22,7 +22,8 @@
 // against 125.9), 256 threads (71.7) and levels of 1024 cells kept inside the first CTA, without cluster barriers but with
 // its one shared-memory pipe (72.4).
 // Measured, a whole CG iteration, grid-wide launches with the former one-block coarsest kernel against this one:
-// 128 x 64 mixed 105 -> 67 us, 320 x 160 DIVA 182 -> 110, 1024 x 512 297 -> 254, 300 x 180 FP64 203 -> 167.
+// 128 x 64 mixed 105 -> 67 us, 320 x 160 DIVA 182 -> 110, 1024 x 512 297 -> 254, 300 x 180 FP64 203 -> 167.  Where the
+// cluster holds the finest level too it also takes the step's r.z: 128 x 64 mixed 51 -> 48 us against a pass of its own.
 #include <cooperative_groups.h>
 
 #include <mutex>
@@ -232,10 +233,10 @@ __device__ __forceinline__ void restriction_axis(int I, int Nc, int Nf, bool per
 }
 
 template <typename T, int CPT>
-__global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __grid_constant__ ClusterLevels<T> C, const int* done) {
+__global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __grid_constant__ ClusterLevels<T> C, const int* done, CGDot dot) {
     long long d;
     if (!batch_slot(C.lv[0].o.g, d)) return;   // the same answer in every CTA of a cluster (one slot)
-    if (d) rebase(done, d);
+    if (d) { rebase(done, d); rebase(dot, d); }
     if (done && *(volatile const int*)done) return;
     using V2 = typename Vec2<T>::type;
     cg::cluster_group cl = cg::this_cluster();
@@ -378,13 +379,45 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
         coarse_buf = cur;
         K = N;
     }
+    double rz = 0.0;
+    const int ze = dot.r && sizeof(T) == 4 ? dot.sc->r32_exp : 0;
 #pragma unroll
     for (int k = 0; k < CPT; ++k)
         if (c.p[k] >= 0) {
             const int e = (int)threadIdx.x + k * CLUSTER_THREADS, i = cell_i<T, CPT>(c, k);
-            K.x[(K.j0 + (e - i) / K.Nx) * K.pitch + i] = c.x[k];
+            const int q = (K.j0 + (e - i) / K.Nx) * K.pitch + i;
+            K.x[q] = c.x[k];
+            if (dot.r) {   // z = x 2^ze
+                const double2 r = dot.r[q];
+                if constexpr (sizeof(T) == 4) rz = fma(r.x, widen_pow2(c.x[k].x, ze), fma(r.y, widen_pow2(c.x[k].y, ze), rz));
+                else rz = fma(r.x, c.x[k].x, fma(r.y, c.x[k].y, rz));
+            }
         }
-    cl.sync();   // no CTA leaves while another may still read its shared memory
+    if (!dot.r) {
+        cl.sync();   // no CTA leaves while another may still read its shared memory
+        return;
+    }
+    // the CTA's sum by one warp, then the CTAs' sums in the first CTA: fixed trees
+    __shared__ double sums[CLUSTER_THREADS], ctas[CLUSTER_MAX_CTAS];
+    sums[threadIdx.x] = rz;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        double a[CLUSTER_THREADS / 32];
+#pragma unroll
+        for (int k = 0; k < CLUSTER_THREADS / 32; ++k) a[k] = sums[threadIdx.x + 32 * k];
+#pragma unroll
+        for (int h = CLUSTER_THREADS / 64; h > 0; h >>= 1)
+#pragma unroll
+            for (int k = 0; k < h; ++k) a[k] += a[k + h];
+        const double t = warp_sum(a[0]);
+        if (threadIdx.x == 0) *cl.map_shared_rank(&ctas[rank], 0) = t;
+    }
+    const CGDotScalars scalars(dot.sc);
+    cl.sync();   // the sums are there, and no CTA leaves while another may still read its shared memory
+    if (rank == 0 && threadIdx.x < 32) {
+        const double t = warp_sum((int)threadIdx.x < C.ctas ? ctas[threadIdx.x] : 0.0);
+        if (threadIdx.x == 0) scalars.finish(dot, t);
+    }
 }
 
 // Rows per CTA and buffer offsets of levels lv[0 .. n-1] (lv[0] the finest of them); false if they do not fit.
@@ -415,7 +448,7 @@ bool cluster_plan(ClusterLevels<T>& C) {
 }
 
 template <typename T, int CPT>
-static void launch_cluster(const ClusterLevels<T>& C, const int* done, cudaStream_t s) {
+static void launch_cluster(const ClusterLevels<T>& C, const int* done, const CGDot& dot, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C.ctas, 1, batch_slots());
     cfg.blockDim = dim3(CLUSTER_THREADS);
@@ -428,15 +461,16 @@ static void launch_cluster(const ClusterLevels<T>& C, const int* done, cudaStrea
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_coarse_cluster<T, CPT>, C, done);
+    cudaLaunchKernelEx(&cfg, k_coarse_cluster<T, CPT>, C, done, dot);
 }
 template <typename T>
-void launch_coarse_cluster(const ClusterLevels<T>& C, const int* done, cudaStream_t s) {
+void launch_coarse_cluster(const ClusterLevels<T>& C, const int* done, const CGDot* with, cudaStream_t s) {
+    const CGDot dot = with ? *with : CGDot{};
     if constexpr (cluster_max_cells<T>() >= 2) {
-        if (C.cells == 2) launch_cluster<T, 2>(C, done, s);
-        else launch_cluster<T, 1>(C, done, s);
+        if (C.cells == 2) launch_cluster<T, 2>(C, done, dot, s);
+        else launch_cluster<T, 1>(C, done, dot, s);
     } else {
-        launch_cluster<T, 1>(C, done, s);
+        launch_cluster<T, 1>(C, done, dot, s);
     }
     count_launch();
 }
@@ -463,7 +497,7 @@ void configure_coarse_cluster() {
 
 template bool cluster_plan<float>(ClusterLevels<float>&);
 template bool cluster_plan<double>(ClusterLevels<double>&);
-template void launch_coarse_cluster<float>(const ClusterLevels<float>&, const int*, cudaStream_t);
-template void launch_coarse_cluster<double>(const ClusterLevels<double>&, const int*, cudaStream_t);
+template void launch_coarse_cluster<float>(const ClusterLevels<float>&, const int*, const CGDot*, cudaStream_t);
+template void launch_coarse_cluster<double>(const ClusterLevels<double>&, const int*, const CGDot*, cudaStream_t);
 
 }  // namespace nk

@@ -94,6 +94,33 @@ void launch_cg_apply(const CGView& v, cudaStream_t s);
 void launch_cg_update(const CGView& v, cudaStream_t s);
 // multigrid: z = V(r) done; r.z, beta
 void launch_cg_dots_after_precondition(const CGView& v, cudaStream_t s);
+// The r.z of a conjugate-gradient step (or of its start) taken by the kernel that finishes the V-cycle, where z is at
+// hand: what launch_cg_dots_after_precondition and launch_cg_init_finish do in a pass of their own.
+struct CGDot {
+    const double2* r = nullptr;
+    SolverScalars* sc = nullptr;
+    double2* partials = nullptr;
+    unsigned long long cond = 0;
+    int start = 0;
+};
+__device__ __forceinline__ void rebase(CGDot& v, long long d) { shift_ptr(v.r, d); shift_ptr(v.sc, d); shift_ptr(v.partials, d); }
+// the scalars beta needs, read before the sum is complete
+struct CGDotScalars {
+    double rho, rz_old;
+    int flexible, done;
+    __device__ __forceinline__ explicit CGDotScalars(const SolverScalars* sc)
+        : rho(sc->rho), rz_old(sc->rz_old), flexible(sc->flexible), done(sc->done) {}
+    // beta = rho_new / rho, or the flexible (Polak-Ribière) form (r.z - r.z_old) / rho when the preconditioner varies
+    __device__ __forceinline__ void finish(const CGDot& v, double rz) const {
+        if (v.start) {
+            if (v.cond) cudaGraphSetConditional(v.cond, done ? 0u : 1u);
+        } else {
+            const double num = flexible ? (rz - rz_old) : rz;
+            v.sc->beta = (rho == 0.0) ? 0.0 : num / rho;
+        }
+        v.sc->rho = rz;
+    }
+};
 // z = r * invd on the Nx x Ny range, z = r on the wall faces (unit diagonal)
 void launch_precondition_diagonal(const DevGrid<double>& g, double2* z, const double2* r, const double2* invd, cudaStream_t s);
 // Picard: xprev = x (over the Nx x Ny range)
@@ -409,7 +436,8 @@ template <typename T>
 void launch_vcycle_down(const LevelView<T>& L, const LevelView<T>& C, typename Vec2<T>::type* x2, const int* done, cudaStream_t s);
 template <typename T>
 void launch_vcycle_up(const LevelView<T>& L, const LevelView<T>& C, const typename Vec2<T>::type* x2, const typename Vec2<T>::type* xc,
-                      typename Vec2<T>::type* xout, const int* done, cudaStream_t s);
+                      typename Vec2<T>::type* xout, const int* done, const CGDot* dot, cudaStream_t s);
+size_t vcycle_up_blocks(int Nx, int Ny);   // its blocks on an Nx x Ny level: the partial sums of r.z
 // The levels from lv[0] down to the coarsest, lv[n - 1], run by one thread-block cluster (nk_cluster.cu).
 template <typename T>
 struct ClusterLevels {
@@ -424,7 +452,7 @@ constexpr long long cluster_limit_cells(bool fp64) { return fp64 ? 8192 : 16384;
 template <typename T>
 bool cluster_plan(ClusterLevels<T>& C);   // fills rows, off, ctas, cells and total; false if the levels do not fit
 template <typename T>
-void launch_coarse_cluster(const ClusterLevels<T>& C, const int* done, cudaStream_t s);
+void launch_coarse_cluster(const ClusterLevels<T>& C, const int* done, const CGDot* dot, cudaStream_t s);
 void configure_coarse_cluster();
 // FP64 <-> FP32 conversions of vectors and of the coefficient record
 void launch_to_float(const DevGrid<double>& g, const double2* src, float2* dst, const int* done, cudaStream_t s);

@@ -479,9 +479,11 @@ static void build(nk_problem* P, bool dry = false) {
     slots.push_back({(void**)&P->usig, A.reserve(d2 * P->Ns)});
     P->staging_count = (size_t)(P->Nx + 1) * (P->Ny + 1) * P->Ns;
     slots.push_back({(void**)&P->staging, A.reserve(P->staging_count * sizeof(double))});
-    // the most blocks of a reduction: one a 2-D tile, or the resident blocks of operator_dims and vec_dims
+    // the most blocks of a reduction: one a 2-D tile, the resident blocks of operator_dims and vec_dims, or the walks of
+    // the V-cycle's last kernel
     LaunchDims big = dims2d(P->Nx + 1, P->Ny + 1);
     size_t nblocks = std::max((size_t)big.grid.x * big.grid.y, (size_t)8 * SM_COUNT);
+    if (P->precond == NK_PRECONDITIONER_MULTIGRID && P->mixed) nblocks = std::max(nblocks, vcycle_up_blocks(P->Nx, P->Ny));
     slots.push_back({(void**)&P->partials, A.reserve(nblocks * sizeof(double2))});
     slots.push_back({(void**)&P->sc, A.reserve(sizeof(SolverScalars))});
     slots.push_back({(void**)&P->sig_tables, A.reserve((4 * P->Ns + 1 + (size_t)P->Ns * P->Ns) * sizeof(double))});
@@ -664,9 +666,10 @@ static void smooth(nk_problem* P, Level<T>& L, int sweeps, bool first, const int
 
 // v_cycle!, multigrid_preconditioner.jl:144-163 (x ≈ A⁻¹ b from a zero guess on level l).  Levels from
 // `fused_level` down run in one k_coarse_vcycle launch; above it each phase is one grid-wide kernel, and the
-// restriction also performs the coarse level's first sweep from zero.
+// restriction also performs the coarse level's first sweep from zero.  `dot`: the last kernel also takes the r.z of the
+// conjugate-gradient step where it can; returns whether it did.
 template <typename T>
-static void v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* done, bool first_done = false) {
+static bool v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* done, bool first_done = false, const CGDot* dot = nullptr) {
     cudaStream_t s = P->stream;
     int lc = fused_level(lv, P->nlevels);
     if (l == lc) {
@@ -678,17 +681,17 @@ static void v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* 
         C.coarsest = P->sd.coarsest_sweeps;
         C.line = P->sd.smoother == NK_SMOOTHER_LINE_JACOBI;
         launch_coarse_vcycle<T>(C, done, s);
-        return;
+        return false;
     }
     Level<T>& L = lv[l];
     ClusterLevels<T> cluster;
     if (!first_done && plan_cluster(P, lv, l, cluster)) {
-        launch_coarse_cluster<T>(cluster, done, s);
-        return;
+        launch_coarse_cluster<T>(cluster, done, dot, s);
+        return dot != nullptr;
     }
     if (l == P->nlevels) {
         smooth(P, L, P->sd.coarsest_sweeps, true, done, first_done);
-        return;
+        return false;
     }
     if constexpr (sizeof(T) == 4) {
         // FP32, the default two point sweeps and both axes halved: one pass down and one up (nk_vcycle.cu).  In FP64 the
@@ -698,8 +701,8 @@ static void v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* 
             LevelView<T> f = P->level_view(L), c = P->level_view(N);
             launch_vcycle_down<T>(f, c, L.x2, done, s);
             v_cycle(P, lv, l + 1, done);
-            launch_vcycle_up<T>(f, c, L.x2, N.x, L.x, done, s);
-            return;
+            launch_vcycle_up<T>(f, c, L.x2, N.x, L.x, done, dot, s);
+            return dot != nullptr;
         }
     }
     smooth(P, L, P->sd.smoothing_sweeps, true, done, first_done);
@@ -714,20 +717,24 @@ static void v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* 
     v_cycle(P, lv, l + 1, done, fuse_first);
     launch_prolongate<T>(v, c, L.x, N.x, done, s);
     smooth(P, L, P->sd.smoothing_sweeps, false, done);
+    return false;
 }
 
 // z = M r with the multigrid preconditioner.  `fused`: inside conjugate gradients, where the FP32 copy of r
 // and the FP64 copy of the result are made by the CG kernels themselves (CGView::r32 / z32).
-static void precondition_mg(nk_problem* P, const int* done, bool fused = false) {
+// `dot`: the r.z to take (v_cycle); returns whether it was taken.
+static bool precondition_mg(nk_problem* P, const int* done, bool fused = false, const CGDot* dot = nullptr) {
     cudaStream_t s = P->stream;
+    bool taken;
     if (!P->mixed) {
-        v_cycle<double>(P, P->lv64, 0, done);
+        taken = v_cycle<double>(P, P->lv64, 0, done, false, dot);
     } else {
         if (!fused) launch_to_float(P->fine.g, P->r, P->lv32[0].b, done, s);
-        v_cycle<float>(P, P->lv32, 0, done);
+        taken = v_cycle<float>(P, P->lv32, 0, done, false, dot);
         if (!fused) launch_to_double(P->fine.g, P->lv32[0].x, P->z, done, s);
     }
     NK_CHECK_LAUNCH();
+    return taken;
 }
 
 // ---- conjugate gradients and Picard as CUDA graphs ------------------------------------------------------------
@@ -765,8 +772,8 @@ static void cg_step(nk_problem* P, const CGView& v) {
     launch_cg_apply(v, s);
     launch_cg_update(v, s);
     if (P->precond == NK_PRECONDITIONER_MULTIGRID) {
-        precondition_mg(P, &P->sc->done, true);
-        launch_cg_dots_after_precondition(v, s);
+        const CGDot dot{v.r, v.sc, v.partials, 0, 0};
+        if (!precondition_mg(P, &P->sc->done, true, &dot)) launch_cg_dots_after_precondition(v, s);
     }
 }
 
@@ -776,8 +783,8 @@ static void cg_start(nk_problem* P, const CGView& v) {
     launch_cg_init(v, P->stream);
     if (P->precond == NK_PRECONDITIONER_MULTIGRID) {
         if (v.r32) launch_cg_scale_r32(v, P->stream);
-        precondition_mg(P, nullptr, true);
-        launch_cg_init_finish(v, P->stream);
+        const CGDot dot{v.r, v.sc, v.partials, v.cond, 1};
+        if (!precondition_mg(P, nullptr, true, &dot)) launch_cg_init_finish(v, P->stream);
     }
     NK_CHECK_LAUNCH();
 }

@@ -309,10 +309,8 @@ __global__ void __launch_bounds__(256) k_cg_init_finish(CGView v) {
                 rz[0] = fma(r.x, z.x, fma(r.y, z.y, rz[0]));
             }
     });
-    if (grid_sum<1>(rz, v.partials, &v.sc->ticket) && threadIdx.x == 0 && threadIdx.y == 0) {
-        v.sc->rho = rz[0];
-        if (v.cond) cudaGraphSetConditional(v.cond, v.sc->done ? 0u : 1u);
-    }
+    if (grid_sum<1>(rz, v.partials, &v.sc->ticket) && threadIdx.x == 0 && threadIdx.y == 0)
+        CGDotScalars(v.sc).finish(CGDot{v.r, v.sc, v.partials, v.cond, 1}, rz[0]);
 }
 void launch_cg_init_finish(const CGView& v, cudaStream_t s) {
     LaunchDims d = vec_dims(v.o.g.Nx, v.o.g.Ny);
@@ -442,13 +440,12 @@ void launch_cg_update(const CGView& v, cudaStream_t s) {
     k_cg_update<<<d.grid, d.block, 0, s>>>(v); count_launch();
 }
 
-// after z = V-cycle(r): rho_new = r.z; beta = rho_new / rho, or the flexible (Polak-Ribière) form
-// beta = (r.z - r.z_old) / rho when the preconditioner varies between steps
+// after z = V-cycle(r), where its last kernel has not taken the sum itself: rho_new = r.z and beta
 __global__ void __launch_bounds__(256) k_cg_dots_after_precondition(CGView v) {
     NK_BATCH_ENTER(v.o.g, v)
     if (read_done(v.sc)) return;
-    const int ze = v.sc->r32_exp, flexible = v.sc->flexible;
-    const double rho = v.sc->rho, rz_old = v.sc->rz_old;
+    const int ze = v.sc->r32_exp;
+    const CGDotScalars scalars(v.sc);
     double rz[1] = {0.0};
     for_each_cell_pair(v.o.g.Nx, v.o.g.Ny, v.o.g.pitch, [&](const int* k, const bool* ok) {
         double2 z[2], r[2];
@@ -459,12 +456,8 @@ __global__ void __launch_bounds__(256) k_cg_dots_after_precondition(CGView v) {
         for (int a = 0; a < 2; ++a)
             if (ok[a]) rz[0] = fma(r[a].x, z[a].x, fma(r[a].y, z[a].y, rz[0]));
     });
-    if (grid_sum<1>(rz, v.partials, &v.sc->ticket) && threadIdx.x == 0 && threadIdx.y == 0) {
-        SolverScalars* sc = v.sc;
-        const double num = flexible ? (rz[0] - rz_old) : rz[0];
-        sc->beta = (rho == 0.0) ? 0.0 : num / rho;
-        sc->rho = rz[0];
-    }
+    if (grid_sum<1>(rz, v.partials, &v.sc->ticket) && threadIdx.x == 0 && threadIdx.y == 0)
+        scalars.finish(CGDot{v.r, v.sc, v.partials, 0, 0}, rz[0]);
 }
 void launch_cg_dots_after_precondition(const CGView& v, cudaStream_t s) {
     LaunchDims d = vec_dims(v.o.g.Nx, v.o.g.Ny);

@@ -170,11 +170,15 @@ __global__ void __launch_bounds__(32 * VCYCLE_WARPS) k_vcycle_down(LevelView<T> 
 }
 
 // The prolongation (prolonged) and two sweeps: xout = two sweeps of x2 + P xc.  Only for levels halved in both directions.
-template <typename T, bool UNI>
-__global__ void __launch_bounds__(32 * VCYCLE_WARPS) k_vcycle_up(LevelView<T> L, LevelView<T> C, const typename Vec2<T>::type* __restrict__ x2,
+// DOT: also the r.z of the conjugate-gradient step, z being xout 2^r32_exp (the finest level's way up).  A pass of its own
+// for it cost 5.5 us at 320 x 160 and 10 us at 2560 x 320; here a row's r is read a row ahead, and four blocks an SM are
+// kept (three rows ahead took 148 registers, three blocks, and a second wave: 2560 x 320 went from 192 to 202 us a step
+// instead of to 189).
+template <typename T, bool UNI, bool DOT>
+__global__ void __launch_bounds__(32 * VCYCLE_WARPS, UNI ? 4 : 3) k_vcycle_up(LevelView<T> L, LevelView<T> C, const typename Vec2<T>::type* __restrict__ x2,
                                                                 const typename Vec2<T>::type* __restrict__ xc,
-                                                                typename Vec2<T>::type* __restrict__ xout, int rows, const int* done) {
-    NK_BATCH_ENTER(L.o.g, L, C, x2, xc, xout, done)
+                                                                typename Vec2<T>::type* __restrict__ xout, int rows, const int* done, CGDot dot) {
+    NK_BATCH_ENTER(L.o.g, L, C, x2, xc, xout, done, dot)
     if (done && *(volatile const int*)done) return;
     using V2 = typename Vec2<T>::type;
     using Row = typename LevelColumn<T>::Row;
@@ -182,7 +186,11 @@ __global__ void __launch_bounds__(32 * VCYCLE_WARPS) k_vcycle_up(LevelView<T> L,
     const int lane = threadIdx.x;
     const int strip = blockIdx.x * VCYCLE_WARPS + threadIdx.y;
     const int j0 = blockIdx.y * rows, j1 = j0 + rows < g.Ny ? j0 + rows : g.Ny;
-    if (strip * UP_COLS >= g.Nx) return;   // whole warp
+    const bool active = strip * UP_COLS < g.Nx;   // whole warp
+    if (!DOT && !active) return;
+    double rz[1] = {0.0};
+    const int ze = DOT ? dot.sc->r32_exp : 0;
+    if (active) {
     const int i = strip * UP_COLS - UP_FIRST + lane;
     const LevelColumn<T> col(L, i);
     const bool own = lane >= UP_FIRST && lane < UP_FIRST + UP_COLS && i < g.Nx;
@@ -223,6 +231,8 @@ __global__ void __launch_bounds__(32 * VCYCLE_WARPS) k_vcycle_up(LevelView<T> L,
     const int ja = j0 - 2, jb = j1;
     Fine ring[4];
     V2 y;                                               // the first sweep at row j - 1, then at row j
+    double2 res = make_double2(0.0, 0.0);               // r at row j - 1
+    const double2* const rr = DOT ? dot.r + (own ? i : 0) : nullptr;
     fetch(ring[0], ja);
     fetch(ring[1], ja + 1);
     fetch(ring[2], ja + 2);
@@ -246,7 +256,9 @@ __global__ void __launch_bounds__(32 * VCYCLE_WARPS) k_vcycle_up(LevelView<T> L,
             o.x = prev.x + (old.b.x - (old.c.z * prev.x - eu)) * old.w.x;
             o.y = prev.y + (old.b.y - (old.c.w * prev.y - ev)) * old.w.y;
             xw[(j - 1) * g.pitch] = o;
+            if (DOT) rz[0] = fma(res.x, widen_pow2(o.x, ze), fma(res.y, widen_pow2(o.y, ze), rz[0]));
         }
+        if (DOT && j >= j0) res = rr[min(j, j1 - 1) * g.pitch];   // a row ahead
         fetch(fo, j + 3);
     };
     for (int j = ja; j <= jb; j += 4) {
@@ -257,6 +269,11 @@ __global__ void __launch_bounds__(32 * VCYCLE_WARPS) k_vcycle_up(LevelView<T> L,
         step(j + 2, ring[1], ring[2], ring[3]);
         if (j + 3 > jb) break;
         step(j + 3, ring[2], ring[3], ring[0]);
+    }
+    }
+    if constexpr (DOT) {
+        const CGDotScalars scalars(dot.sc);
+        if (grid_sum<1>(rz, dot.partials, &dot.sc->ticket) && threadIdx.x == 0 && threadIdx.y == 0) scalars.finish(dot, rz[0]);
     }
 }
 
@@ -275,17 +292,31 @@ void launch_vcycle_down(const LevelView<T>& L, const LevelView<T>& C, typename V
     else k_vcycle_down<T, false><<<grid, block, 0, s>>>(L, C, x2, rows, done);
     count_launch();
 }
+static dim3 vcycle_up_grid(int Nx, int Ny, int& rows) {
+    const int strips = (Nx + UP_COLS - 1) / UP_COLS;
+    rows = vcycle_rows(strips, Ny, 4);
+    return dim3((strips + VCYCLE_WARPS - 1) / VCYCLE_WARPS, (Ny + rows - 1) / rows);
+}
+size_t vcycle_up_blocks(int Nx, int Ny) {
+    int rows;
+    const dim3 grid = vcycle_up_grid(Nx, Ny, rows);
+    return (size_t)grid.x * grid.y;
+}
 template <typename T>
 void launch_vcycle_up(const LevelView<T>& L, const LevelView<T>& C, const typename Vec2<T>::type* x2, const typename Vec2<T>::type* xc,
-                      typename Vec2<T>::type* xout, const int* done, cudaStream_t s) {
-    const int strips = (L.o.g.Nx + UP_COLS - 1) / UP_COLS, rows = vcycle_rows(strips, L.o.g.Ny, 4);
-    dim3 block(32, VCYCLE_WARPS), grid((strips + VCYCLE_WARPS - 1) / VCYCLE_WARPS, (L.o.g.Ny + rows - 1) / rows, batch_slots());
-    if (L.o.g.h != T(0)) k_vcycle_up<T, true><<<grid, block, 0, s>>>(L, C, x2, xc, xout, rows, done);
-    else k_vcycle_up<T, false><<<grid, block, 0, s>>>(L, C, x2, xc, xout, rows, done);
+                      typename Vec2<T>::type* xout, const int* done, const CGDot* dot, cudaStream_t s) {
+    int rows;
+    dim3 block(32, VCYCLE_WARPS), grid = vcycle_up_grid(L.o.g.Nx, L.o.g.Ny, rows);
+    grid.z = batch_slots();
+    const bool uni = L.o.g.h != T(0);
+    if (dot && uni) k_vcycle_up<T, true, true><<<grid, block, 0, s>>>(L, C, x2, xc, xout, rows, done, *dot);
+    else if (dot) k_vcycle_up<T, false, true><<<grid, block, 0, s>>>(L, C, x2, xc, xout, rows, done, *dot);
+    else if (uni) k_vcycle_up<T, true, false><<<grid, block, 0, s>>>(L, C, x2, xc, xout, rows, done, CGDot{});
+    else k_vcycle_up<T, false, false><<<grid, block, 0, s>>>(L, C, x2, xc, xout, rows, done, CGDot{});
     count_launch();
 }
 template void launch_vcycle_down<float>(const LevelView<float>&, const LevelView<float>&, float2*, const int*, cudaStream_t);
 template void launch_vcycle_up<float>(const LevelView<float>&, const LevelView<float>&, const float2*, const float2*, float2*, const int*,
-                                      cudaStream_t);
+                                      const CGDot*, cudaStream_t);
 
 }  // namespace nk

@@ -165,6 +165,37 @@ def test_cg_steps_at_the_launch_shapes_edges(oracle_cls, gpu_cls, nx, ny, topolo
         assert np.max(np.abs(g - w)) <= 1e-12 * np.max(np.abs(w))
 
 
+# The r.z of a preconditioned step is taken by the kernel that ends the V-cycle: one cluster (60 x 40), the FP32 way up
+# with both metrics (200 x 150) and with more blocks than the grid has 2-D tiles (24 x 5000), and a pass of its own after
+# the grid-wide FP64 levels.  Three steps from rest against the oracle's: an FP64 V-cycle agrees to 1e-12 of its largest
+# value, and three steps' quotients leave that below 1e-9; an FP32 one to 1e-4, below 1e-3.
+@gpu
+@pytest.mark.parametrize("precision, tol", [("fp64", 1e-9), ("mixed", 1e-3)])
+@pytest.mark.parametrize("nx, ny, topology, stretch", [
+    (60, 40, ("Bounded", "Bounded"), 1.0),
+    (200, 150, ("Periodic", "Bounded"), 1.0),
+    (200, 150, ("Bounded", "Bounded"), 1.25),
+    (24, 5000, ("Bounded", "Periodic"), 1.0),
+])
+def test_preconditioned_steps(oracle_cls, gpu_cls, nx, ny, topology, stretch, precision, tol):
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 2e3 * stretch), topology=topology)
+    H = np.clip(1000.0 + 300.0 * np.random.default_rng(nx).standard_normal((ny, nx)), 100.0, None)
+    out = []
+    for cls, p in ((gpu_cls, precision), (oracle_cls, "fp64")):
+        solver = nk.StressBalanceSolver(linear_iteration_control=nk.FixedIterations(3), picard_iteration_control=nk.FixedIterations(1),
+                                        preconditioner=nk.StressBalanceMultigridPreconditioner(minimum_coarse_size=8), precision=p)
+        P = cls(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                                          stress_balance=nk.DepthIntegrated(side_walls=nk.NoSlipWalls()), velocity_solver=solver))
+        for n, a in (("H", H), ("bed", 10.0), ("C", 1e9), ("A", 3e-24)):
+            P.set(n, a)
+        P.compute_geometry()
+        assert P.picard_solve().linear_iterations_total == 3
+        out.append((P.get("u"), P.get("v")))
+        P.close()
+    for g, w in zip(*out):
+        assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
+
+
 # The FP64 <-> FP32 conversions on the integer units are the hardware conversions' bits, so a mixed solve keeps its
 # residuals' scale: right-hand sides far outside the FP32 range (2^-400 to 2^400, whose squared norms FP64 still holds)
 # converge in the same steps, to the same digits, as those near one.
