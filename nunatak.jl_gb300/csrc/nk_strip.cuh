@@ -412,7 +412,8 @@ struct Stage {
             rdxc = g.rdxc[iw]; dxc = g.dxc[iw]; rdxf = g.rdxf[iw]; dxf = g.dxf[iw];
         }
     }
-    __device__ __forceinline__ void push(int jm, T un, T vn, T eta, T cff, T& divu, T& divv) {   // jm: the stored row of j
+    __device__ __forceinline__ void push(int jm, int jf, T un, T vn, T eta, T cff, T& divu, T& divv) {
+        // jm: the stored row of j, jf: the face row j + 1 (0 below a Bounded edge, where row 0 stands for the rows below it)
         const unsigned full = 0xffffffffu;
         const T ue = __shfl_down_sync(full, mu, 1), vw = __shfl_up_sync(full, vn, 1);
         const T du = ue - mu, dv = vn - mv;
@@ -425,7 +426,7 @@ struct Stage {
             const T exx = du * rdxc, eyy = dv * g.rdyc[jm], e2 = T(2) * eta;
             sx = g.dyc[jm] * (e2 * (T(2) * exx + eyy));
             syn = dxc * (e2 * (T(2) * eyy + exx));
-            tn = cff * ((un - mu) * g.rdyf[jm + 1] + (vn - vw) * rdxf);
+            tn = cff * ((un - mu) * g.rdyf[jf] + (vn - vw) * rdxf);
         }
         const T sxw = __shfl_up_sync(full, sx, 1), te = __shfl_down_sync(full, t, 1);
         if (UNI) {
@@ -492,7 +493,7 @@ __device__ __forceinline__ void strip_march(const OpView<T>& o, Load&& load, Val
         if (j + 3 <= j1) fetch(far, j + 3);
         settle(nxt, j + 1);
         T du, dv;
-        s.push(UNI ? 0 : row(j), (nxt.m & U_INACTIVE) ? T(0) : nxt.x.x, (nxt.m & V_INACTIVE) ? T(0) : nxt.x.y, cur.c.x, nxt.c.y, du, dv);
+        s.push(UNI ? 0 : row(j), UNI ? 0 : (!g.py && j < 0 ? 0 : row(j) + 1), (nxt.m & U_INACTIVE) ? T(0) : nxt.x.x, (nxt.m & V_INACTIVE) ? T(0) : nxt.x.y, cur.c.x, nxt.c.y, du, dv);
         if (own && j >= j0) {
             const T au = UNI ? h2 : g.dxf[i] * g.dyc[j], av = UNI ? h2 : g.dxc[i] * g.dyf[j];
             V2 q;

@@ -45,6 +45,7 @@ struct LevelColumn {
         if (g.py) return j < 0 ? j + g.Ny : (j >= g.Ny ? j - g.Ny : j);
         return j < 0 ? 0 : (j > g.Ny ? g.Ny : j);
     }
+    __device__ __forceinline__ int face(int j) const { return !L.o.g.py && j < 0 ? 0 : row(j) + 1; }   // Stage::push's jf
     template <bool WITH_X>
     __device__ __forceinline__ void fetch(Row& r, int j, const V2* __restrict__ x) const {
         const DevGrid<T>& g = L.o.g;
@@ -122,14 +123,14 @@ __global__ void __launch_bounds__(32 * VCYCLE_WARPS) k_vcycle_down(LevelView<T> 
     auto step = [&](int j, Row& old, Row& cur, Row& nxt) {
         col.template settle<UNI, false>(nxt, j + 1);
         T du, dv;
-        s1.push(UNI ? 0 : col.row(j), active_u<T>(nxt, nxt.x.x), active_v<T>(nxt, nxt.x.y), cur.c.x, nxt.c.y, du, dv);
+        s1.push(UNI ? 0 : col.row(j), UNI ? 0 : col.face(j), active_u<T>(nxt, nxt.x.x), active_v<T>(nxt, nxt.x.y), cur.c.x, nxt.c.y, du, dv);
         const V2 prev = x;
         x.x = cur.x.x + (cur.b.x - (cur.c.z * cur.x.x - du)) * cur.w.x;   // the second sweep at row j
         x.y = cur.x.y + (cur.b.y - (cur.c.w * cur.x.y - dv)) * cur.w.y;
         if (xw && j >= 2 * J0 && j < 2 * J1) xw[j * g.pitch] = x;
         const T mx = active_u<T>(cur, x.x), my = active_v<T>(cur, x.y);
         T eu, ev;                                   // the residual of row j - 1
-        s2.push(UNI ? 0 : col.row(j - 1), mx, my, old.c.x, cur.c.y, eu, ev);
+        s2.push(UNI ? 0 : col.row(j - 1), UNI ? 0 : col.face(j - 1), mx, my, old.c.x, cur.c.y, eu, ev);
         const T ru = active_u<T>(old, old.b.x - ((old.m & U_DIRICHLET) ? prev.x : old.c.z * prev.x - eu));
         const T rv = active_v<T>(old, old.b.y - ((old.m & V_DIRICHLET) ? prev.y : old.c.w * prev.y - ev));
         const unsigned full = 0xffffffffu;
@@ -245,12 +246,12 @@ __global__ void __launch_bounds__(32 * VCYCLE_WARPS, UNI ? 4 : 3) k_vcycle_up(Le
         settle(fn, j + 1);
         const Row &old = fo.r, &cur = fc.r, &nxt = fn.r;
         T du, dv;
-        s1.push(UNI ? 0 : col.row(j), active_u<T>(nxt, nxt.x.x), active_v<T>(nxt, nxt.x.y), cur.c.x, nxt.c.y, du, dv);
+        s1.push(UNI ? 0 : col.row(j), UNI ? 0 : col.face(j), active_u<T>(nxt, nxt.x.x), active_v<T>(nxt, nxt.x.y), cur.c.x, nxt.c.y, du, dv);
         const V2 prev = y;
         y.x = cur.x.x + (cur.b.x - (cur.c.z * cur.x.x - du)) * cur.w.x;
         y.y = cur.x.y + (cur.b.y - (cur.c.w * cur.x.y - dv)) * cur.w.y;
         T eu, ev;                                       // the second sweep at row j - 1
-        s2.push(UNI ? 0 : col.row(j - 1), active_u<T>(cur, y.x), active_v<T>(cur, y.y), old.c.x, cur.c.y, eu, ev);
+        s2.push(UNI ? 0 : col.row(j - 1), UNI ? 0 : col.face(j - 1), active_u<T>(cur, y.x), active_v<T>(cur, y.y), old.c.x, cur.c.y, eu, ev);
         if (xw && j > j0 && j <= j1) {
             V2 o;
             o.x = prev.x + (old.b.x - (old.c.z * prev.x - eu)) * old.w.x;

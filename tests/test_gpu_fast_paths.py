@@ -196,6 +196,39 @@ def test_preconditioned_steps(oracle_cls, gpu_cls, nx, ny, topology, stretch, pr
         assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
 
 
+# Axes of unequal spacing: at a wall the face spacing (the edge cell's own width) is not that of the next face, and with
+# no-slip walls the corners on the wall enter the rows beside it.  Ten steps against the oracle's as above (1e-12), and an
+# FP32 V-cycle against its FP64 one (1e-4).
+@gpu
+@pytest.mark.parametrize("nx, ny, topology", [(70, 61, ("Bounded", "Bounded")), (160, 150, ("Bounded", "Bounded")), (160, 150, ("Periodic", "Periodic"))])
+def test_unequal_spacing_at_the_walls(oracle_cls, gpu_cls, nx, ny, topology):
+    rng = np.random.default_rng(nx)
+    faces = [np.concatenate([[0.0], np.cumsum(rng.uniform(1e3, 3e3, n))]).tolist() for n in (nx, ny)]
+    grid = nk.RectilinearGrid(size=(nx, ny), x=faces[0], y=faces[1], topology=topology)
+    H = np.clip(1000.0 + 300.0 * rng.standard_normal((ny, nx)), 100.0, None)
+    ru, rv = 1e10 * rng.standard_normal((ny, grid.face_count(0))), 1e10 * rng.standard_normal((grid.face_count(1), nx))
+    for kw, tol in ((dict(), 1e-12), (dict(preconditioner=nk.StressBalanceMultigridPreconditioner(minimum_coarse_size=20)), 1e-4)):
+        out = []
+        for cls in (gpu_cls, oracle_cls):
+            mixed = {"precision": "mixed"} if kw and cls is gpu_cls else {}
+            solver = nk.StressBalanceSolver(linear_iteration_control=nk.FixedIterations(10),
+                                            picard_iteration_control=nk.FixedIterations(1), **kw, **mixed)
+            P = cls(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                                              stress_balance=nk.DepthIntegrated(side_walls=nk.NoSlipWalls()), velocity_solver=solver))
+            for n, a in (("H", H), ("bed", 10.0), ("C", 1e9), ("A", 3e-24)):
+                P.set(n, a)
+            P.compute_geometry()
+            if kw:
+                P.update_coefficients()
+                out.append([a[:ny, :nx] for a in P.precondition(ru, rv)])
+            else:
+                P.picard_solve()
+                out.append([P.get("u"), P.get("v")])
+            P.close()
+        for g, w in zip(*out):
+            assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
+
+
 # The FP64 <-> FP32 conversions on the integer units are the hardware conversions' bits, so a mixed solve keeps its
 # residuals' scale: right-hand sides far outside the FP32 range (2^-400 to 2^400, whose squared norms FP64 still holds)
 # converge in the same steps, to the same digits, as those near one.
