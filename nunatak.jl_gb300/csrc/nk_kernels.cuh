@@ -121,6 +121,23 @@ struct CGDotScalars {
         v.sc->rho = rz;
     }
 };
+// The stopping rule's settings, read at a kernel's start so that the last block's decision waits for no load
+struct StopRule {
+    double tol;
+    int fixed, iterations, maxiter;
+    __device__ __forceinline__ explicit StopRule(const SolverScalars* sc)
+        : tol(sc->tol), fixed(sc->fixed), iterations(sc->iterations), maxiter(sc->maxiter) {}
+    __device__ __forceinline__ int stop(double rnorm, int it) const {
+        if (!finite_bits(rnorm)) return 1;
+        if (fixed) return it >= iterations;
+        return !(rnorm > tol && it < maxiter);
+    }
+};
+__device__ __forceinline__ int read_done(const SolverScalars* sc) { return *(volatile const int*)&sc->done; }
+// The whole iteration after launch_cg_init, without multigrid, in one thread-block cluster (nk_cg_cluster.cu).
+int cg_cluster_rows(int Nx, int Ny);   // rows per CTA, 0 if the grid does not fit
+void launch_cg_cluster(const CGView& v, cudaStream_t s);
+void configure_cg_cluster();
 // z = r * invd on the Nx x Ny range, z = r on the wall faces (unit diagonal)
 void launch_precondition_diagonal(const DevGrid<double>& g, double2* z, const double2* r, const double2* invd, cudaStream_t s);
 // Picard: xprev = x (over the Nx x Ny range)

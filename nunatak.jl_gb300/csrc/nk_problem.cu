@@ -743,7 +743,7 @@ static bool precondition_mg(nk_problem* P, const int* done, bool fused = false, 
 // so a solve needs no host round trip until it has finished:
 //
 //   picard_begin ─► WHILE(picard) { x⁻ = x ─► coefficient update ─► coarse coefficients ─► CG start
-//                                    ─► WHILE(cg) { apply ─► update ─► [V-cycle ─► dots] }
+//                                    ─► WHILE(cg) { apply ─► update ─► [V-cycle ─► dots] }, or one cluster kernel
 //                                    ─► picard_end (Δ, X, stopping test) }
 static SolverScalars control_scalars(const nk_problem* P) {
     SolverScalars h{};
@@ -775,6 +775,13 @@ static void cg_step(nk_problem* P, const CGView& v) {
         const CGDot dot{v.r, v.sc, v.partials, 0, 0};
         if (!precondition_mg(P, &P->sc->done, true, &dot)) launch_cg_dots_after_precondition(v, s);
     }
+}
+
+// Whether one cluster runs the whole iteration (launch_cg_cluster) in place of the loop of cg_step: without multigrid, on
+// every grid that fits, one solve or a batch of them (a step of 84 x 40 takes 7.0 us, 16.6 in grid-wide kernels; of 128 x 64
+// 9.4 against 16.8; of 32 such in a batch 47 against 81).
+static bool cg_in_cluster(const nk_problem* P) {
+    return P->precond != NK_PRECONDITIONER_MULTIGRID && cg_cluster_rows(P->Nx, P->Ny) > 0;
 }
 
 // conjugate_gradient!, conjugate_gradient.jl:165-171 (everything before the iteration loop)
@@ -928,21 +935,25 @@ static void build_picard_graph(nk_problem* P) {
     NK_CUDA(cudaGraphConditionalHandleCreate(&hp, g, 0, 0));
     capture_into(P, g, {}, [&] { launch_picard_begin(P->sc, hp, 0, P->stream); });
     cudaGraph_t body = add_while(g, leaves(g), hp);
-    cudaGraphConditionalHandle hc;
-    NK_CUDA(cudaGraphConditionalHandleCreate(&hc, body, 0, 0));
+    const bool cluster = cg_in_cluster(P);
+    cudaGraphConditionalHandle hc = 0;
+    if (!cluster) NK_CUDA(cudaGraphConditionalHandleCreate(&hc, body, 0, 0));
     CGView v = P->cg_view(P->tau);
     v.cond = hc;
     capture_into(P, body, {}, [&] {
         launch_copy_range(P->fine.g, P->xprev, P->x, P->stream);
         update_coefficients(P);
         cg_start(P, v);
+        if (cluster) launch_cg_cluster(v, P->stream);
     });
-    cudaGraph_t cg_body = add_while(body, leaves(body), hc);
-    capture_into(P, cg_body, {}, [&] { cg_step(P, v); });
+    if (!cluster) {
+        cudaGraph_t cg_body = add_while(body, leaves(body), hc);
+        capture_into(P, cg_body, {}, [&] { cg_step(P, v); });
+        P->picard_kernels[2] = kernel_nodes(cg_body);
+    }
     capture_into(P, body, leaves(body), [&] { picard_end(P, hp); });
     P->picard_kernels[0] = kernel_nodes(g);
     P->picard_kernels[1] = kernel_nodes(body);
-    P->picard_kernels[2] = kernel_nodes(cg_body);
     auto ti0 = std::chrono::steady_clock::now();
     NK_CUDA(cudaGraphInstantiate(&P->picard_exec, g, 0));
     P->instantiate_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - ti0).count();
@@ -953,15 +964,21 @@ static void build_linear_graph(nk_problem* P) {
     autotune_strips(P);
     cudaGraph_t g;
     NK_CUDA(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle hc;
-    NK_CUDA(cudaGraphConditionalHandleCreate(&hc, g, 0, 0));
+    const bool cluster = cg_in_cluster(P);
+    cudaGraphConditionalHandle hc = 0;
+    if (!cluster) NK_CUDA(cudaGraphConditionalHandleCreate(&hc, g, 0, 0));
     CGView v = P->cg_view(P->tmp_b);
     v.cond = hc;
-    capture_into(P, g, {}, [&] { cg_start(P, v); });
-    cudaGraph_t cg_body = add_while(g, leaves(g), hc);
-    capture_into(P, cg_body, {}, [&] { cg_step(P, v); });
+    capture_into(P, g, {}, [&] {
+        cg_start(P, v);
+        if (cluster) launch_cg_cluster(v, P->stream);
+    });
+    if (!cluster) {
+        cudaGraph_t cg_body = add_while(g, leaves(g), hc);
+        capture_into(P, cg_body, {}, [&] { cg_step(P, v); });
+        P->linear_kernels[1] = kernel_nodes(cg_body);
+    }
     P->linear_kernels[0] = kernel_nodes(g);
-    P->linear_kernels[1] = kernel_nodes(cg_body);
     NK_CUDA(cudaGraphInstantiate(&P->linear_exec, g, 0));
     P->linear_graph = g;
 }
@@ -989,6 +1006,12 @@ static void host_cg(nk_problem* P, const double2* b) {
     autotune_strips(P);
     CGView v = P->cg_view(b);
     cg_start(P, v);
+    if (cg_in_cluster(P)) {
+        launch_cg_cluster(v, P->stream);
+        NK_CHECK_LAUNCH();
+        read_scalars(P);
+        return;
+    }
     const nk_iteration_control& ctl = P->sd.linear;
     int limit = ctl.kind == NK_FIXED_ITERATIONS ? ctl.iterations : ctl.maxiter;
     int issued = 0, batch = 4;
@@ -1397,6 +1420,7 @@ static nk_status problem_create(nk_context* ctx, const nk_grid_desc* grid, const
         NK_CUDA(cudaEventCreate(&P->ev1));
         build(P);
         if (P->precond == NK_PRECONDITIONER_MULTIGRID) configure_coarse_cluster();   // outside any capture
+        else if (cg_in_cluster(P)) configure_cg_cluster();
         P->gd.x_faces = nullptr; P->gd.y_faces = nullptr; P->gd.sigma_faces = nullptr;   // no pointer kept after the call
         NK_CUDA(cudaStreamSynchronize(P->stream));
     });
@@ -2832,28 +2856,32 @@ static void build_batch_graph(nk_batch* B) {
             launch_batch_condition(P->sc, stride, S, 0, hp, cp, P->stream);
         });
         cudaGraph_t body = add_while(g, leaves(g), hp);
-        cudaGraphConditionalHandle hc;
-        NK_CUDA(cudaGraphConditionalHandleCreate(&hc, body, 0, 0));
+        cudaGraphConditionalHandle hc = 0;
+        if (!cg_in_cluster(P)) NK_CUDA(cudaGraphConditionalHandleCreate(&hc, body, 0, 0));
         CGView v = P->cg_view(P->tau);   // its grids carry the stride (set above)
         v.cond = 0;
+        const bool cluster = cg_in_cluster(P);
         capture_into(P, body, {}, [&] {
             launch_copy_range(P->fine.g, P->xprev, P->x, P->stream);
             update_coefficients(P);
             cg_start(P, v);
-            launch_batch_condition(P->sc, stride, S, 1, hc, cc, P->stream);
+            if (cluster) launch_cg_cluster(v, P->stream);
+            else launch_batch_condition(P->sc, stride, S, 1, hc, cc, P->stream);
         });
-        cudaGraph_t cg_body = add_while(body, leaves(body), hc);
-        capture_into(P, cg_body, {}, [&] {
-            cg_step(P, v);
-            launch_batch_condition(P->sc, stride, S, 1, hc, cc, P->stream);
-        });
+        if (!cluster) {
+            cudaGraph_t cg_body = add_while(body, leaves(body), hc);
+            capture_into(P, cg_body, {}, [&] {
+                cg_step(P, v);
+                launch_batch_condition(P->sc, stride, S, 1, hc, cc, P->stream);
+            });
+            B->kernels[2] = kernel_nodes(cg_body);
+        }
         capture_into(P, body, leaves(body), [&] {
             picard_end(P, 0);
             launch_batch_condition(P->sc, stride, S, 0, hp, cp, P->stream);
         });
         B->kernels[0] = kernel_nodes(g);
         B->kernels[1] = kernel_nodes(body);
-        B->kernels[2] = kernel_nodes(cg_body);
         NK_CUDA(cudaGraphInstantiate(&B->exec, g, 0));
     } catch (...) {
         set_batch_grids(P, 0);

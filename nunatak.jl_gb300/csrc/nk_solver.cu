@@ -212,20 +212,6 @@ template void launch_inverse_row_sum<double>(const OpView<double>&, double2*, cu
 template void launch_inverse_row_sum<float>(const OpView<float>&, float2*, cudaStream_t, float4*);
 
 // ---- conjugate gradients ------------------------------------------------------------------------------------
-__device__ __forceinline__ int read_done(const SolverScalars* sc) { return *(volatile const int*)&sc->done; }
-
-// The stopping rule's settings, read at a kernel's start so that the last block's decision waits for no load
-struct StopRule {
-    double tol;
-    int fixed, iterations, maxiter;
-    __device__ __forceinline__ explicit StopRule(const SolverScalars* sc)
-        : tol(sc->tol), fixed(sc->fixed), iterations(sc->iterations), maxiter(sc->maxiter) {}
-    __device__ __forceinline__ int stop(double rnorm, int it) const {
-        if (!finite_bits(rnorm)) return 1;
-        if (fixed) return it >= iterations;
-        return !(rnorm > tol && it < maxiter);
-    }
-};
 
 // conjugate_gradient!, conjugate_gradient.jl:165-171: r = b - A x, z = M r, p = z, rho = r.z
 template <bool UNI>

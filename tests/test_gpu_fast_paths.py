@@ -196,6 +196,41 @@ def test_preconditioned_steps(oracle_cls, gpu_cls, nx, ny, topology, stretch, pr
         assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
 
 
+# Conjugate gradients in one cluster: fewer rows than CTAs, several rows a CTA with a shorter last one, a full row of
+# threads (512 columns) and one column more (the grid-wide kernels), both seams, with the Jacobi preconditioner and without.
+# Ten steps against the oracle's as above (1e-12), and one solve to convergence in the oracle's number of steps.
+@gpu
+@pytest.mark.parametrize("preconditioner", [nk.StressBalanceDiagonalPreconditioner(), None])
+@pytest.mark.parametrize("nx, ny, topology", [
+    (4, 4, ("Periodic", "Periodic")),
+    (5, 33, ("Bounded", "Periodic")),
+    (9, 300, ("Periodic", "Bounded")),
+    (64, 128, ("Bounded", "Bounded")),
+    (512, 16, ("Bounded", "Bounded")),
+    (513, 16, ("Periodic", "Bounded")),
+])
+def test_cg_in_a_cluster(oracle_cls, gpu_cls, nx, ny, topology, preconditioner):
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 2e3), topology=topology)
+    H = np.clip(1000.0 + 300.0 * np.random.default_rng(nx).standard_normal((ny, nx)), 0.0, None)
+    H[ny // 3] = 0.0
+    for control, tol in ((nk.FixedIterations(10), 1e-12), (nk.Convergence(reltol=1e-3, maxiter=3000), 1e-6)):
+        solver = nk.StressBalanceSolver(linear_iteration_control=control, picard_iteration_control=nk.FixedIterations(1),
+                                        preconditioner=preconditioner)
+        out = []
+        for cls in (gpu_cls, oracle_cls):
+            P = cls(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                                              stress_balance=nk.DepthIntegrated(side_walls=nk.NoSlipWalls()), velocity_solver=solver))
+            for n, a in (("H", H), ("bed", 10.0), ("C", 1e9), ("A", 3e-24)):
+                P.set(n, a)
+            P.compute_geometry()
+            st = P.picard_solve()
+            out.append((P.get("u"), P.get("v"), st.linear_iterations_total, st.status))
+            P.close()
+        assert out[0][2:] == out[1][2:]
+        for g, w in zip(out[0][:2], out[1][:2]):
+            assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
+
+
 # Axes of unequal spacing: at a wall the face spacing (the edge cell's own width) is not that of the next face, and with
 # no-slip walls the corners on the wall enter the rows beside it.  Ten steps against the oracle's as above (1e-12), and an
 # FP32 V-cycle against its FP64 one (1e-4).
