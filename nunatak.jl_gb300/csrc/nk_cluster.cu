@@ -42,6 +42,8 @@ constexpr size_t CLUSTER_SMEM_LIMIT = 200 * 1024;
 
 constexpr int CLUSTER_MAX_ROWS = 1000;           // (j magic) >> 20 divides exactly while j * rows < 2^20
 
+constexpr int CLUSTER_MAX_HALO = 8;
+
 // Cells a thread may own.  A cell's stencil, right-hand side and iterate take 26 registers in FP32 and 52 in FP64, of
 // the 128 a thread has; four cells in FP32 spilled (1360 bytes) and were slower than leaving the level to the grid.
 template <typename T>
@@ -232,6 +234,96 @@ __device__ __forceinline__ void restriction_axis(int I, int Nc, int Nf, bool per
     }
 }
 
+// The sweeps of the coarsest level with `halo` rows of the neighbours swept along, one cell a thread: the rows that are right
+// shrink by one a sweep on either side, and only when a CTA's own are next does it take the halo anew, for one cluster
+// barrier in `halo` sweeps instead of one a sweep (894 cycles a sweep, 700 of them the barrier): a CG step of 128 x 64 mixed
+47.2 -> 43.8 us, of 320 x 160 DIVA 72.6 -> 70.7, of 1024 x 512 156.5 -> 153.5.  As many rows as one cell a thread allows, up
+to 8 (the next would save a barrier in 72 sweeps).  `c` are the CTA's own cells
+// with w b in place; their iterate goes to c.x and, masked, to the level's first buffer.  FP32 only: the rows that
+// several CTAs sweep would be paid for on the FP64 pipe.
+template <typename T, int CPT>
+__device__ __forceinline__ void coarsest_window(cg::cluster_group& cl, typename Vec2<T>::type* sm, const ClusterLevels<T>& C,
+                                                const ClusterLevel<T>& K, ClusterCells<T, CPT>& c, int rank) {
+    using V2 = typename Vec2<T>::type;
+    using V4 = typename Vec4<T>::type;
+    const int Nx = K.Nx, halo = C.halo, own = K.cnt * Nx, share = K.rows * Nx, size = (K.rows + 2 * halo + 2) * K.W;
+    V2* const shared_rows = sm + C.window;            // the own rows as the neighbours read them, twice
+    V2* const x0 = shared_rows + 2 * share;
+    const int tid = threadIdx.x;
+    if (tid < own) shared_rows[tid] = c.bw[0];        // (share >= own: one cell a thread)
+    int lo = K.j0 - halo, hi = K.j0 + K.cnt + halo;
+    if (!K.py) { lo = lo < 0 ? 0 : lo; hi = hi > K.Ny ? K.Ny : hi; }
+    if (K.cnt == 0) hi = lo;
+    const int row = tid / Nx, i = tid - row * Nx, jw = lo + row;
+    const bool in = jw < hi;
+    int j = jw % K.Ny;
+    if (j < 0) j += K.Ny;
+    const int far = jw < K.j0 ? K.j0 - jw : (jw >= K.j0 + K.cnt ? jw - (K.j0 + K.cnt - 1) : 0);   // rows from the own ones
+    ClusterCells<T, 1> z;
+    z.p[0] = (row + 1) * K.W + i + 1;
+    z.flags[0] = 0;
+    int from = 0;
+    if (in) {
+        const uint8_t m = __ldg(K.mask + j * K.pitch + i);
+        const int plane = Nx * K.Ny;
+        const V4* st = K.st + j * Nx + i;
+        const V4 a = st[0], b = st[plane], f = st[2 * plane], h = st[3 * plane], o = st[4 * plane];
+        T *u = z.u[0], *v = z.v[0];
+        u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w; u[4] = b.x; u[5] = b.y; u[6] = b.z; u[7] = b.w; u[8] = o.x;
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; v[4] = h.x; v[5] = h.y; v[6] = h.z; v[7] = h.w; v[8] = o.y;
+        z.flags[0] = ((m & U_INACTIVE) ? 0u : CELL_U) | ((m & V_INACTIVE) ? 0u : CELL_V);
+        from = K.owner(j);
+    }
+    const int at = (j - from * K.rows) * Nx + i;      // the cell in its CTA's shared_rows
+    auto put = [&](int buf) {
+        V2 *b = x0 + buf * size + z.p[0], m = cluster_masked<T, 1>(z, 0, z.x[0]);
+        b[0] = m;
+        if (K.px && i == 0) b[Nx] = m;
+        if (K.px && i == Nx - 1) b[-Nx] = m;
+    };
+    cl.sync();
+    if (in) {                                         // the first sweep from zero: x = w b
+        z.bw[0] = z.x[0] = cl.map_shared_rank(shared_rows, from)[at];
+        put(0);
+    }
+    __syncthreads();
+    int cur = 0, depth = halo, turn = 1;
+    for (int s = 1; s < C.coarsest; ++s) {
+        if (depth == 0) {
+            V2* const rows = shared_rows + turn * share;   // the other one may still be read
+            if (in && far == 0) rows[at] = z.x[0];
+            cl.sync();
+            if (in && far > 0) {
+                z.x[0] = cl.map_shared_rank(rows, from)[at];
+                put(cur);
+            }
+            __syncthreads();
+            turn ^= 1;
+            depth = halo;
+        }
+        --depth;
+        if (in && far <= depth) {
+            const V2 d = cluster_delta<T, 1>(K, z, 0, x0 + cur * size);
+            z.x[0].x += d.x;
+            z.x[0].y += d.y;
+            put(cur ^ 1);
+        }
+        __syncthreads();
+        cur ^= 1;
+    }
+    V2* const result = shared_rows + turn * share;    // the one that no CTA reads any more
+    if (in && far == 0) {
+        result[at] = z.x[0];
+        const V2 m = cluster_masked<T, 1>(z, 0, z.x[0]);
+        V2* b = sm + K.off + (jw - K.j0 + 1) * K.W + i + 1;
+        b[0] = m;
+        if (K.px && i == 0) b[Nx] = m;
+        if (K.px && i == Nx - 1) b[-Nx] = m;
+    }
+    cl.sync();
+    if (tid < own) c.x[0] = result[tid];
+}
+
 template <typename T, int CPT>
 __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __grid_constant__ ClusterLevels<T> C, const int* done, CGDot dot) {
     long long d;
@@ -262,6 +354,11 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
     for (int l = 0;; ++l) {
         const int buf0 = K.off, buf1 = K.off + K.size;
         const int ns = l == last ? C.coarsest : C.sweeps;
+        if constexpr (sizeof(T) == 4)
+            if (l == last && C.halo) {
+                coarsest_window<T, CPT>(cl, sm, C, K, c, rank);
+                break;
+            }
 #pragma unroll
         for (int k = 0; k < CPT; ++k)   // the first sweep from zero: x = w b
             if (c.p[k] >= 0) {
@@ -328,7 +425,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
         K = N;
     }
     // up: the coarser level's iterate is in the buffer its last sweep wrote
-    int coarse_buf = K.off + (((C.coarsest - 1) & 1) ? K.size : 0);
+    int coarse_buf = K.off + (!C.halo && ((C.coarsest - 1) & 1) ? K.size : 0);
     for (int l = last - 1; l >= 0; --l) {
         ClusterLevel<T> N = cluster_level(C, l, rank, d);
         cluster_setup<T, CPT>(N, c, w);
@@ -442,6 +539,17 @@ bool cluster_plan(ClusterLevels<T>& C) {
         C.off[l] = (int)off;
         off += 2ll * (rows + 2) * (g.Nx + 2);
         if (off * (long long)sizeof(typename Vec2<T>::type) > (long long)CLUSTER_SMEM_LIMIT) return false;
+    }
+    C.halo = 0;
+    if constexpr (sizeof(T) == 4) {
+        const DevGrid<T>& g = C.lv[C.n - 1].o.g;
+        const int rows = C.rows[C.n - 1], fit = (CLUSTER_THREADS / g.Nx - rows) / 2, halo = fit < CLUSTER_MAX_HALO ? fit : CLUSTER_MAX_HALO;
+        const long long window = off + 2ll * rows * g.Nx + 2ll * (rows + 2 * halo + 2) * (g.Nx + 2);
+        if (C.ctas > 1 && halo >= 2 && C.coarsest >= 4 && window * (long long)sizeof(typename Vec2<T>::type) <= (long long)CLUSTER_SMEM_LIMIT) {
+            C.halo = halo;
+            C.window = (int)off;
+            off = window;
+        }
     }
     C.total = (int)off;
     return true;

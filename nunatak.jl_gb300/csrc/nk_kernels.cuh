@@ -463,11 +463,12 @@ struct ClusterLevels {
     unsigned magic[MAX_COARSE_LEVELS];                     // j / rows by multiplication
     int n, sweeps, coarsest;                               // levels, smoothing_sweeps, coarsest_sweeps
     int ctas, cells, total;                                // cluster size, cells per thread (1, 2), pairs of shared memory
+    int halo, window;                                      // the coarsest level's halo rows (0: one, exchanged every sweep) and buffers
 };
 // Cells of the largest level that a cluster holds: 16 CTAs x 512 threads x 2 cells in FP32 (1 cell in FP64)
 constexpr long long cluster_limit_cells(bool fp64) { return fp64 ? 8192 : 16384; }
 template <typename T>
-bool cluster_plan(ClusterLevels<T>& C);   // fills rows, off, ctas, cells and total; false if the levels do not fit
+bool cluster_plan(ClusterLevels<T>& C);   // fills rows, off, ctas, cells, total, halo and window; false if the levels do not fit
 template <typename T>
 void launch_coarse_cluster(const ClusterLevels<T>& C, const int* done, const CGDot* dot, cudaStream_t s);
 void configure_coarse_cluster();

@@ -90,6 +90,39 @@ def test_coarse_levels_in_a_cluster(oracle_cls, gpu_cls, nx, ny, topology, sweep
         assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
 
 
+# The coarsest level's sweeps with several halo rows (FP32, clusters of more than one CTA): sweep counts that end on an
+# exchange, one after it and before the first, windows that wrap round a periodic axis and that reach both walls, CTAs
+# without rows, no finer level.  Tolerance as above.
+@gpu
+@pytest.mark.parametrize("coarsest", [4, 9, 17, 20])
+@pytest.mark.parametrize("nx, ny, topology, minimum", [
+    (64, 64, ("Periodic", "Periodic"), 16),
+    (160, 80, ("Bounded", "Bounded"), 20),
+    (64, 48, ("Bounded", "Periodic"), 3),
+    (60, 44, ("Periodic", "Bounded"), 44),
+])
+def test_coarsest_sweeps_with_a_halo(oracle_cls, gpu_cls, nx, ny, topology, minimum, coarsest):
+    rng = np.random.default_rng(nx + ny)
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 1.5e3), topology=topology)
+    mg = nk.StressBalanceMultigridPreconditioner(coarsest_sweeps=coarsest, minimum_coarse_size=minimum)
+    H = np.clip(1000.0 + 400.0 * rng.standard_normal((ny, nx)), 0.0, None)
+    H[:, : nx // 8] = 0.0
+    ru, rv = 1e10 * rng.standard_normal((ny, grid.face_count(0))), 1e10 * rng.standard_normal((grid.face_count(1), nx))
+    z = []
+    for cls, precision in ((gpu_cls, "mixed"), (oracle_cls, "fp64")):
+        P = cls(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                                          stress_balance=nk.DepthIntegrated(side_walls=nk.NoSlipWalls()),
+                                          velocity_solver=nk.StressBalanceSolver(preconditioner=mg, precision=precision)))
+        for n, a in (("H", H), ("bed", 10.0), ("C", 1e9), ("A", 3e-24)):
+            P.set(n, a)
+        P.compute_geometry()
+        P.update_coefficients()
+        z.append([a[:ny, :nx] for a in P.precondition(ru, rv)])
+        P.close()
+    for g, w in zip(*z):
+        assert np.max(np.abs(g - w)) <= 1e-4 * np.max(np.abs(w))
+
+
 # One pass down and one up a level (FP32 levels above the cluster's 16384 cells, two sweeps, both axes halved): widths at
 # and beside multiples of the 26 and 28 columns that a warp writes, rows that do not divide by a walk, one and two such
 # levels, periodic seams, faces that are not square, walls with shear, ice-free cells.  Tolerance as above.
