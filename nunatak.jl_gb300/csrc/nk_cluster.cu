@@ -237,8 +237,8 @@ __device__ __forceinline__ void restriction_axis(int I, int Nc, int Nf, bool per
 // The sweeps of the coarsest level with `halo` rows of the neighbours swept along, one cell a thread: the rows that are right
 // shrink by one a sweep on either side, and only when a CTA's own are next does it take the halo anew, for one cluster
 // barrier in `halo` sweeps instead of one a sweep (894 cycles a sweep, 700 of them the barrier): a CG step of 128 x 64 mixed
-47.2 -> 43.8 us, of 320 x 160 DIVA 72.6 -> 70.7, of 1024 x 512 156.5 -> 153.5.  As many rows as one cell a thread allows, up
-to 8 (the next would save a barrier in 72 sweeps).  `c` are the CTA's own cells
+// 47.2 -> 43.8 us, of 320 x 160 DIVA 72.6 -> 70.7, of 1024 x 512 156.5 -> 153.5.  As many rows as one cell a thread allows, up
+// to 8 (the next would save a barrier in 72 sweeps).  `c` are the CTA's own cells
 // with w b in place; their iterate goes to c.x and, masked, to the level's first buffer.  FP32 only: the rows that
 // several CTAs sweep would be paid for on the FP64 pipe.
 template <typename T, int CPT>
