@@ -3,9 +3,8 @@
 //
 // One nk_problem owns one device arena (a single cudaMalloc) holding every field, coefficient record,
 // solver vector and multigrid level of its grid, and one CUDA stream on which every call is ordered.
-// Conjugate gradients run without host synchronisation inside a solve: the host issues steps in
-// batches and reads the device stopping flag once per batch.  Picard reads two device norms per
-// iteration.
+// A solve is one CUDA graph whose loops the device controls; in the host loop (NK_SOLVER_HOST_LOOP) the host
+// issues steps in batches and reads the device stopping flag once per batch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -41,10 +40,10 @@ struct Failure {
 
 static void bad(const std::string& m) { throw Failure{NK_BAD_ARGUMENT, m}; }
 
-// Rows per warp of the column-marching kernels: NK_STRIP_ROWS (1, 2, 4 or 8) when set, else 2 for FP32
-// (56 registers: the memory-bound sweeps want occupancy; the 2048x1024 sweep takes 36.9 us against 41.6 us at 4
-// rows, and the serving stream is unchanged) and, for FP64, 4 from 2^18 cells (the FP64 kernels are bound by
-// the FP64 pipe; the two extra rows of each walk are a smaller share at 4).
+// Rows per warp of the unrolled walks (multigrid sweeps and residuals that the one-pass kernels and the cluster do not
+// take): NK_STRIP_ROWS (1, 2, 4 or 8) when set, else 2 for FP32 (56 registers: the memory-bound sweeps want occupancy; the
+// 2048x1024 sweep takes 36.9 us against 41.6 us at 4 rows, and the serving stream is unchanged) and strip_rows' sizes for
+// FP64.  The FP64 operator kernels roll (operator_shape) and take from here only a forced length.
 // Walk lengths measured by the strip autotuner, per (kernel kind, Nx, Ny, element bytes), shared by every
 // problem of the process.
 static std::mutex& tuned_mutex() {
@@ -71,8 +70,8 @@ int strip_rows(int nx, int ny, int elem_bytes, int kind) {
     }
     long long cells = (long long)nx * ny;
     // FP64 multigrid sweeps and residuals: what the autotuner measured for one solve at a time on GB300 (one row
-    // below 2^16 cells, two above; 1.48 -> 1.68 solves/s on the FP64 stream); FP32 and the FP64 operator kernels
-    // keep two rows (four from 2^18 cells for the operator), which the concurrent mixed stream prefers
+    // below 2^16 cells, two above; 1.48 -> 1.68 solves/s on the FP64 stream); FP32 keeps two rows, which the
+    // concurrent mixed stream prefers
     if (elem_bytes == 8 && kind != STRIP_OPERATOR) return cells < (1 << 16) ? 1 : 2;
     return 2;
 }
@@ -664,9 +663,10 @@ static void smooth(nk_problem* P, Level<T>& L, int sweeps, bool first, const int
     }
 }
 
-// v_cycle!, multigrid_preconditioner.jl:144-163 (x ≈ A⁻¹ b from a zero guess on level l).  Levels from
-// `fused_level` down run in one k_coarse_vcycle launch; above it each phase is one grid-wide kernel, and the
-// restriction also performs the coarse level's first sweep from zero.  `dot`: the last kernel also takes the r.z of the
+// v_cycle!, multigrid_preconditioner.jl:144-163 (x ≈ A⁻¹ b from a zero guess on level l).  The levels that fit
+// run in one cluster (plan_cluster); above them an FP32 level with the default settings takes one pass down and one up
+// (nk_vcycle.cu), and any other level one grid-wide kernel a phase, its restriction also performing the coarse level's
+// first sweep from zero.  (Levels from `fused_level` down run in one block instead where NK_COARSE_CELLS asks for it.)  `dot`: the last kernel also takes the r.z of the
 // conjugate-gradient step where it can; returns whether it did.
 template <typename T>
 static bool v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* done, bool first_done = false, const CGDot* dot = nullptr) {

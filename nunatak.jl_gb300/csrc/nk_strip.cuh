@@ -33,7 +33,7 @@ inline LaunchDims strip_dims(int nx, int ny, int rows) {
 // amortise the two priming rows on large grids; short ones keep enough warps in flight on small grids.
 // `kind` names the kernel: the multigrid sweeps and residuals write one value per cell with no reduction, so
 // their walk length cannot change a bit of the result and is taken from the autotuner's table when it has an
-// entry (nk_problem.cu); the FP64 operator kernels carry block reductions and keep the fixed rule.
+// entry (nk_problem.cu); the FP64 operator kernels roll (operator_shape) and take only a length forced by NK_STRIP_ROWS.
 enum StripKernel { STRIP_OPERATOR = 0, STRIP_SMOOTH = 1, STRIP_RESIDUAL = 2 };
 int strip_rows(int nx, int ny, int elem_bytes, int kind = STRIP_OPERATOR);
 

@@ -1,16 +1,17 @@
 // nk_time_adjoint.cu — the reverse of one thickness stage, for the gradient through time steps.
 //
-// The forward stage (k_thickness_faces, k_thickness_limiter, k_thickness_stage in nk_coefficients.cu) is
+// The forward stage (k_thickness_faces and k_thickness_stage in nk_coefficients.cu) is
 //   H = max(0, H⁻ + Δτ (S - ∇⋅F(Hs, u))),  S = a - (1 - φ(Hs)) w m  on full cells,
 // with F the face fluxes u H_face, H_face the scheme's upwind-biased reconstruction of Hs, limited for a bounded
-// WENO by the upwind cell's θ (H̄ + θ (H_face - H̄)).  Its reverse runs as four gathers, each thread owning one cell or
+// WENO by the upwind cell's θ (H̄ + θ (H_face - H̄)).  Its reverse runs as gathers, each thread owning one cell or
 // one face, so no two threads add into one value and the result does not depend on the order of the launch:
 //   cells    the clip, the sources and the divergence: λ★ = [H > 0] λ, λH⁻ += λ★, λa += Δτ λ★, λm -= Δτ λ★ (1 - φ) w;
 //   faces    λF = λ of each face flux, from the divergence of its two cells, and λu += Δy H_face λF;
 //   limiter  per cell, the faces it is upwind of: λHs += (1 - θ) Δy u λF, λθ += (H_face - H̄) Δy u λF, then θ's own
 //            derivative back to H̄ and to the cell's four reconstructions;
-//   stencils per cell, every reconstruction whose stencil holds it (∂H_face/∂s by face_value_gradient) and every
-//            centre grounded fraction that reads its flotation.
+//   recon    per cell, the derivatives of its own reconstructions and of its own grounded fraction, to scratch planes;
+//   stencils per cell, what every reconstruction whose stencil holds it and every centre grounded fraction that reads
+//            its flotation left there for it.
 // Wherever the forward takes a min, a max or a clip, the reverse follows the branch the forward took.
 #include <cmath>
 
@@ -152,7 +153,7 @@ __global__ void k_stage_adjoint_limiter(StageAdjointView a) {
     }
     double2 lwx = make_double2(0.0, 0.0), lwy = make_double2(0.0, 0.0);
     if (bounded && lt != 0.0) {
-        // θ = min(1, |(upper - H̄) / (M - H̄ + ε)|, |(lower - H̄) / (m - H̄ - ε)|) of k_thickness_limiter
+        // θ = min(1, |(upper - H̄) / (M - H̄ + ε)|, |(lower - H̄) / (m - H̄ - ε)|) of the forward limiter
         double E = v.fx[g.idx(i + 1, j)].x, W = v.fx[g.idx(i, j)].y;
         double N = v.fy[g.idx(i, j + 1)].x, S = v.fy[g.idx(i, j)].y;
         const double w = 5.0 / 18, eps = 2 * 2.220446049250313e-16, r12 = 1 / (1 - 2 * w);
