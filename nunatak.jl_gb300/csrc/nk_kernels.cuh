@@ -449,6 +449,8 @@ template <typename T>
 void launch_coarse_vcycle(const CoarseLevels<T>& C, const int* done, cudaStream_t s);
 // One half of a V-cycle's visit to a level in one pass (nk_vcycle.cu; two sweeps each way, both axes halved).  Down:
 // x2 = two sweeps from zero on L.b, C.b = R (L.b - A x2).  Up: xout = two sweeps on x2 + P xc.
+// Its walks ask for rows -3 .. Ny + 4 and wrap them once, which needs five rows of a periodic axis.
+constexpr bool vcycle_rows_wrap_once(int Ny, int periodic) { return !periodic || Ny >= 5; }
 template <typename T>
 void launch_vcycle_down(const LevelView<T>& L, const LevelView<T>& C, typename Vec2<T>::type* x2, const int* done, cudaStream_t s);
 template <typename T>

@@ -697,7 +697,8 @@ static bool v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* 
         // FP32, the default two point sweeps and both axes halved: one pass down and one up (nk_vcycle.cu).  In FP64 the
         // rows and columns that neighbouring walks share would cost the FP64 pipe more than the launches they save.
         Level<T>& N = lv[l + 1];
-        if (!first_done && P->sd.smoother == NK_SMOOTHER_POINT_JACOBI && P->sd.smoothing_sweeps == 2 && N.cx == 2 && N.cy == 2 && l + 1 != lc) {
+        if (!first_done && P->sd.smoother == NK_SMOOTHER_POINT_JACOBI && P->sd.smoothing_sweeps == 2 && N.cx == 2 && N.cy == 2 && l + 1 != lc &&
+            vcycle_rows_wrap_once(L.Ny, P->py)) {
             LevelView<T> f = P->level_view(L), c = P->level_view(N);
             launch_vcycle_down<T>(f, c, L.x2, done, s);
             v_cycle(P, lv, l + 1, done);

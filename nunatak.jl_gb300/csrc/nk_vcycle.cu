@@ -40,7 +40,7 @@ struct LevelColumn {
         wall_x = !g.px && (i <= 0 || i >= g.Nx) ? L.o.wall_factor : T(1);
         au = av = g.h * g.h;
     }
-    __device__ __forceinline__ int row(int j) const {   // the stored row of j
+    __device__ __forceinline__ int row(int j) const {   // the stored row of j (vcycle_rows_wrap_once)
         const DevGrid<T>& g = L.o.g;
         if (g.py) return j < 0 ? j + g.Ny : (j >= g.Ny ? j - g.Ny : j);
         return j < 0 ? 0 : (j > g.Ny ? g.Ny : j);
