@@ -8,18 +8,42 @@ import nunatak_gb300 as nk
 gpu = pytest.mark.gpu
 
 
-def sheet(cls, grid, solver, H):
+def sheet(cls, grid, solver, H, u_prescribed=None):
     """An SSA sheet with no-slip walls after its first coefficient update."""
     P = cls(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
                                       stress_balance=nk.DepthIntegrated(side_walls=nk.NoSlipWalls()), velocity_solver=solver))
     for n, a in (("H", H), ("bed", 10.0), ("C", 1e9), ("A", 3e-24)):
         P.set(n, a)
+    if u_prescribed is not None:
+        P.set("u_prescribed", u_prescribed)
     P.compute_geometry()
     r = np.random.default_rng(2)
     P.set("u", 1e-5 * r.standard_normal(P.shape("u")))
     P.set("v", 1e-5 * r.standard_normal(P.shape("v")))
     P.update_coefficients()
     return P
+
+
+def residual(grid, seed):
+    rng = np.random.default_rng(seed)
+    return 1e10 * rng.standard_normal((grid.Ny, grid.face_count(0))), 1e10 * rng.standard_normal((grid.face_count(1), grid.Nx))
+
+
+def assert_close(got, want, r, tol):
+    """V-cycles of r: `tol` of the largest entry on the rows that couple, and r itself on the identity rows (walls and ice-free
+    faces), whose entries are 1e19 times those and would hide them in one norm."""
+    assert tol < 1e-3
+    for g, w, b in zip(got, want, r):
+        ny, nx = min(g.shape[0], b.shape[0]), min(g.shape[1], b.shape[1])
+        g, w, b = g[:ny, :nx], w[:ny, :nx], b[:ny, :nx]
+        identity = np.abs(w - b) <= 1e-7 * np.abs(b)   # (b rounded to FP32 in a mixed V-cycle)
+        assert np.all(np.abs(g - b)[identity] <= 1e-7 * np.abs(b)[identity])
+        assert np.max(np.abs(w[~identity])) < 1e-6 * np.max(np.abs(b))   # no identity row is left among them
+        assert np.max(np.abs(g - w)[~identity]) <= tol * np.max(np.abs(w[~identity]))
+
+
+def interior(grid, z):
+    return [a[:grid.Ny, :grid.Nx] for a in z]
 
 
 # A flowline of two, four and six rows round a periodic axis, too wide for the cluster: the one-pass kernels' walks ask for
@@ -32,13 +56,66 @@ def test_one_pass_levels_on_a_short_periodic_axis(oracle_cls, gpu_cls, nx, ny):
     grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 2e3), topology=("Bounded", "Periodic"), halo=(1, 1))
     H = np.clip(1000.0 + 400.0 * rng.standard_normal((ny, nx)), 0.0, None)
     H[:, : nx // 8] = 0.0
-    ru, rv = 1e10 * rng.standard_normal((ny, grid.face_count(0))), 1e10 * rng.standard_normal((grid.face_count(1), nx))
+    r = residual(grid, nx)
     z = []
     for cls, precision in ((gpu_cls, "mixed"), (oracle_cls, "fp64")):
         mg = nk.StressBalanceMultigridPreconditioner(minimum_coarse_size=1)
         P = sheet(cls, grid, nk.StressBalanceSolver(preconditioner=mg, precision=precision), H)
-        z.append(P.precondition(ru, rv))
+        z.append(interior(grid, P.precondition(*r)))
         P.close()
-    for g, w in zip(*z):
-        g, w = g[:ny, :nx], w[:ny, :nx]
-        assert np.max(np.abs(g - w)) <= 1e-4 * np.max(np.abs(w))
+    assert_close(z[0], z[1], interior(grid, r), 1e-4)
+
+
+# One V-cycle against the oracle's: FP64 to 1e-12 and FP32 to 1e-4 of the largest entry on the rows that couple (rounding of
+# 1e-16 and 6e-8 of rowsum |x| in each of its ~50 sweeps).  Faces: None for equal spacing, else the range of the cell widths.
+def vcycles(gpu_cls, oracle_cls, grid, mg, precision, tol, seed):
+    nx, ny = grid.Nx, grid.Ny
+    H = np.clip(1000.0 + 400.0 * np.random.default_rng(seed).standard_normal((ny, nx)), 0.0, None)
+    H[:, : nx // 8] = 0.0   # ice free: identity rows
+    H[ny // 2, : nx // 2] = 0.0
+    r = residual(grid, seed)
+    z = []
+    for cls, p in ((gpu_cls, precision), (oracle_cls, "fp64")):
+        P = sheet(cls, grid, nk.StressBalanceSolver(preconditioner=mg, precision=p), H)
+        z.append(interior(grid, P.precondition(*r)))
+        P.close()
+    assert_close(z[0], z[1], interior(grid, r), tol)
+
+
+PRECISIONS = pytest.mark.parametrize("precision, tol", [("fp64", 1e-12), ("mixed", 1e-4)])
+BB, PB, BP, PP = ("Bounded", "Bounded"), ("Periodic", "Bounded"), ("Bounded", "Periodic"), ("Periodic", "Periodic")
+
+
+# The coarse levels' cluster: one CTA and many, rows that do not divide by the CTAs, CTAs without rows, axes that stop
+# halving before the other, seams inside and across CTAs, odd and even sweep counts, no coarse level, FP64's largest grid
+# (8192 cells) and FP32's (16384) and one row beyond, coarsest sweeps that end on, after and before an exchange of halos.
+@gpu
+@PRECISIONS
+@pytest.mark.parametrize("nx, ny, topology, sweeps, coarsest, minimum", [
+    (16, 16, BB, 2, 20, 4), (64, 34, BB, 2, 20, 16), (96, 40, PB, 1, 7, 2), (40, 96, BP, 3, 6, 4), (72, 48, PP, 2, 1, 3),
+    (75, 45, BB, 2, 20, 4), (512, 16, BB, 2, 5, 8), (128, 64, PB, 2, 20, 8), (128, 128, BB, 2, 20, 32), (128, 130, BB, 2, 20, 32),
+    (64, 64, PP, 2, 4, 16), (64, 64, PP, 2, 9, 16), (160, 80, BB, 2, 17, 20), (64, 48, BP, 2, 9, 3), (60, 44, PB, 2, 20, 44),
+])
+def test_vcycle_in_a_cluster(oracle_cls, gpu_cls, nx, ny, topology, sweeps, coarsest, minimum, precision, tol):
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 1.5e3), topology=topology)
+    mg = nk.StressBalanceMultigridPreconditioner(smoothing_sweeps=sweeps, coarsest_sweeps=coarsest, minimum_coarse_size=minimum)
+    vcycles(gpu_cls, oracle_cls, grid, mg, precision, tol, nx + ny)
+
+
+# The one-pass levels (FP32) and the grid-wide ones (FP64): widths at and beside multiples of the 26 and 28 columns of a
+# warp, rows that do not divide by a walk, one and two such levels, seams, cells that are not square, unequal spacing
+# with each pair of boundaries.
+@gpu
+@PRECISIONS
+@pytest.mark.parametrize("nx, ny, topology, stretch", [
+    (260, 66, BB, 1.0), (280, 62, PB, 1.0), (262, 90, BP, 1.5), (150, 130, PP, 1.0), (364, 210, BB, 0.7), (416, 224, BB, 1.0),
+    (160, 150, BB, None), (160, 150, PP, None), (160, 150, PB, None), (160, 150, BP, None),
+])
+def test_vcycle_above_the_cluster(oracle_cls, gpu_cls, nx, ny, topology, stretch, precision, tol):
+    if stretch is None:
+        rng = np.random.default_rng(nx)
+        x, y = (np.concatenate([[0.0], np.cumsum(rng.uniform(1e3, 3e3, n))]).tolist() for n in (nx, ny))
+    else:
+        x, y = (0.0, nx * 2e3), (0.0, ny * 2e3 * stretch)
+    grid = nk.RectilinearGrid(size=(nx, ny), x=x, y=y, topology=topology)
+    vcycles(gpu_cls, oracle_cls, grid, nk.StressBalanceMultigridPreconditioner(minimum_coarse_size=20), precision, tol, nx + ny)
