@@ -12,10 +12,10 @@
 // prolongation read the other level's rows wherever they live.
 //
 // Arithmetic.  A sweep is x' = x + w (b - A x) with w = 1 / rowsum.  A row of A couples five points of its own component
-// and four of the other, and its nine coefficients change only with the coefficients, so -w A is formed once per solve
-// (k_inverse_row_sum, nk_solver.cu) and a sweep costs eighteen multiply-adds a cell.  (The grid-wide kernels difference the
+// and four of the other, and its nine coefficients change only with the coefficients, so -A is formed once per solve
+// (k_inverse_row_sum, nk_solver.cu) and a sweep costs twenty multiply-adds a cell.  (The grid-wide kernels difference the
 // neighbours before they multiply; against the sum of products that only moves the rounding, by the size of the rounding
-// of x' itself.)  The residual is the same expression over w.
+// of x' itself.)  The residual is the sweep's own b - A x: a prescribed row, whose w is zero, keeps its b in it.
 //
 // What binds it: latency, a sweep being seven shared loads, the multiply-adds and one cluster barrier.  Split: sixteen
 // CTAs of 512 threads with one cell a thread where the level allows beat eight CTAs (128 x 64 solve 66.8 against 70.5 us a CG iteration, 320 x 160 DIVA 109.9
@@ -92,12 +92,12 @@ __device__ __forceinline__ ClusterLevel<T> cluster_level(const ClusterLevels<T>&
     return K;
 }
 
-// A thread's cells of one level: the iterate, w b and the rows of -w A (E, W, N, S, centre of the own component; centre
+// A thread's cells of one level: the iterate, b, w and the rows of -A (E, W, N, S, centre of the own component; centre
 // and three neighbours of the other), so that a sweep is a chain of multiply-adds.
 template <typename T, int CPT>
 struct ClusterCells {
     using V2 = typename Vec2<T>::type;
-    V2 x[CPT], bw[CPT];
+    V2 x[CPT], b[CPT], w[CPT];
     T u[CPT][9], v[CPT][9];
     int p[CPT];                // index in a buffer, -1 for no cell
     unsigned flags[CPT];
@@ -111,9 +111,9 @@ constexpr int CELL_COL = 8;                           // the column index starts
 template <typename T, int CPT>
 __device__ __forceinline__ int cell_i(const ClusterCells<T, CPT>& c, int k) { return (int)(c.flags[k] >> CELL_COL); }
 
-// The cells' places and stencil rows; w[k] = 1 / rowsum.
+// The cells' places, stencil rows and weights w = 1 / rowsum.
 template <typename T, int CPT>
-__device__ __forceinline__ void cluster_setup(const ClusterLevel<T>& K, ClusterCells<T, CPT>& c, typename Vec2<T>::type* w) {
+__device__ __forceinline__ void cluster_setup(const ClusterLevel<T>& K, ClusterCells<T, CPT>& c) {
     using V4 = typename Vec4<T>::type;
     const int n = K.cnt * K.Nx, plane = K.Nx * K.Ny;
 #pragma unroll
@@ -131,40 +131,42 @@ __device__ __forceinline__ void cluster_setup(const ClusterLevel<T>& K, ClusterC
         T* v = c.v[k];
         u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w; u[4] = b.x; u[5] = b.y; u[6] = b.z; u[7] = b.w; u[8] = o.x;
         v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; v[4] = h.x; v[5] = h.y; v[6] = h.z; v[7] = h.w; v[8] = o.y;
-        w[k].x = o.z;
-        w[k].y = o.w;
+        c.w[k].x = o.z;
+        c.w[k].y = o.w;
         c.flags[k] = ((m & U_INACTIVE) ? 0u : CELL_U) | ((m & V_INACTIVE) ? 0u : CELL_V) | ((K.px && i == 0) ? CELL_WEST : 0u) |
                      ((K.px && i == K.Nx - 1) ? CELL_EAST : 0u) | ((jl == 0 && K.south >= 0) ? CELL_SOUTH : 0u) |
                      ((jl == K.cnt - 1 && K.north >= 0) ? CELL_NORTH : 0u) | ((m & U_IDENTITY) ? CELL_IU : 0u) |
                      ((m & V_IDENTITY) ? CELL_IV : 0u) | ((unsigned)i << CELL_COL);
     }
 }
-// 1 / rowsum of cell k (the residual's divisor)
+// b - A x of cell k from the masked iterate in `in`
 template <typename T, int CPT>
-__device__ __forceinline__ typename Vec2<T>::type cluster_weight(const ClusterLevel<T>& K, int k) {
-    auto o = K.st[4 * K.Nx * K.Ny + K.j0 * K.Nx + (int)threadIdx.x + k * CLUSTER_THREADS];
-    typename Vec2<T>::type w;
-    w.x = o.z;
-    w.y = o.w;
-    return w;
-}
-
-// w (b - A x) of cell k from the masked iterate in `in`
-template <typename T, int CPT>
-__device__ __forceinline__ typename Vec2<T>::type cluster_delta(const ClusterLevel<T>& K, const ClusterCells<T, CPT>& c, int k,
-                                                                const typename Vec2<T>::type* in) {
+__device__ __forceinline__ typename Vec2<T>::type cluster_residual(const ClusterLevel<T>& K, const ClusterCells<T, CPT>& c, int k,
+                                                                   const typename Vec2<T>::type* in) {
     using V2 = typename Vec2<T>::type;
     const V2* q = in + c.p[k];
     V2 E = q[1], Wt = q[-1], N = q[K.W], S = q[-K.W], NW = q[K.W - 1], SE = q[1 - K.W];
     T mu = (c.flags[k] & CELL_U) ? c.x[k].x : T(0), mv = (c.flags[k] & CELL_V) ? c.x[k].y : T(0);
     const T* u = c.u[k];
     const T* v = c.v[k];
-    T ya = c.bw[k].x + u[4] * c.x[k].x + u[0] * E.x + u[1] * Wt.x, yb = u[5] * mv + u[6] * N.y + u[7] * NW.y + u[8] * Wt.y;
-    T za = c.bw[k].y + v[4] * c.x[k].y + v[0] * N.y + v[1] * S.y, zb = v[5] * mu + v[6] * E.x + v[7] * SE.x + v[8] * S.x;
-    V2 d;
-    d.x = ya + (yb + (u[2] * N.x + u[3] * S.x));
-    d.y = za + (zb + (v[2] * E.y + v[3] * Wt.y));
-    return d;
+    T ya = c.b[k].x + u[4] * c.x[k].x + u[0] * E.x + u[1] * Wt.x, yb = u[5] * mv + u[6] * N.y + u[7] * NW.y + u[8] * Wt.y;
+    T za = c.b[k].y + v[4] * c.x[k].y + v[0] * N.y + v[1] * S.y, zb = v[5] * mu + v[6] * E.x + v[7] * SE.x + v[8] * S.x;
+    V2 r;
+    r.x = ya + (yb + (u[2] * N.x + u[3] * S.x));
+    r.y = za + (zb + (v[2] * E.y + v[3] * Wt.y));
+    return r;
+}
+// The first sweep of cell k, from zero, and a further one from the masked iterate in `in`
+template <typename T, int CPT>
+__device__ __forceinline__ void cluster_first(ClusterCells<T, CPT>& c, int k) {
+    c.x[k].x = c.w[k].x * c.b[k].x;
+    c.x[k].y = c.w[k].y * c.b[k].y;
+}
+template <typename T, int CPT>
+__device__ __forceinline__ void cluster_sweep(const ClusterLevel<T>& K, ClusterCells<T, CPT>& c, int k, const typename Vec2<T>::type* in) {
+    const auto r = cluster_residual<T, CPT>(K, c, k, in);
+    c.x[k].x += c.w[k].x * r.x;
+    c.x[k].y += c.w[k].y * r.y;
 }
 
 // Cell k's masked pair m into buffer `buf` (offset from the start of shared memory), its periodic copies, and the halo
@@ -239,7 +241,7 @@ __device__ __forceinline__ void restriction_axis(int I, int Nc, int Nf, bool per
 // barrier in `halo` sweeps instead of one a sweep (894 cycles a sweep, 700 of them the barrier): a CG step of 128 x 64 mixed
 // 47.2 -> 43.8 us, of 320 x 160 DIVA 72.6 -> 70.7, of 1024 x 512 156.5 -> 153.5.  As many rows as one cell a thread allows, up
 // to 8 (the next would save a barrier in 72 sweeps).  `c` are the CTA's own cells
-// with w b in place; their iterate goes to c.x and, masked, to the level's first buffer.  FP32 only: the rows that
+// with b in place; their iterate goes to c.x and, masked, to the level's first buffer.  FP32 only: the rows that
 // several CTAs sweep would be paid for on the FP64 pipe.
 template <typename T, int CPT>
 __device__ __forceinline__ void coarsest_window(cg::cluster_group& cl, typename Vec2<T>::type* sm, const ClusterLevels<T>& C,
@@ -250,7 +252,7 @@ __device__ __forceinline__ void coarsest_window(cg::cluster_group& cl, typename 
     V2* const shared_rows = sm + C.window;            // the own rows as the neighbours read them, twice
     V2* const x0 = shared_rows + 2 * share;
     const int tid = threadIdx.x;
-    if (tid < own) shared_rows[tid] = c.bw[0];        // (share >= own: one cell a thread)
+    if (tid < own) shared_rows[tid] = c.b[0];         // (share >= own: one cell a thread)
     int lo = K.j0 - halo, hi = K.j0 + K.cnt + halo;
     if (!K.py) { lo = lo < 0 ? 0 : lo; hi = hi > K.Ny ? K.Ny : hi; }
     if (K.cnt == 0) hi = lo;
@@ -271,6 +273,8 @@ __device__ __forceinline__ void coarsest_window(cg::cluster_group& cl, typename 
         T *u = z.u[0], *v = z.v[0];
         u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w; u[4] = b.x; u[5] = b.y; u[6] = b.z; u[7] = b.w; u[8] = o.x;
         v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; v[4] = h.x; v[5] = h.y; v[6] = h.z; v[7] = h.w; v[8] = o.y;
+        z.w[0].x = o.z;
+        z.w[0].y = o.w;
         z.flags[0] = ((m & U_INACTIVE) ? 0u : CELL_U) | ((m & V_INACTIVE) ? 0u : CELL_V);
         from = K.owner(j);
     }
@@ -283,7 +287,8 @@ __device__ __forceinline__ void coarsest_window(cg::cluster_group& cl, typename 
     };
     cl.sync();
     if (in) {                                         // the first sweep from zero: x = w b
-        z.bw[0] = z.x[0] = cl.map_shared_rank(shared_rows, from)[at];
+        z.b[0] = cl.map_shared_rank(shared_rows, from)[at];
+        cluster_first<T, 1>(z, 0);
         put(0);
     }
     __syncthreads();
@@ -303,9 +308,7 @@ __device__ __forceinline__ void coarsest_window(cg::cluster_group& cl, typename 
         }
         --depth;
         if (in && far <= depth) {
-            const V2 d = cluster_delta<T, 1>(K, z, 0, x0 + cur * size);
-            z.x[0].x += d.x;
-            z.x[0].y += d.y;
+            cluster_sweep<T, 1>(K, z, 0, x0 + cur * size);
             put(cur ^ 1);
         }
         __syncthreads();
@@ -337,16 +340,13 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
     V2* sm = reinterpret_cast<V2*>(smem_raw);
 
     ClusterCells<T, CPT> c;
-    V2 w[CPT];
     ClusterLevel<T> K = cluster_level(C, 0, rank, d);
-    cluster_setup<T, CPT>(K, c, w);
+    cluster_setup<T, CPT>(K, c);
 #pragma unroll
     for (int k = 0; k < CPT; ++k)
         if (c.p[k] >= 0) {
             const int e = (int)threadIdx.x + k * CLUSTER_THREADS, i = cell_i<T, CPT>(c, k);
-            V2 b = K.b[(K.j0 + (e - i) / K.Nx) * K.pitch + i];
-            c.bw[k].x = b.x * w[k].x;
-            c.bw[k].y = b.y * w[k].y;
+            c.b[k] = K.b[(K.j0 + (e - i) / K.Nx) * K.pitch + i];
         }
     for (int e = threadIdx.x; e < C.total; e += CLUSTER_THREADS) { V2 z; z.x = z.y = T(0); sm[e] = z; }
     cl.sync();   // the zeroed halos are in place before a neighbour writes into them
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
 #pragma unroll
         for (int k = 0; k < CPT; ++k)   // the first sweep from zero: x = w b
             if (c.p[k] >= 0) {
-                c.x[k] = c.bw[k];
+                cluster_first<T, CPT>(c, k);
                 cluster_put<T, CPT>(cl, sm, K, buf0, c, k, cluster_masked<T, CPT>(c, k, c.x[k]));
             }
         cl.sync();
@@ -372,9 +372,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
 #pragma unroll
             for (int k = 0; k < CPT; ++k)
                 if (c.p[k] >= 0) {
-                    V2 dl = cluster_delta<T, CPT>(K, c, k, sm + cur);
-                    c.x[k].x += dl.x;
-                    c.x[k].y += dl.y;
+                    cluster_sweep<T, CPT>(K, c, k, sm + cur);
                     cluster_put<T, CPT>(cl, sm, K, nxt, c, k, cluster_masked<T, CPT>(c, k, c.x[k]));
                 }
             cl.sync();
@@ -384,14 +382,9 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
         const int res = cur == buf0 ? buf1 : buf0;   // the residual takes the free buffer
 #pragma unroll
         for (int k = 0; k < CPT; ++k)
-            if (c.p[k] >= 0) {
-                V2 r = cluster_delta<T, CPT>(K, c, k, sm + cur), wk = cluster_weight<T, CPT>(K, k);
-                r.x = wk.x == T(0) ? T(0) : r.x / wk.x;
-                r.y = wk.y == T(0) ? T(0) : r.y / wk.y;
-                sm[res + c.p[k]] = cluster_masked<T, CPT>(c, k, r);
-            }
+            if (c.p[k] >= 0) sm[res + c.p[k]] = cluster_masked<T, CPT>(c, k, cluster_residual<T, CPT>(K, c, k, sm + cur));
         ClusterLevel<T> N = cluster_level(C, l + 1, rank, d);
-        cluster_setup<T, CPT>(N, c, w);
+        cluster_setup<T, CPT>(N, c);
         cl.sync();
 #pragma unroll
         for (int k = 0; k < CPT; ++k) {
@@ -419,8 +412,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
             b.x = (c.flags[k] & CELL_IU) ? T(0) : su;
             b.y = (c.flags[k] & CELL_IV) ? T(0) : sv;
             N.b[J * N.pitch + I] = b;   // read back by this thread on the way up
-            c.bw[k].x = b.x * w[k].x;
-            c.bw[k].y = b.y * w[k].y;
+            c.b[k] = b;
         }
         K = N;
     }
@@ -428,7 +420,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
     int coarse_buf = K.off + (!C.halo && ((C.coarsest - 1) & 1) ? K.size : 0);
     for (int l = last - 1; l >= 0; --l) {
         ClusterLevel<T> N = cluster_level(C, l, rank, d);
-        cluster_setup<T, CPT>(N, c, w);
+        cluster_setup<T, CPT>(N, c);
         const int down = (C.sweeps - 1) & 1;   // the buffer that holds the iterate of the way down
         int cur = N.off + (down ? 0 : N.size);
         const int old = N.off + (down ? N.size : 0);
@@ -436,12 +428,11 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
         for (int k = 0; k < CPT; ++k) {
             if (c.p[k] < 0) continue;
             const int e = (int)threadIdx.x + k * CLUSTER_THREADS, i = cell_i<T, CPT>(c, k), j = N.j0 + (e - i) / N.Nx;
-            V2 b = N.b[j * N.pitch + i], x = sm[old + c.p[k]];
-            c.bw[k].x = b.x * w[k].x;
-            c.bw[k].y = b.y * w[k].y;
+            V2 x = sm[old + c.p[k]];
+            c.b[k] = N.b[j * N.pitch + i];
             // an inactive row is an identity row: its iterate is w b after every sweep, and shared memory holds zero
-            if (!(c.flags[k] & CELL_U)) x.x = c.bw[k].x;
-            if (!(c.flags[k] & CELL_V)) x.y = c.bw[k].y;
+            if (!(c.flags[k] & CELL_U)) x.x = c.w[k].x * c.b[k].x;
+            if (!(c.flags[k] & CELL_V)) x.y = c.w[k].y * c.b[k].y;
             int fi1, fi2, ci1, ci2, fj1, fj2, cj1, cj2;   // face and centre parents of each axis
             T fa1, fa2, ca1, ca2, fb1, fb2, cb1, cb2;
             parents<T>(i, K.Nx, K.px, true, K.cx, fi1, fi2, fa1, fa2);
@@ -465,9 +456,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_coarse_cluster(const __g
 #pragma unroll
             for (int k = 0; k < CPT; ++k)
                 if (c.p[k] >= 0) {
-                    V2 dl = cluster_delta<T, CPT>(N, c, k, sm + cur);
-                    c.x[k].x += dl.x;
-                    c.x[k].y += dl.y;
+                    cluster_sweep<T, CPT>(N, c, k, sm + cur);
                     if (!out) cluster_put<T, CPT>(cl, sm, N, nxt, c, k, cluster_masked<T, CPT>(c, k, c.x[k]));
                 }
             if (!out) cl.sync();

@@ -158,7 +158,7 @@ void launch_inverse_diagonal(const OpView<double>& o, double2* invd, cudaStream_
     k_inverse_diagonal<<<d.grid, d.block, 0, s>>>(o, invd); count_launch();
 }
 
-// The rows of -w A at (i, j), w = (1/rowsum)u, (1/rowsum)v: five own-component and four cross couplings of each
+// The rows of -A at (i, j) and w = (1/rowsum)u, (1/rowsum)v: five own-component and four cross couplings of each
 // component (ssa_operator.jl:69-89 expanded by its operands; the metric quotients that cancel are left out).
 // Planes of Nx Ny records, dense: (uE, uW, uN, uS), (uC, vC, vN, vNW, vW) of the u row in st[0] and st[1] with vW in
 // st[4].x, the v row (vN, vS, vE, vW), (vC, uC, uE, uSE, uS) in st[2], st[3] and st[4].y, and w in st[4].zw.
@@ -177,15 +177,17 @@ __device__ __forceinline__ void stencil_rows(const OpView<T>& o, int i, int j, u
     T a1c = x_normal_diagonal(o, i, j), a1w = x_normal_diagonal(o, i - 1, j);
     T a3c = y_normal_diagonal(o, i, j), a3s = y_normal_diagonal(o, i, j - 1);
     T e2 = T(2) * rc.x, e2w = T(2) * etaw, e2s = T(2) * etas;
-    T wu = (m & U_IDENTITY) ? T(0) : w.x, wv = (m & V_IDENTITY) ? T(0) : w.y;   // an identity row has its centre alone
+    const bool iu = m & U_IDENTITY, iv = m & V_IDENTITY;   // an identity row has its centre alone
+    auto uc = [iu](T x) { return iu ? T(0) : x; };
+    auto vc = [iv](T x) { return iv ? T(0) : x; };
     V4 a, b, f, h, r;
-    a.x = wu * a1c; a.y = wu * a1w; a.z = wu * c01x; a.w = wu * c00x;
-    b.x = (m & U_IDENTITY) ? -w.x : -wu * (dxf * dyc * rc.z + a1c + a1w + c01x + c00x);
-    b.y = -wu * (e2 + c00); b.z = wu * (e2 + c01); b.w = -wu * (e2w + c01);
-    f.x = wv * a3c; f.y = wv * a3s; f.z = wv * c10y; f.w = wv * c00y;
-    h.x = (m & V_IDENTITY) ? -w.y : -wv * (dxc * dyf * rc.w + a3c + a3s + c10y + c00y);
-    h.y = -wv * (e2 + c00); h.z = wv * (e2 + c10); h.w = -wv * (e2s + c10);
-    r.x = wu * (e2w + c00); r.y = wv * (e2s + c00); r.z = w.x; r.w = w.y;
+    a.x = uc(a1c); a.y = uc(a1w); a.z = uc(c01x); a.w = uc(c00x);
+    b.x = iu ? T(-1) : -(dxf * dyc * rc.z + a1c + a1w + c01x + c00x);
+    b.y = uc(-(e2 + c00)); b.z = uc(e2 + c01); b.w = uc(-(e2w + c01));
+    f.x = vc(a3c); f.y = vc(a3s); f.z = vc(c10y); f.w = vc(c00y);
+    h.x = iv ? T(-1) : -(dxc * dyf * rc.w + a3c + a3s + c10y + c00y);
+    h.y = vc(-(e2 + c00)); h.z = vc(e2 + c10); h.w = vc(-(e2s + c10));
+    r.x = uc(e2w + c00); r.y = vc(e2s + c00); r.z = w.x; r.w = w.y;
     const int n = g.Nx * g.Ny;
     st += j * g.Nx + i;
     st[0] = a; st[n] = b; st[2 * n] = f; st[3 * n] = h; st[4 * n] = r;

@@ -1,11 +1,16 @@
 """The V-cycle's kernels where one hands over to another: short periodic axes, prescribed faces, devices without room for a
 cluster, batches above the clusters' sizes, and the FP32 rows' rounding."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import nunatak_gb300 as nk
 
 gpu = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def sheet(cls, grid, solver, H, u_prescribed=None):
@@ -119,3 +124,47 @@ def test_vcycle_above_the_cluster(oracle_cls, gpu_cls, nx, ny, topology, stretch
         x, y = (0.0, nx * 2e3), (0.0, ny * 2e3 * stretch)
     grid = nk.RectilinearGrid(size=(nx, ny), x=x, y=y, topology=topology)
     vcycles(gpu_cls, oracle_cls, grid, nk.StressBalanceMultigridPreconditioner(minimum_coarse_size=20), precision, tol, nx + ny)
+
+
+# One V-cycle of a residual that does not vanish on prescribed faces: such a row keeps its part of the right-hand side in
+# the residual that a level restricts, in whichever kernel the level runs.  (Conjugate gradients start from the prescribed
+# values, so their residual is zero there.)
+def prescribed_vcycle(nx, ny, precision):
+    rng = np.random.default_rng(nx + ny)
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 2e3))
+    ud = np.full((ny, nx + 1), np.nan)
+    ud[:, 0] = 1e-5
+    ud[ny // 2, nx // 3: nx // 2] = 2e-5
+    H = np.clip(1000.0 + 300.0 * rng.standard_normal((ny, nx)), 100.0, None)
+    P = sheet(nk.Problem, grid, nk.StressBalanceSolver(preconditioner=nk.StressBalanceMultigridPreconditioner(minimum_coarse_size=8),
+                                                       precision=precision), H, ud)
+    r = residual(grid, nx)
+    z = P.precondition(*r)
+    P.close()
+    return np.stack(interior(grid, z) + interior(grid, r))   # z, then r
+
+
+def in_a_process(tmp_path, call, **env):
+    """`call` (an expression over this module's names, giving an array) evaluated in a process with `env` set."""
+    out = str(tmp_path / "out.npy")
+    code = f"import sys; sys.path[:0] = {[ROOT, ROOT + '/nunatak.jl_gb300', ROOT + '/oracle', ROOT + '/tests']!r}\n" \
+           f"import numpy as np\nfrom {__name__.rpartition('.')[2]} import *\nnp.save({out!r}, {call})\n"
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, **env), capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    return np.load(out)
+
+
+# The coarse levels' cluster against the grid-wide launches (NK_COARSEST_SMEM=0), and the one-pass levels against the FP64
+# ones, which are grid-wide at that size.  Both sides round at 1e-16 (FP32: 6e-8) of rowsum |x| in each of the ~50 sweeps.
+@gpu
+@pytest.mark.parametrize("precision, tol", [("fp64", 1e-12), ("mixed", 1e-4)])
+def test_prescribed_faces_in_the_cluster(gpu_cls, tmp_path, precision, tol):
+    got = prescribed_vcycle(40, 20, precision)
+    want = in_a_process(tmp_path, f"prescribed_vcycle(40, 20, {precision!r})", NK_COARSEST_SMEM="0")
+    assert_close(got[:2], want[:2], want[2:], tol)
+
+
+@gpu
+def test_prescribed_faces_on_one_pass_levels(gpu_cls):
+    got, want = (prescribed_vcycle(260, 66, p) for p in ("mixed", "fp64"))
+    assert_close(got[:2], want[:2], want[2:], 1e-4)
