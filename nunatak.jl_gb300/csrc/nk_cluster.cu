@@ -13,9 +13,12 @@
 //
 // Arithmetic.  A sweep is x' = x + w (b - A x) with w = 1 / rowsum.  A row of A couples five points of its own component
 // and four of the other, and its nine coefficients change only with the coefficients, so -A is formed once per solve
-// (k_inverse_row_sum, nk_solver.cu) and a sweep costs twenty multiply-adds a cell.  (The grid-wide kernels difference the
-// neighbours before they multiply; against the sum of products that only moves the rounding, by the size of the rounding
-// of x' itself.)  The residual is the sweep's own b - A x: a prescribed row, whose w is zero, keeps its b in it.
+// (k_inverse_row_sum, nk_solver.cu) and a sweep costs twenty multiply-adds and twelve subtractions a cell: as in the
+// grid-wide kernels neighbours are differenced before they are multiplied, so that a residual rounds at the size of its own
+// terms and not of rowsum |x|.  (Sums of products of whole values cost twelve operations less, 44.2 against 44.7 us a CG step
+// of 128 x 64, 67.8 against 68.3 of 320 x 160 DIVA, 150 against 160 of 300 x 180 FP64, and left a smooth mode wrong by 2e-5
+// in FP32 where differences leave 1e-6, tests/test_gpu_preconditioner_edges.py.)
+// The residual is the sweep's own b - A x: a prescribed row, whose w is zero, keeps its b in it.
 //
 // What binds it: latency, a sweep being seven shared loads, the multiply-adds and one cluster barrier.  Split: sixteen
 // CTAs of 512 threads with one cell a thread where the level allows beat eight CTAs (128 x 64 solve 66.8 against 70.5 us a CG iteration, 320 x 160 DIVA 109.9
@@ -92,8 +95,8 @@ __device__ __forceinline__ ClusterLevel<T> cluster_level(const ClusterLevels<T>&
     return K;
 }
 
-// A thread's cells of one level: the iterate, b, w and the rows of -A (E, W, N, S, centre of the own component; centre
-// and three neighbours of the other), so that a sweep is a chain of multiply-adds.
+// A thread's cells of one level: the iterate, b, w and the rows of -A (stencil_rows, nk_solver.cu), so that a sweep is a
+// chain of multiply-adds over differences of neighbours.
 template <typename T, int CPT>
 struct ClusterCells {
     using V2 = typename Vec2<T>::type;
@@ -149,11 +152,19 @@ __device__ __forceinline__ typename Vec2<T>::type cluster_residual(const Cluster
     T mu = (c.flags[k] & CELL_U) ? c.x[k].x : T(0), mv = (c.flags[k] & CELL_V) ? c.x[k].y : T(0);
     const T* u = c.u[k];
     const T* v = c.v[k];
-    T ya = c.b[k].x + u[4] * c.x[k].x + u[0] * E.x + u[1] * Wt.x, yb = u[5] * mv + u[6] * N.y + u[7] * NW.y + u[8] * Wt.y;
-    T za = c.b[k].y + v[4] * c.x[k].y + v[0] * N.y + v[1] * S.y, zb = v[5] * mu + v[6] * E.x + v[7] * SE.x + v[8] * S.x;
+    const T nc = N.y - mv, wc = Wt.y - mv, ec = E.x - mu, sc = S.x - mu;   // in both rows
     V2 r;
-    r.x = ya + (yb + (u[2] * N.x + u[3] * S.x));
-    r.y = za + (zb + (v[2] * E.y + v[3] * Wt.y));
+    if constexpr (sizeof(T) == 8) {   // the FP64 pipe: one chain, with no additions of its own (300 x 180: 162 us a CG step, 169 with three)
+        r.x = c.b[k].x + u[4] * c.x[k].x + u[0] * ec + u[1] * (Wt.x - mu) + u[2] * (N.x - mu) + u[3] * sc + u[5] * nc +
+              u[6] * (Wt.y - NW.y) + u[7] * (N.y - NW.y) + u[8] * wc;
+        r.y = c.b[k].y + v[4] * c.x[k].y + v[0] * nc + v[1] * (S.y - mv) + v[2] * (E.y - mv) + v[3] * wc + v[5] * ec +
+              v[6] * (S.x - SE.x) + v[7] * (E.x - SE.x) + v[8] * sc;
+    } else {                          // FP32, latency: three short ones
+        T ya = c.b[k].x + u[4] * c.x[k].x + u[0] * ec + u[1] * (Wt.x - mu), yb = u[5] * nc + u[6] * (Wt.y - NW.y) + u[7] * (N.y - NW.y) + u[8] * wc;
+        T za = c.b[k].y + v[4] * c.x[k].y + v[0] * nc + v[1] * (S.y - mv), zb = v[5] * ec + v[6] * (S.x - SE.x) + v[7] * (E.x - SE.x) + v[8] * sc;
+        r.x = ya + (yb + (u[2] * (N.x - mu) + u[3] * sc));
+        r.y = za + (zb + (v[2] * (E.y - mv) + v[3] * wc));
+    }
     return r;
 }
 // The first sweep of cell k, from zero, and a further one from the masked iterate in `in`

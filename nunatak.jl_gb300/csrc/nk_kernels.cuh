@@ -392,7 +392,7 @@ struct LevelView {
     typename Vec2<T>::type* q;
     T* t;                            // line-smoother scratch (one T per cell)
     const typename Vec2<T>::type* irs;  // inverse ℓ1 row sums
-    const typename Vec4<T>::type* st = nullptr;   // -A by rows, and irs (a level that nk_cluster.cu may hold, or null)
+    const typename Vec4<T>::type* st = nullptr;   // rows of -A, and irs (a level that nk_cluster.cu may hold, or null)
     int cx, cy;                      // coarsening factor from the finer level (1 or 2)
 };
 template <typename T>

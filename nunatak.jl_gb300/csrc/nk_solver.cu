@@ -158,10 +158,11 @@ void launch_inverse_diagonal(const OpView<double>& o, double2* invd, cudaStream_
     k_inverse_diagonal<<<d.grid, d.block, 0, s>>>(o, invd); count_launch();
 }
 
-// The rows of -A at (i, j) and w = (1/rowsum)u, (1/rowsum)v: five own-component and four cross couplings of each
-// component (ssa_operator.jl:69-89 expanded by its operands; the metric quotients that cancel are left out).
-// Planes of Nx Ny records, dense: (uE, uW, uN, uS), (uC, vC, vN, vNW, vW) of the u row in st[0] and st[1] with vW in
-// st[4].x, the v row (vN, vS, vE, vW), (vC, uC, uE, uSE, uS) in st[2], st[3] and st[4].y, and w in st[4].zw.
+// The rows of -A at (i, j) by differences of neighbours (C: the cell's own value, cardinal letters: its neighbours'), with
+// the metric quotients that cancel left out (ssa_operator.jl:69-89), and w = (1/rowsum)u, (1/rowsum)v.  Planes of Nx Ny
+// records, dense.  u row: st[0] of uE - uC, uW - uC, uN - uC, uS - uC; st[1] of uC, vN - vC, vW - vNW, vN - vNW; st[4].x
+// of vW - vC.  v row: st[2] of vN - vC, vS - vC, vE - vC, vW - vC; st[3] of vC, uE - uC, uS - uSE, uE - uSE; st[4].y of
+// uS - uC.  w in st[4].zw.
 template <typename T>
 __device__ __forceinline__ void stencil_rows(const OpView<T>& o, int i, int j, uint8_t m, typename Vec2<T>::type w,
                                              typename Vec4<T>::type* st) {
@@ -182,12 +183,10 @@ __device__ __forceinline__ void stencil_rows(const OpView<T>& o, int i, int j, u
     auto vc = [iv](T x) { return iv ? T(0) : x; };
     V4 a, b, f, h, r;
     a.x = uc(a1c); a.y = uc(a1w); a.z = uc(c01x); a.w = uc(c00x);
-    b.x = iu ? T(-1) : -(dxf * dyc * rc.z + a1c + a1w + c01x + c00x);
-    b.y = uc(-(e2 + c00)); b.z = uc(e2 + c01); b.w = uc(-(e2w + c01));
+    b.x = iu ? T(-1) : -(dxf * dyc * rc.z); b.y = uc(e2); b.z = uc(e2w); b.w = uc(c01);
     f.x = vc(a3c); f.y = vc(a3s); f.z = vc(c10y); f.w = vc(c00y);
-    h.x = iv ? T(-1) : -(dxc * dyf * rc.w + a3c + a3s + c10y + c00y);
-    h.y = vc(-(e2 + c00)); h.z = vc(e2 + c10); h.w = vc(-(e2s + c10));
-    r.x = uc(e2w + c00); r.y = vc(e2s + c00); r.z = w.x; r.w = w.y;
+    h.x = iv ? T(-1) : -(dxc * dyf * rc.w); h.y = vc(e2); h.z = vc(e2s); h.w = vc(c10);
+    r.x = uc(c00); r.y = vc(c00); r.z = w.x; r.w = w.y;
     const int n = g.Nx * g.Ny;
     st += j * g.Nx + i;
     st[0] = a; st[n] = b; st[2 * n] = f; st[3 * n] = h; st[4 * n] = r;

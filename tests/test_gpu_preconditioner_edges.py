@@ -168,3 +168,27 @@ def test_prescribed_faces_in_the_cluster(gpu_cls, tmp_path, precision, tol):
 def test_prescribed_faces_on_one_pass_levels(gpu_cls):
     got, want = (prescribed_vcycle(260, 66, p) for p in ("mixed", "fp64"))
     assert_close(got[:2], want[:2], want[2:], 1e-4)
+
+
+# The residual of a smooth iterate.  On a doubly periodic grid of one value everywhere the operator is a multiplication by the
+# drag's part d = (A 1), a 750th of rowsum.  Enough sweeps (15 x 750) take an iterate to where a step no longer changes its
+# last bit, a relative error of about 750 roundings; the residual b - A x must still know that error, by differences that are
+# zero here, so that the coarse level corrects it.  What is left of b / d are the roundings of b, of d (the area's product and
+# its product with the drag) and of the iterate: 16 of them allowed.  (A sum of products of whole values rounds the residual
+# at rowsum |x|, and 750 roundings stay.)
+@gpu
+@pytest.mark.parametrize("precision, rounding", [("fp64", 2.0 ** -53), ("mixed", 2.0 ** -24)])
+@pytest.mark.parametrize("nx, ny, dy", [(64, 64, 2e3), (128, 64, 1.5e3)])
+def test_residual_of_a_smooth_iterate(gpu_cls, nx, ny, dy, precision, rounding):
+    grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * dy), topology=PP)
+    mg = nk.StressBalanceMultigridPreconditioner(smoothing_sweeps=12000, coarsest_sweeps=12000, minimum_coarse_size=32)
+    P = gpu_cls(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                                          velocity_solver=nk.StressBalanceSolver(preconditioner=mg, precision=precision)))
+    for n, a in (("H", 1000.0), ("bed", 10.0), ("C", 1e8), ("A", 3e-24), ("u", 1e-5), ("v", 1e-5)):
+        P.set(n, a)
+    P.compute_geometry()
+    P.update_coefficients()
+    one = np.ones((ny, nx))
+    for z, d, b in zip(P.precondition(1.7e10 * one, -0.9e10 * one), P.apply_operator(one, one), (1.7e10, -0.9e10)):
+        assert np.max(np.abs(z * d / b - 1.0)) <= 16 * rounding
+    P.close()
