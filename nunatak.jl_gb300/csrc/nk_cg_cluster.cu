@@ -17,8 +17,6 @@
 // 128 x 64 16.8 -> 9.4; batches of 32: 64 x 32 34.5 -> 10.3, 84 x 40 48.4 -> 29.3, 128 x 64 81.0 -> 47.1.
 #include <cooperative_groups.h>
 
-#include <mutex>
-
 #include "nk_kernels.cuh"
 
 namespace nk {
@@ -299,20 +297,12 @@ void launch_cg_cluster(const CGView& v, cudaStream_t s) {
     else cudaLaunchKernelEx(&cfg, k_cg_cluster<false>, v, rows);
     count_launch();
 }
-// Once per device: clusters above eight CTAs and the shared memory of the largest grid (one row of 512 cells a CTA).
-void configure_cg_cluster() {
-    constexpr int MAX_DEVICES = 64;
-    static std::once_flag once[MAX_DEVICES];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
-    auto allow = [] {
-        for (auto* kernel : {k_cg_cluster<true>, k_cg_cluster<false>}) {
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        }
-    };
-    if (dev < 0 || dev >= MAX_DEVICES) allow();
-    else std::call_once(once[dev], allow);
+// Clusters above eight CTAs and the shared memory of the largest grid (one row of 512 cells a CTA) on the current device
+// (never in a capture), and whether it has room for one.
+bool cg_cluster_available() {
+    const size_t smem = 96 * 1024;
+    return cluster_can_be_placed(k_cg_cluster<true>, CG_CLUSTER_CTAS, CG_CLUSTER_THREADS, smem) &&
+           cluster_can_be_placed(k_cg_cluster<false>, CG_CLUSTER_CTAS, CG_CLUSTER_THREADS, smem);
 }
 
 }  // namespace nk

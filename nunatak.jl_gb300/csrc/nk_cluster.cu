@@ -29,8 +29,6 @@
 // cluster holds the finest level too it also takes the step's r.z: 128 x 64 mixed 51 -> 48 us against a pass of its own.
 #include <cooperative_groups.h>
 
-#include <mutex>
-
 #include "nk_kernels.cuh"
 #include "nk_transfer.cuh"
 
@@ -583,25 +581,12 @@ void launch_coarse_cluster(const ClusterLevels<T>& C, const int* done, const CGD
     count_launch();
 }
 template <typename T, int CPT>
-static void allow_cluster() {
-    cudaFuncSetAttribute(k_coarse_cluster<T, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLUSTER_SMEM_LIMIT);
-    cudaFuncSetAttribute(k_coarse_cluster<T, CPT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+static bool cluster_fits() {
+    return cluster_can_be_placed(k_coarse_cluster<T, CPT>, CLUSTER_MAX_CTAS, CLUSTER_THREADS, CLUSTER_SMEM_LIMIT);
 }
-// The kernels' shared-memory limit and cluster size on the current device: set once a device, when its first multigrid
-// problem is created (the attributes are the device's, and setting them is not captured).
-void configure_coarse_cluster() {
-    constexpr int MAX_DEVICES = 64;
-    static std::once_flag once[MAX_DEVICES];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
-    auto allow = [] {
-        allow_cluster<float, 1>();
-        allow_cluster<float, 2>();
-        allow_cluster<double, 1>();
-    };
-    if (dev < 0 || dev >= MAX_DEVICES) allow();
-    else std::call_once(once[dev], allow);
-}
+// The kernels' shared-memory limit and cluster size on the current device (never in a capture), and whether it has room for
+// the largest cluster that cluster_plan asks for.
+bool coarse_cluster_available() { return cluster_fits<float, 1>() && cluster_fits<float, 2>() && cluster_fits<double, 1>(); }
 
 template bool cluster_plan<float>(ClusterLevels<float>&);
 template bool cluster_plan<double>(ClusterLevels<double>&);

@@ -134,10 +134,32 @@ struct StopRule {
     }
 };
 __device__ __forceinline__ int read_done(const SolverScalars* sc) { return *(volatile const int*)&sc->done; }
+// Whether the current device can hold a cluster of `ctas` blocks of `kernel`: more than eight and more than 48 KB are opt-in
+// attributes of the kernel, and a partitioned device may have fewer free SMs in a GPC than the cluster takes.
+template <typename Kernel>
+bool cluster_can_be_placed(Kernel* kernel, int ctas, int threads, size_t smem) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    const bool fits = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+                      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                      cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+    if (!fits) cudaGetLastError();   // the grid-wide kernels take over
+    return fits;
+}
 // The whole iteration after launch_cg_init, without multigrid, in one thread-block cluster (nk_cg_cluster.cu).
 int cg_cluster_rows(int Nx, int Ny);   // rows per CTA, 0 if the grid does not fit
 void launch_cg_cluster(const CGView& v, cudaStream_t s);
-void configure_cg_cluster();
+bool cg_cluster_available();
 // z = r * invd on the Nx x Ny range, z = r on the wall faces (unit diagonal)
 void launch_precondition_diagonal(const DevGrid<double>& g, double2* z, const double2* r, const double2* invd, cudaStream_t s);
 // Picard: xprev = x (over the Nx x Ny range)
@@ -473,7 +495,7 @@ template <typename T>
 bool cluster_plan(ClusterLevels<T>& C);   // fills rows, off, ctas, cells, total, halo and window; false if the levels do not fit
 template <typename T>
 void launch_coarse_cluster(const ClusterLevels<T>& C, const int* done, const CGDot* dot, cudaStream_t s);
-void configure_coarse_cluster();
+bool coarse_cluster_available();
 // FP64 <-> FP32 conversions of vectors and of the coefficient record
 void launch_to_float(const DevGrid<double>& g, const double2* src, float2* dst, const int* done, cudaStream_t s);
 void launch_to_double(const DevGrid<double>& g, const float2* src, double2* dst, const int* done, cudaStream_t s);

@@ -179,6 +179,7 @@ struct nk_problem {
     nk_solver_desc sd{};
     int Nx = 0, Ny = 0, pitch = 0, Ns = 1;
     bool px = false, py = false;
+    bool clusters = false;   // the device has room for the cluster kernels of the problem's solver (problem_create)
     size_t plane = 0;
     bool mixed = false;
     int precond = NK_PRECONDITIONER_DIAGONAL;
@@ -575,12 +576,18 @@ static int coarse_cells_limit() {
     return limit;
 }
 
-// NK_COARSEST_SMEM=0 runs the coarse levels as grid-wide launches instead of in one thread-block cluster.
+// NK_COARSEST_SMEM=0 runs the coarse levels as grid-wide launches instead of in one thread-block cluster, NK_CLUSTERS=0
+// every solve, as on a device without room for a cluster.
+static bool environment_allows(const char* name) {
+    const char* e = std::getenv(name);
+    return !(e && std::atoi(e) == 0);
+}
 static bool coarse_levels_in_a_cluster() {
-    static bool on = [] {
-        const char* e = std::getenv("NK_COARSEST_SMEM");
-        return !(e && std::atoi(e) == 0);
-    }();
+    static bool on = environment_allows("NK_COARSEST_SMEM");
+    return on;
+}
+static bool cluster_kernels() {
+    static bool on = environment_allows("NK_CLUSTERS");
     return on;
 }
 
@@ -608,7 +615,7 @@ static bool use_graphs(const nk_problem* P) {
 // One cell more a thread spills; above the limit the grid-wide launches, which use every SM, are the faster ones.
 template <typename T>
 static bool plan_cluster(nk_problem* P, std::vector<Level<T>>& lv, int l, ClusterLevels<T>& C) {
-    if (P->sd.smoother != NK_SMOOTHER_POINT_JACOBI || !coarse_levels_in_a_cluster()) return false;
+    if (!P->clusters || P->sd.smoother != NK_SMOOTHER_POINT_JACOBI || !coarse_levels_in_a_cluster()) return false;
     if (P->nlevels - l + 1 > MAX_COARSE_LEVELS) return false;
     C = ClusterLevels<T>{};
     C.n = P->nlevels - l + 1;
@@ -779,10 +786,10 @@ static void cg_step(nk_problem* P, const CGView& v) {
 }
 
 // Whether one cluster runs the whole iteration (launch_cg_cluster) in place of the loop of cg_step: without multigrid, on
-// every grid that fits, one solve or a batch of them (a step of 84 x 40 takes 7.0 us, 16.6 in grid-wide kernels; of 128 x 64
+// every grid that fits and device with room, one solve or a batch of them (a step of 84 x 40 takes 7.0 us, 16.6 in grid-wide kernels; of 128 x 64
 // 9.4 against 16.8; of 32 such in a batch 47 against 81).
 static bool cg_in_cluster(const nk_problem* P) {
-    return P->precond != NK_PRECONDITIONER_MULTIGRID && cg_cluster_rows(P->Nx, P->Ny) > 0;
+    return P->clusters && P->precond != NK_PRECONDITIONER_MULTIGRID && cg_cluster_rows(P->Nx, P->Ny) > 0;
 }
 
 // conjugate_gradient!, conjugate_gradient.jl:165-171 (everything before the iteration loop)
@@ -1420,8 +1427,9 @@ static nk_status problem_create(nk_context* ctx, const nk_grid_desc* grid, const
         NK_CUDA(cudaEventCreate(&P->ev0));
         NK_CUDA(cudaEventCreate(&P->ev1));
         build(P);
-        if (P->precond == NK_PRECONDITIONER_MULTIGRID) configure_coarse_cluster();   // outside any capture
-        else if (cg_in_cluster(P)) configure_cg_cluster();
+        // asked anew for each problem (microseconds beside its allocation), outside any capture
+        P->clusters = cluster_kernels() && (P->precond == NK_PRECONDITIONER_MULTIGRID ? coarse_cluster_available()
+                                            : cg_cluster_rows(P->Nx, P->Ny) > 0 && cg_cluster_available());
         P->gd.x_faces = nullptr; P->gd.y_faces = nullptr; P->gd.sigma_faces = nullptr;   // no pointer kept after the call
         NK_CUDA(cudaStreamSynchronize(P->stream));
     });

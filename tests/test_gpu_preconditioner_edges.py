@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import nunatak_gb300 as nk
+from nunatak_gb300 import library
 
 gpu = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -192,3 +193,34 @@ def test_residual_of_a_smooth_iterate(gpu_cls, nx, ny, dy, precision, rounding):
     for z, d, b in zip(P.precondition(1.7e10 * one, -0.9e10 * one), P.apply_operator(one, one), (1.7e10, -0.9e10)):
         assert np.max(np.abs(z * d / b - 1.0)) <= 16 * rounding
     P.close()
+
+
+# A device without room for a cluster (NK_CLUSTERS=0): the grid-wide kernels take every solve, Jacobi on a small grid as well
+# as multigrid, with the same steps and, after a fixed number of them, the same velocities.  Ten steps from rest carry the
+# operator's 1e-16 to 1e-12 of the largest velocity; with FP64 V-cycles (1e-12) three quotients a step to 1e-9.
+def fixed_solve(preconditioner):
+    grid = nk.RectilinearGrid(size=(40, 33), x=(0.0, 80e3), y=(0.0, 66e3), topology=PB)
+    solver = nk.StressBalanceSolver(linear_iteration_control=nk.FixedIterations(10), picard_iteration_control=nk.FixedIterations(1),
+                                    preconditioner=preconditioner)
+    P = nk.Problem(grid, nk.make_descriptors(grid, rheology=nk.GlenFlowLaw(rate_factor=3e-24), friction=nk.WeertmanFriction(),
+                                             velocity_solver=solver))
+    H = np.clip(1000.0 + 300.0 * np.random.default_rng(3).standard_normal((33, 40)), 0.0, None)
+    for n, a in (("H", H), ("bed", 10.0), ("C", 1e9), ("A", 3e-24)):
+        P.set(n, a)
+    P.compute_geometry()
+    n0 = library.launch_count()
+    st = P.picard_solve()
+    out = np.concatenate([P.get("u").ravel(), P.get("v").ravel(), [st.linear_iterations_total, library.launch_count() - n0]])
+    P.close()
+    return out
+
+
+@gpu
+@pytest.mark.parametrize("preconditioner, tol", [("nk.StressBalanceDiagonalPreconditioner()", 1e-12), ("None", 1e-12),
+                                                 ("nk.StressBalanceMultigridPreconditioner(minimum_coarse_size=8)", 1e-9)])
+def test_without_clusters(gpu_cls, tmp_path, preconditioner, tol):
+    got = fixed_solve(eval(preconditioner))
+    want = in_a_process(tmp_path, f"fixed_solve({preconditioner})", NK_CLUSTERS="0")
+    assert got[-2] == want[-2] == 10
+    assert want[-1] - got[-1] >= 2 * 10 - 1   # in a cluster: one launch for the whole iteration, or one for a whole V-cycle
+    assert np.max(np.abs(got[:-2] - want[:-2])) <= tol * np.max(np.abs(want[:-2]))
