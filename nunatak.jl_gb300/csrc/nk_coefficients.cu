@@ -291,8 +291,10 @@ void launch_velocity_profile(const PhysView& ph, int diva, const double2* x, con
 
 // ---- geometry ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ double nonzero(double x) { return x == 0.0 ? 1.0 : x; }
-// x > 0 of a finite x, and a + b == 0, on the integer units (the sum itself where one is negative)
-__device__ __forceinline__ bool positive(double x) { return surely_grounded(x) && __double_as_longlong(x) != 0; }
+// x > 0 (also of infinities; not of NaN) and a + b == 0 on the integer units (the sum itself where one is negative)
+__device__ __forceinline__ bool positive(double x) {
+    return (unsigned long long)(__double_as_longlong(x) - 1) < 0x7ff0000000000000ull;
+}
 __device__ __forceinline__ bool sum_is_zero(double a, double b) {
     const long long p = __double_as_longlong(a), q = __double_as_longlong(b);
     return (p | q) >= 0 ? (p | q) == 0 : a + b == 0.0;
