@@ -680,7 +680,10 @@ __global__ void __launch_bounds__(128) k_step_enthalpy(EnergyView v, double dt) 
     auto Tpm = [&](double p) { return q.T0 - q.beta * p; };
     auto Epm = [&](double p) { return q.c * (Tpm(p) - q.Tr); };
     auto enthalpy = [&](double T, double p) { return q.c * (dmin(T, Tpm(p)) - q.Tr) + 0.0 * q.L; };
-    auto water_fraction = [&](double E, double p) { return at_least_zero(E - Epm(p)) * r_L; };
+    auto water_fraction = [&](double E, double p) {   // none also where E is NaN: max(0, E - E_pm) keeps its first operand
+        const double x = E - Epm(p);
+        return (positive(x) ? x : 0.0) * r_L;
+    };
     auto thickness = [&](double h) { return dmax(h, q.min_thickness); };
     auto layer_pressure = [&](int k) { return rho * ga * H * (1 - sg.zc[k - 1]); };
     auto Eold = [&](int k, int ii, int jj) { return v.E_old[(k - 1) * P + g.c_idx(ii, jj)]; };

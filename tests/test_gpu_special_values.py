@@ -32,3 +32,27 @@ def test_an_unbounded_velocity_is_upwinded(oracle_cls, gpu_cls, component, value
         P.close()
     assert np.array_equal(out[0], out[1], equal_nan=True)
     assert not value > 0 or np.any(np.isinf(out[1]))
+
+
+# A column whose enthalpy is NaN holds no water: max(0, E - E_pm) keeps its first operand, in the diagnosed fraction as in
+# what drains.  The other column, at rest beside it, is untouched.  (E, T and ω; 1e-10 as in the energy step's other tests.)
+@gpu
+def test_nan_enthalpy_holds_no_water(oracle_cls, gpu_cls):
+    grid = nk.RectilinearGrid(size=(2, 1), x=(0.0, 2e3), y=(0.0, 1e3))
+    out = []
+    for cls in (gpu_cls, oracle_cls):
+        P = make(cls, grid, Nsigma=6, rheology=nk.GlenFlowLaw(rate_factor="sigma"), friction=nk.WeertmanFriction())
+        E = np.full((6, 1, 2), 2009.0 * 51.0)   # temperate
+        E[3, 0, 0] = np.nan
+        for n, a in (("H", 1000.0), ("bed", 10.0), ("E", E)):
+            P.set(n, a)
+        P.compute_geometry()
+        for n, a in (("geothermal_flux", 0.042), ("surface_temperature", 243.15), ("ocean_temperature", 271.15), ("H_previous", 1000.0),
+                     ("Hw", 0.0), ("basal_melt_rate", 0.0)):
+            P.energy_set(n, a)
+        P.step_enthalpy(1e7)
+        out.append([P.get(n) for n in ("E", "T", "omega")] + [P.energy_get(n) for n in ("Hw", "grounded_melt")])
+        P.close()
+    for g, w in zip(*out):
+        assert np.allclose(g, w, rtol=1e-10, atol=0.0, equal_nan=True)
+    assert np.all(np.isnan(out[1][0][:, 0, 0])) and np.all(out[1][2][:, 0, 0] == 0.0) and np.any(out[1][2][:, 0, 1] > 0.0)
