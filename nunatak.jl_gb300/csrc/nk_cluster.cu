@@ -50,6 +50,13 @@ constexpr int CLUSTER_MAX_HALO = 8;
 template <typename T>
 constexpr int cluster_max_cells() { return sizeof(T) == 4 ? 2 : 1; }
 
+// Cells a CTA of the coarsest level in FP64.  Its twenty sweeps are the FP64 pipe's, sixteen SMs against all of them: a CG step
+// with that level alone takes 92 us in the cluster and 97 grid-wide at 64 x 96 (384 cells a CTA), 99 and 96 at 100 x 64 (400),
+// 103 and 97 at 64 x 112 (448), 113 and 95 at 128 x 64 (512); on cells that are not square 94 and 105, 100 and 107, 104 and
+// 106, 114 and 105.  A finer level of 512 cells a CTA takes four sweeps and saves its transfers' launches: 256 x 128, with
+// 128 x 64 and three more in the cluster, 156 against 258 us.
+constexpr int CLUSTER_FP64_COARSEST = 384;
+
 // One level as a CTA of the cluster sees it.
 template <typename T>
 struct ClusterLevel {
@@ -530,6 +537,7 @@ bool cluster_plan(ClusterLevels<T>& C) {
         int rows = (g.Ny + C.ctas - 1) / C.ctas;
         long long cells = (long long)rows * g.Nx;
         if (!C.lv[l].st || g.Ny > CLUSTER_MAX_ROWS || cells > (long long)cluster_max_cells<T>() * CLUSTER_THREADS) return false;
+        if (sizeof(T) == 8 && l == C.n - 1 && cells > CLUSTER_FP64_COARSEST) return false;
         int need = (int)((cells + CLUSTER_THREADS - 1) / CLUSTER_THREADS);
         while (C.cells < need) C.cells *= 2;
         C.rows[l] = rows;

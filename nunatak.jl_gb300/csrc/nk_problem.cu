@@ -611,7 +611,8 @@ static bool use_graphs(const nk_problem* P) {
 }
 
 // Whether the levels from l down run in one cluster (k_coarse_cluster), and how: levels whose rows, split over the
-// cluster's CTAs, leave a thread at most two cells in FP32 (16384 cells on a level of enough rows) or one in FP64 (8192).
+// cluster's CTAs, leave a thread at most two cells in FP32 (16384 cells on a level of enough rows) or one in FP64 (8192, the
+// coarsest level 6144, CLUSTER_FP64_COARSEST).
 // One cell more a thread spills; above the limit the grid-wide launches, which use every SM, are the faster ones.
 template <typename T>
 static bool plan_cluster(nk_problem* P, std::vector<Level<T>>& lv, int l, ClusterLevels<T>& C) {

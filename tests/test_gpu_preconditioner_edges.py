@@ -94,13 +94,13 @@ BB, PB, BP, PP = ("Bounded", "Bounded"), ("Periodic", "Bounded"), ("Bounded", "P
 
 # The coarse levels' cluster: one CTA and many, rows that do not divide by the CTAs, CTAs without rows, axes that stop
 # halving before the other, seams inside and across CTAs, odd and even sweep counts, no coarse level, FP64's largest grid
-# (8192 cells) and FP32's (16384) and one row beyond, coarsest sweeps that end on, after and before an exchange of halos.
+# (8192 cells, 6144 of the coarsest level) and FP32's (16384) and one row beyond, coarsest sweeps that end on, after and before an exchange of halos.
 @gpu
 @PRECISIONS
 @pytest.mark.parametrize("nx, ny, topology, sweeps, coarsest, minimum", [
     (16, 16, BB, 2, 20, 4), (64, 34, BB, 2, 20, 16), (96, 40, PB, 1, 7, 2), (40, 96, BP, 3, 6, 4), (72, 48, PP, 2, 1, 3),
     (75, 45, BB, 2, 20, 4), (512, 16, BB, 2, 5, 8), (128, 64, PB, 2, 20, 8), (128, 128, BB, 2, 20, 32), (128, 130, BB, 2, 20, 32),
-    (64, 64, PP, 2, 4, 16), (64, 64, PP, 2, 9, 16), (160, 80, BB, 2, 17, 20), (64, 48, BP, 2, 9, 3), (60, 44, PB, 2, 20, 44),
+    (64, 64, PP, 2, 4, 16), (64, 64, PP, 2, 9, 16), (64, 96, BB, 2, 20, 99), (80, 80, PB, 2, 7, 99), (160, 80, BB, 2, 17, 20), (64, 48, BP, 2, 9, 3), (60, 44, PB, 2, 20, 44),
 ])
 def test_vcycle_in_a_cluster(oracle_cls, gpu_cls, nx, ny, topology, sweeps, coarsest, minimum, precision, tol):
     grid = nk.RectilinearGrid(size=(nx, ny), x=(0.0, nx * 2e3), y=(0.0, ny * 1.5e3), topology=topology)
