@@ -21,12 +21,13 @@
 // The residual is the sweep's own b - A x: a prescribed row, whose w is zero, keeps its b in it.
 //
 // What binds it: latency, a sweep being seven shared loads, the multiply-adds and one cluster barrier.  Split: sixteen
-// CTAs of 512 threads with one cell a thread where the level allows beat eight CTAs (128 x 64 solve 66.8 against 70.5 us a CG iteration, 320 x 160 DIVA 109.9
-// against 125.9), 256 threads (71.7) and levels of 1024 cells kept inside the first CTA, without cluster barriers but with
+// CTAs of 512 threads with one cell a thread where the level allows beat eight CTAs (128 x 64 solve 66.8 against 70.5 us a
+// CG iteration, 320 x 160 DIVA 109.9 against 125.9), 256 threads (71.7) and levels of 1024 cells kept inside the first CTA, without cluster barriers but with
 // its one shared-memory pipe (72.4).
 // Measured, a whole CG iteration, grid-wide launches with the former one-block coarsest kernel against this one:
-// 128 x 64 mixed 105 -> 67 us, 320 x 160 DIVA 182 -> 110, 1024 x 512 297 -> 254, 300 x 180 FP64 203 -> 167.  Where the
-// cluster holds the finest level too it also takes the step's r.z: 128 x 64 mixed 51 -> 48 us against a pass of its own.
+// 128 x 64 mixed 105 -> 67 us, 320 x 160 DIVA 182 -> 110, 1024 x 512 297 -> 254, 300 x 180 FP64 203 -> 167 (with the other
+// kernels of a step as they are now 108, 130, 224 and 189 without it, 43, 70, 153 and 162 with it).  Where the cluster
+// holds the finest level too it also takes the step's r.z: 128 x 64 mixed 51 -> 48 us against a pass of its own.
 #include <cooperative_groups.h>
 
 #include "nk_kernels.cuh"
@@ -229,7 +230,8 @@ __device__ __forceinline__ const typename Vec2<T>::type* cluster_row(cg::cluster
 }
 
 // The fine points 2 I - 1 .. 2 I + 2 (I alone on an axis that is not halved) of one axis of the restriction: their
-// indices and the weights of a face-located and of a centre-located component (ridx and rweight; a point beyond a Bounded
+// indices and the weights of a face-located and of a centre-located component (ridx and rweight of nk_transfer.cuh, whose
+// rule this writes out for four points at once; a point beyond a Bounded
 // edge has weight zero and reads the edge).
 template <typename T>
 __device__ __forceinline__ void restriction_axis(int I, int Nc, int Nf, bool periodic, int c, int* at, T* face, T* centre) {

@@ -506,9 +506,11 @@ void launch_thermal_diagnostics(const DevGrid<double>& g, const SigmaTable& sig,
     k_thermal_diagnostics<<<d.grid, d.block, 0, s>>>(g, sig, plane, H, E, T, omega, A, rho_i, gacc, params); count_launch();
 }
 
-// The reconstructions of every cell at its four faces, and the limiter of a bounded WENO: one thread a cell, because a cell's two reconstructions along an axis share most of their work (weno5_cell)
-// and the limiter needs all four.  Face f of an axis holds (from cell f - 1, from cell f); a periodic axis keeps its
-// first face's pair on face N too.  θ divides only where its bound is nearer than the reconstructions' extreme: a
+// The reconstructions of every cell at its four faces, and the limiter of a bounded WENO (update_bounds_preserving_limiter!,
+// src/Models/time_stepping.jl:35-42, restated as the Zhang-Shu (2010) limiter per direction from the cell's own face values
+// and the interior quadrature values): one thread a cell, because a cell's two reconstructions along an axis share most of
+// their work (weno5_cell) and the limiter needs all four.  Face f of an axis holds (from cell f - 1, from cell f); a periodic
+// axis keeps its first face's pair on face N too.  θ divides only where its bound is nearer than the reconstructions' extreme: a
 // quotient of |numerator| >= |denominator| is at least one.  Bound by the FP64 pipe; 1500 x 1001: 774 us for the faces
 // and 166 us for the limiter as two kernels, 547 us together.
 __global__ void k_thickness_faces(ThicknessView v) {

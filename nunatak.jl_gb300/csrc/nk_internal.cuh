@@ -112,7 +112,6 @@ __device__ __forceinline__ bool prescribed_v(const DevGrid<double>& g, const dou
 // Per-solve scalars of conjugate gradients and Picard, device resident.
 struct SolverScalars {
     double rho;          // r . z of the current step
-    double rho_new;
     double alpha, beta;
     double pq;
     double rr;           // r . r

@@ -501,6 +501,5 @@ void launch_to_float(const DevGrid<double>& g, const double2* src, float2* dst, 
 void launch_to_double(const DevGrid<double>& g, const float2* src, double2* dst, const int* done, cudaStream_t s);
 void launch_coef_to_float(const DevGrid<double>& g, const double4* src, float4* dst, cudaStream_t s);
 // FP64 vector copy on the Nx x Ny range under the done predicate
-void launch_copy_vec(const DevGrid<double>& g, double2* dst, const double2* src, const int* done, cudaStream_t s);
 
 }  // namespace nk

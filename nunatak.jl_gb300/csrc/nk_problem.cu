@@ -479,7 +479,7 @@ static void build(nk_problem* P, bool dry = false) {
     slots.push_back({(void**)&P->usig, A.reserve(d2 * P->Ns)});
     P->staging_count = (size_t)(P->Nx + 1) * (P->Ny + 1) * P->Ns;
     slots.push_back({(void**)&P->staging, A.reserve(P->staging_count * sizeof(double))});
-    // the most blocks of a reduction: one a 2-D tile, the resident blocks of operator_dims and vec_dims, or the walks of
+    // the most blocks of a reduction: one a 2-D tile, the resident blocks of operator_shape and vec_dims, or the walks of
     // the V-cycle's last kernel
     LaunchDims big = dims2d(P->Nx + 1, P->Ny + 1);
     size_t nblocks = std::max((size_t)big.grid.x * big.grid.y, (size_t)8 * SM_COUNT);
@@ -674,8 +674,8 @@ static void smooth(nk_problem* P, Level<T>& L, int sweeps, bool first, const int
 // v_cycle!, multigrid_preconditioner.jl:144-163 (x ≈ A⁻¹ b from a zero guess on level l).  The levels that fit
 // run in one cluster (plan_cluster); above them an FP32 level with the default settings takes one pass down and one up
 // (nk_vcycle.cu), and any other level one grid-wide kernel a phase, its restriction also performing the coarse level's
-// first sweep from zero.  (Levels from `fused_level` down run in one block instead where NK_COARSE_CELLS asks for it.)  `dot`: the last kernel also takes the r.z of the
-// conjugate-gradient step where it can; returns whether it did.
+// first sweep from zero.  (Levels from `fused_level` down run in one block instead where NK_COARSE_CELLS asks for it.)
+// `dot`: the last kernel also takes the r.z of the conjugate-gradient step where it can; returns whether it did.
 template <typename T>
 static bool v_cycle(nk_problem* P, std::vector<Level<T>>& lv, int l, const int* done, bool first_done = false, const CGDot* dot = nullptr) {
     cudaStream_t s = P->stream;

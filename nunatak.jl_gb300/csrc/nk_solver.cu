@@ -608,18 +608,6 @@ void launch_picard_end_viscosity(const DevGrid<double>& g, const double4* coef, 
 }
 
 // ---- vector helpers under the done predicate -------------------------------------------------------------------
-__global__ void k_copy_vec(DevGrid<double> g, double2* dst, const double2* __restrict__ src, const int* done) {
-    NK_BATCH_ENTER(g, g, dst, src, done)
-    if (done && *(volatile const int*)done) return;
-    int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y;
-    if (i >= g.Nx || j >= g.Ny) return;
-    dst[g.idx(i, j)] = src[g.idx(i, j)];
-}
-void launch_copy_vec(const DevGrid<double>& g, double2* dst, const double2* src, const int* done, cudaStream_t s) {
-    LaunchDims d = dims2d(g.Nx, g.Ny);
-    k_copy_vec<<<d.grid, d.block, 0, s>>>(g, dst, src, done); count_launch();
-}
-
 __global__ void k_to_float(DevGrid<double> g, const double2* __restrict__ src, float2* dst, const int* done) {
     NK_BATCH_ENTER(g, g, src, dst, done)
     if (done && *(volatile const int*)done) return;

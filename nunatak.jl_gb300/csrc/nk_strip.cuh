@@ -493,7 +493,8 @@ __device__ __forceinline__ void strip_march(const OpView<T>& o, Load&& load, Val
         if (j + 3 <= j1) fetch(far, j + 3);
         settle(nxt, j + 1);
         T du, dv;
-        s.push(UNI ? 0 : row(j), UNI ? 0 : (!g.py && j < 0 ? 0 : row(j) + 1), (nxt.m & U_INACTIVE) ? T(0) : nxt.x.x, (nxt.m & V_INACTIVE) ? T(0) : nxt.x.y, cur.c.x, nxt.c.y, du, dv);
+        s.push(UNI ? 0 : row(j), UNI ? 0 : (!g.py && j < 0 ? 0 : row(j) + 1), (nxt.m & U_INACTIVE) ? T(0) : nxt.x.x,
+               (nxt.m & V_INACTIVE) ? T(0) : nxt.x.y, cur.c.x, nxt.c.y, du, dv);
         if (own && j >= j0) {
             const T au = UNI ? h2 : g.dxf[i] * g.dyc[j], av = UNI ? h2 : g.dxc[i] * g.dyf[j];
             V2 q;
