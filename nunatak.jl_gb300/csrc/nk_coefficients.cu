@@ -293,7 +293,7 @@ void launch_velocity_profile(const PhysView& ph, int diva, const double2* x, con
 __device__ __forceinline__ double nonzero(double x) { return x == 0.0 ? 1.0 : x; }
 // x > 0 (also of infinities; not of NaN) and a + b == 0 on the integer units (the sum itself where one is negative)
 __device__ __forceinline__ bool positive(double x) {
-    return (unsigned long long)(__double_as_longlong(x) - 1) < 0x7ff0000000000000ull;
+    return (unsigned long long)__double_as_longlong(x) - 1 < 0x7ff0000000000000ull;   // wraps at +0, above it for -0
 }
 __device__ __forceinline__ bool sum_is_zero(double a, double b) {
     const long long p = __double_as_longlong(a), q = __double_as_longlong(b);
